@@ -370,68 +370,162 @@ bool blas_dot(qcdgpu_field a, qcdgpu_field b, double out[2])
 }
 
 
-// ------------------------------------------------ multi-dot, multi-axpy
-// Gram-Schmidt and solution updates of the Krylov solvers: k dot products
-// against one field in one pass, and one field plus k scaled fields in one
-// pass (FP64 fields of one shape, taken as flat arrays of 12 x stride complex
-// numbers: the padding holds zeros). Up to kMulti fields per launch; block
-// partial sums are added in a fixed order, so the results are deterministic.
-constexpr int kMulti = 8, kMultiThreads = 256, kMultiBlocks = 1024;
+// ------------------------------------------------ Gram-Schmidt steps
+// The Gram-Schmidt step of GCR: k dot products against one field and one
+// field plus k scaled fields, in passes of up to kMulti fields (FP64 fields
+// of one shape, taken as flat arrays of 12 x stride complex numbers: the
+// padding holds zeros). The scalars stay on the device: a pass of dots leaves
+// the coefficients that the update pass reads, and the last update pass sums
+// the norm and the dot with the source of the field it writes, so no step
+// waits for the host. Block partial sums are added in a fixed order by the
+// block that finishes last, so the results are deterministic.
+//
+// FP64 arithmetic bounds both passes (four multiply-adds per complex element
+// and field: 80 us for 8 fields at 16^3 x 32, against 34 us for their bytes).
+// Two resident blocks per SM share the elements evenly, and the warps' sums
+// are reduced by halves (16 adds for 16 values instead of 80): with 1,024
+// blocks and a shuffle tree per value a pass of dots took 132 us there, now
+// 96; an update pass 104 us, now 87.
+constexpr int kMulti = 8, kMultiThreads = 256, kMultiBlocks = 304;
 
 struct MultiPtr {
   const double2 *p[kMulti];
-  double2 a[kMulti];
 };
 
-template <int J>
-__global__ void __launch_bounds__(kMultiThreads) k_multi_dot(MultiPtr x, const double2 *y, int64_t n, double *part)
+// v[0 .. W-1] summed over the warp: lane l returns the sum of entry l >> (5 - log2 W)
+template <int W>
+__device__ __forceinline__ double warp_sums(double *v)
 {
-  double re[J], im[J];
+  const int lane = threadIdx.x & 31;
+  int o = 16;
 #pragma unroll
-  for (int j = 0; j < J; j++) re[j] = im[j] = 0.0;
+  for (int w = W / 2; w >= 1; w /= 2, o /= 2) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < w; i++) {
+      const double keep = up ? v[i + w] : v[i], send = up ? v[i] : v[i + w];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+  for (; o >= 1; o /= 2) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+  return v[0];
+}
+
+// the block's sums of W values per thread to part[blockIdx.x * 16 + entry]; in
+// the block that finishes last, total[0 .. W-1] (shared) of all blocks and
+// true. done is zero between launches.
+template <int W>
+__device__ __forceinline__ bool multi_total(double *v, double *part, unsigned *done, double *total)
+{
+  constexpr int S = W == 16 ? 1 : W == 8 ? 2 : W == 4 ? 3 : 4;  // 5 - log2 W
+  __shared__ double sh[kMultiThreads / 16][16];
+  __shared__ unsigned last;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const double t = warp_sums<W>(v);
+  if ((lane & ((1 << S) - 1)) == 0) sh[tid >> 5][lane >> S] = t;
+  __syncthreads();
+  if (tid < W) {
+    double s = 0.0;
+    for (int k = 0; k < kMultiThreads / 32; k++) s += sh[k][tid];
+    part[(int64_t)blockIdx.x * 16 + tid] = s;
+  }
+  __threadfence();  // the block's partials before its count
+  __syncthreads();
+  if (tid == 0) last = atomicAdd(done, 1u) == gridDim.x - 1 ? 1u : 0u;
+  __syncthreads();
+  if (!last) return false;
+  __threadfence();
+  const int col = tid & 15, row = tid >> 4;
+  double s = 0.0;
+  if (col < W)
+    for (int b = row; b < (int)gridDim.x; b += kMultiThreads / 16) s += __ldcg(part + (int64_t)b * 16 + col);
+  sh[row][col] = s;
+  __syncthreads();
+  if (tid < W) {
+    double r = 0.0;
+    for (int k = 0; k < kMultiThreads / 16; k++) r += sh[k][tid];
+    total[tid] = r;
+  }
+  if (tid == 0) *done = 0u;
+  __syncthreads();
+  return true;
+}
+
+// dots[j] = <x_j, y> and coef[j] = -dots[j] inv2[j]
+template <int J>
+__global__ void __launch_bounds__(kMultiThreads, 2) k_multi_dot(MultiPtr x, const double2 *y, int64_t n, double *part,
+                                                                unsigned *done, double2 *dots, const double *inv2,
+                                                                double2 *coef)
+{
+  constexpr int W = J > 4 ? 16 : J > 2 ? 8 : J > 1 ? 4 : 2;
+  double v[W];
+#pragma unroll
+  for (int j = 0; j < W; j++) v[j] = 0.0;
   for (int64_t i = (int64_t)blockIdx.x * kMultiThreads + threadIdx.x; i < n; i += (int64_t)gridDim.x * kMultiThreads) {
     const double2 b = y[i];
 #pragma unroll
     for (int j = 0; j < J; j++) {
       const double2 a = x.p[j][i];  // conj(a) b
-      re[j] = fma(a.x, b.x, fma(a.y, b.y, re[j]));
-      im[j] = fma(a.x, b.y, fma(-a.y, b.x, im[j]));
+      v[2 * j] = fma(a.x, b.x, fma(a.y, b.y, v[2 * j]));
+      v[2 * j + 1] = fma(a.x, b.y, fma(-a.y, b.x, v[2 * j + 1]));
     }
   }
-  __shared__ double sh[kMultiThreads / 32][2 * kMulti];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-  for (int j = 0; j < J; j++) {
-    for (int o = 16; o > 0; o >>= 1) {
-      re[j] += __shfl_xor_sync(0xffffffffu, re[j], o);
-      im[j] += __shfl_xor_sync(0xffffffffu, im[j], o);
-    }
-    if (lane == 0) {
-      sh[w][2 * j] = re[j];
-      sh[w][2 * j + 1] = im[j];
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x < 2 * J) {
-    double t = 0.0;
-    for (int k = 0; k < kMultiThreads / 32; k++) t += sh[k][threadIdx.x];
-    part[(int64_t)blockIdx.x * 2 * kMulti + threadIdx.x] = t;
+  __shared__ double total[16];
+  if (!multi_total<W>(v, part, done, total)) return;
+  if (threadIdx.x < J) {
+    const int j = threadIdx.x;
+    dots[j] = make_double2(total[2 * j], total[2 * j + 1]);
+    coef[j] = make_double2(-total[2 * j] * inv2[j], -total[2 * j + 1] * inv2[j]);
   }
 }
 
-template <int J>
-__global__ void __launch_bounds__(kMultiThreads) k_multi_axpy(MultiPtr x, double2 *y, int64_t n)
+// y += sum_j coef[j] x_j; SUMS: also the sums of the updated y
+template <int J, bool SUMS>
+__global__ void __launch_bounds__(kMultiThreads, 2) k_multi_axpy(MultiPtr x, const double2 *coef, double2 *y, int64_t n,
+                                                                 const double2 *src, double *part, unsigned *done,
+                                                                 double *inv2, GsSums *sums)
 {
+  double2 c[J > 0 ? J : 1];
+#pragma unroll
+  for (int j = 0; j < J; j++) c[j] = coef[j];
+  double s[4] = {0.0, 0.0, 0.0, 0.0};
   for (int64_t i = (int64_t)blockIdx.x * kMultiThreads + threadIdx.x; i < n; i += (int64_t)gridDim.x * kMultiThreads) {
     double2 v = y[i];
 #pragma unroll
     for (int j = 0; j < J; j++) {
-      const double2 b = x.p[j][i], c = x.a[j];
-      v.x = fma(c.x, b.x, fma(-c.y, b.y, v.x));
-      v.y = fma(c.x, b.y, fma(c.y, b.x, v.y));
+      const double2 b = x.p[j][i];
+      v.x = fma(c[j].x, b.x, fma(-c[j].y, b.y, v.x));
+      v.y = fma(c[j].x, b.y, fma(c[j].y, b.x, v.y));
     }
-    y[i] = v;
+    if (J > 0) y[i] = v;
+    if (SUMS) {
+      const double2 b = src[i];
+      s[0] = fma(v.x, v.x, fma(v.y, v.y, s[0]));
+      s[1] = fma(v.x, b.x, fma(v.y, b.y, s[1]));
+      s[2] = fma(v.x, b.y, fma(-v.y, b.x, s[2]));
+    }
   }
+  if (!SUMS) return;
+  __shared__ double total[16];
+  if (!multi_total<4>(s, part, done, total)) return;
+  if (threadIdx.x == 0) {
+    const double r = 1.0 / total[0];
+    *inv2 = r;
+    sums->n2 = total[0];
+    sums->inv2 = r;
+    sums->dot = make_double2(total[1], total[2]);
+    sums->step = make_double2(-total[1] * r, -total[2] * r);
+  }
+}
+
+// out = y + *c x
+__global__ void __launch_bounds__(kMultiThreads) k_axpy_dev(double2 *out, const double2 *c, const double2 *x,
+                                                            const double2 *y, int64_t n)
+{
+  const int64_t i = (int64_t)blockIdx.x * kMultiThreads + threadIdx.x;
+  if (i >= n) return;
+  const double2 a = *c, b = x[i], v = y[i];
+  out[i] = make_double2(fma(a.x, b.x, fma(-a.y, b.y, v.x)), fma(a.x, b.y, fma(a.y, b.x, v.y)));
 }
 
 static unsigned multi_blocks(int64_t n)
@@ -440,84 +534,79 @@ static unsigned multi_blocks(int64_t n)
   return (unsigned)(b < kMultiBlocks ? b : kMultiBlocks);
 }
 
-bool blas_multi_dot(const qcdgpu_field *x, int k, qcdgpu_field y, std::complex<double> *out)
+static bool multi_shapes(const char *what, const qcdgpu_field *x, int k, qcdgpu_field y)
 {
-  if (k <= 0) return true;
-  for (int j = 0; j < k; j++)
-    if (!same_shape(x[j], y) || x[j]->prec != QCDGPU_F64 || y->prec != QCDGPU_F64) {
-      set_error("multi-dot: FP64 fields of one shape");
-      return false;
-    }
-  static double *part = nullptr, *host = nullptr;
-  if (!part) {
-    if (!QG_CUDA(cudaMalloc(&part, sizeof(double) * 2 * kMulti * kMultiBlocks))) return false;
-    if (!QG_CUDA(cudaMallocHost(&host, sizeof(double) * 2 * kMulti * kMultiBlocks))) return false;
-  }
+  bool ok = y->prec == QCDGPU_F64;
+  for (int j = 0; j < k; j++) ok = ok && same_shape(x[j], y) && x[j]->prec == QCDGPU_F64;
+  if (!ok) set_error("%s: FP64 fields of one shape", what);
+  return ok;
+}
+
+// scratch of the passes: block partials, then the counter
+constexpr int64_t kGsPart = 16 * kMultiBlocks;
+int64_t gs_scratch_doubles() { return kGsPart + 2; }
+bool gs_init(double *scratch) { return QG_CUDA(cudaMemsetAsync(scratch + kGsPart, 0, 2 * sizeof(double), stream())); }
+
+bool gs_dots(const qcdgpu_field *x, int k, qcdgpu_field y, double *scratch, double2 *dots, const double *inv2,
+             double2 *coef)
+{
+  if (!multi_shapes("multi-dot", x, k, y)) return false;
   const int64_t n = 12 * y->stride;
   const unsigned nb = multi_blocks(n);
+  const double2 *yy = (const double2 *)y->data;
+  unsigned *done = (unsigned *)(scratch + kGsPart);
   cudaStream_t st = stream();
   for (int j0 = 0; j0 < k; j0 += kMulti) {
-    const int J = k - j0 < kMulti ? k - j0 : kMulti;
     MultiPtr mp{};
+    const int J = k - j0 < kMulti ? k - j0 : kMulti;
     for (int j = 0; j < J; j++) mp.p[j] = (const double2 *)x[j0 + j]->data;
-    const double2 *yy = (const double2 *)y->data;
+#define QG_DOTS(J) \
+  case J: k_multi_dot<J><<<nb, kMultiThreads, 0, st>>>(mp, yy, n, scratch, done, dots + j0, inv2 + j0, coef + j0); break;
     switch (J) {
-    case 1: k_multi_dot<1><<<nb, kMultiThreads, 0, st>>>(mp, yy, n, part); break;
-    case 2: k_multi_dot<2><<<nb, kMultiThreads, 0, st>>>(mp, yy, n, part); break;
-    case 3: k_multi_dot<3><<<nb, kMultiThreads, 0, st>>>(mp, yy, n, part); break;
-    case 4: k_multi_dot<4><<<nb, kMultiThreads, 0, st>>>(mp, yy, n, part); break;
-    case 5: k_multi_dot<5><<<nb, kMultiThreads, 0, st>>>(mp, yy, n, part); break;
-    case 6: k_multi_dot<6><<<nb, kMultiThreads, 0, st>>>(mp, yy, n, part); break;
-    case 7: k_multi_dot<7><<<nb, kMultiThreads, 0, st>>>(mp, yy, n, part); break;
-    default: k_multi_dot<8><<<nb, kMultiThreads, 0, st>>>(mp, yy, n, part); break;
+      QG_DOTS(1) QG_DOTS(2) QG_DOTS(3) QG_DOTS(4) QG_DOTS(5) QG_DOTS(6) QG_DOTS(7) QG_DOTS(8)
     }
+#undef QG_DOTS
     if (!QG_LAUNCHED("multi_dot")) return false;
-    if (!QG_CUDA(cudaMemcpyAsync(host, part, sizeof(double) * 2 * kMulti * nb, cudaMemcpyDeviceToHost, st)) ||
-        !QG_CUDA(cudaStreamSynchronize(st)))
-      return false;
-    for (int j = 0; j < J; j++) {
-      double re = 0.0, im = 0.0;  // block order: deterministic
-      for (unsigned b = 0; b < nb; b++) {
-        re += host[(size_t)b * 2 * kMulti + 2 * j];
-        im += host[(size_t)b * 2 * kMulti + 2 * j + 1];
-      }
-      out[j0 + j] = std::complex<double>(re, im);
-    }
   }
   return true;
 }
 
-bool blas_multi_axpy(qcdgpu_field y, const qcdgpu_field *x, const std::complex<double> *a, int k)
+bool gs_update(qcdgpu_field y, const qcdgpu_field *x, const double2 *coef, int k, qcdgpu_field src, double *scratch,
+               double *inv2, GsSums *sums)
 {
-  for (int j = 0; j < k; j++)
-    if (!same_shape(x[j], y) || x[j]->prec != QCDGPU_F64 || y->prec != QCDGPU_F64) {
-      set_error("multi-axpy: FP64 fields of one shape");
-      return false;
-    }
+  if (!multi_shapes("multi-axpy", x, k, y) || (src && !multi_shapes("multi-axpy", &src, 1, y))) return false;
   const int64_t n = 12 * y->stride;
   const unsigned nb = multi_blocks(n);
+  double2 *yy = (double2 *)y->data;
+  const double2 *ss = src ? (const double2 *)src->data : nullptr;
+  unsigned *done = (unsigned *)(scratch + kGsPart);
   cudaStream_t st = stream();
-  for (int j0 = 0; j0 < k; j0 += kMulti) {
-    const int J = k - j0 < kMulti ? k - j0 : kMulti;
+  for (int j0 = 0; j0 < k || (j0 == 0 && src); j0 += kMulti) {
     MultiPtr mp{};
-    for (int j = 0; j < J; j++) {
-      mp.p[j] = (const double2 *)x[j0 + j]->data;
-      mp.a[j] = make_double2(a[j0 + j].real(), a[j0 + j].imag());
-    }
-    double2 *yy = (double2 *)y->data;
+    const int J = k - j0 < kMulti ? k - j0 : kMulti;
+    const bool last = src && j0 + J == k;
+    for (int j = 0; j < J; j++) mp.p[j] = (const double2 *)x[j0 + j]->data;
+#define QG_AXPY(J)                                                                                                      \
+  case J:                                                                                                               \
+    if (last) k_multi_axpy<J, true><<<nb, kMultiThreads, 0, st>>>(mp, coef + j0, yy, n, ss, scratch, done, inv2, sums); \
+    else k_multi_axpy<J, false><<<nb, kMultiThreads, 0, st>>>(mp, coef + j0, yy, n, ss, scratch, done, inv2, sums);     \
+    break;
     switch (J) {
-    case 1: k_multi_axpy<1><<<nb, kMultiThreads, 0, st>>>(mp, yy, n); break;
-    case 2: k_multi_axpy<2><<<nb, kMultiThreads, 0, st>>>(mp, yy, n); break;
-    case 3: k_multi_axpy<3><<<nb, kMultiThreads, 0, st>>>(mp, yy, n); break;
-    case 4: k_multi_axpy<4><<<nb, kMultiThreads, 0, st>>>(mp, yy, n); break;
-    case 5: k_multi_axpy<5><<<nb, kMultiThreads, 0, st>>>(mp, yy, n); break;
-    case 6: k_multi_axpy<6><<<nb, kMultiThreads, 0, st>>>(mp, yy, n); break;
-    case 7: k_multi_axpy<7><<<nb, kMultiThreads, 0, st>>>(mp, yy, n); break;
-    default: k_multi_axpy<8><<<nb, kMultiThreads, 0, st>>>(mp, yy, n); break;
+      QG_AXPY(0) QG_AXPY(1) QG_AXPY(2) QG_AXPY(3) QG_AXPY(4) QG_AXPY(5) QG_AXPY(6) QG_AXPY(7) QG_AXPY(8)
     }
+#undef QG_AXPY
     if (!QG_LAUNCHED("multi_axpy")) return false;
   }
   return true;
+}
+
+bool blas_axpy_dev(qcdgpu_field out, const double2 *c, qcdgpu_field x, qcdgpu_field y)
+{
+  if (!multi_shapes("axpy", &x, 1, y) || !same_shape(out, y) || out->prec != QCDGPU_F64) return false;
+  const int64_t n = 12 * y->stride;
+  k_axpy_dev<<<(unsigned)((n + kMultiThreads - 1) / kMultiThreads), kMultiThreads, 0, stream()>>>(
+      (double2 *)out->data, c, (const double2 *)x->data, (const double2 *)y->data, n);
+  return QG_LAUNCHED("axpy_dev");
 }
 
 }  // namespace qg

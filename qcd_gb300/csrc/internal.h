@@ -196,10 +196,23 @@ bool blas_norm2_dev(qcdgpu_field x, double *res);
 bool blas_dot_dev(qcdgpu_field a, qcdgpu_field b, double *res);
 // host-returning versions (synchronise)
 bool blas_norm2(qcdgpu_field x, double *out);
-// FP64 fields: out[j] = <x_j, y> for j < k in one pass per 8 fields (host
-// results, fixed summation order); y += sum_j a_j x_j in one pass per 8
-bool blas_multi_dot(const qcdgpu_field *x, int k, qcdgpu_field y, std::complex<double> *out);
-bool blas_multi_axpy(qcdgpu_field y, const qcdgpu_field *x, const std::complex<double> *a, int k);
+// The Gram-Schmidt step on FP64 fields with its scalars on the device (fixed
+// summation order, no synchronisation). scratch: gs_scratch_doubles() doubles,
+// cleared once by gs_init.
+//   gs_dots:   dots[j] = <x_j, y>, coef[j] = -dots[j] inv2[j], j < k
+//   gs_update: y += sum_j coef[j] x_j; with src also *sums of y, and *inv2
+//   blas_axpy_dev: out = y + *c x
+struct GsSums {
+  double n2, inv2;    // |y|^2 and 1 / |y|^2
+  double2 dot, step;  // <y, src> and -<y, src> / |y|^2
+};
+int64_t gs_scratch_doubles();
+bool gs_init(double *scratch);
+bool gs_dots(const qcdgpu_field *x, int k, qcdgpu_field y, double *scratch, double2 *dots, const double *inv2,
+             double2 *coef);
+bool gs_update(qcdgpu_field y, const qcdgpu_field *x, const double2 *coef, int k, qcdgpu_field src, double *scratch,
+               double *inv2, GsSums *sums);
+bool blas_axpy_dev(qcdgpu_field out, const double2 *c, qcdgpu_field x, qcdgpu_field y);
 bool blas_dot(qcdgpu_field a, qcdgpu_field b, double out[2]);
 // fused: y = y + a*x  followed by |y|^2 (device result)
 bool blas_axpy_norm2_dev(qcdgpu_field y, double ar, double ai, qcdgpu_field x, double *res);

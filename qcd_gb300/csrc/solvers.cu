@@ -31,6 +31,8 @@ namespace qg {
 
 using cplx = std::complex<double>;
 
+double *big_partials(int64_t n);
+
 int g_gcr_shipped = 0;
 
 // ------------------------------------------------------------- helpers
@@ -67,7 +69,6 @@ static bool caxpy(qcdgpu_field out, cplx a, qcdgpu_field x, qcdgpu_field y)
 {
   return blas_axpby(out, a.real(), a.imag(), x, 1.0, 0.0, y);
 }
-static bool scale(qcdgpu_field x, double s) { return blas_axpby(x, s, 0.0, x, 0.0, 0.0, x); }
 
 // low-precision copies of gauge fields, keyed by the FP64 field
 struct LowKey {
@@ -124,48 +125,58 @@ int gcr_dropin(qcdgpu_field sol, qcdgpu_field src, qcdgpu_gauge g, double mp4, d
       return 1;
     }
   }
-  std::vector<cplx> a((size_t)n * n), c((size_t)n);
-  auto A = [&](int i, int j) -> cplx & { return a[(size_t)i * n + j]; };
-  double nv;
-  if (!blas_copy(res[0], src)) return 1;
-  if (!dslash(chi[0], res[0], g, mp4, tm, QCDGPU_OP_Q, -1)) return 1;
-  if (!norm(chi[0], &nv)) return 1;
-  A(0, 0) = 1.0 / nv;
-  if (!scale(chi[0], A(0, 0).real())) return 1;
-  if (!dot(chi[0], src, &c[0])) return 1;
-  if (!blas_zero(sol)) return 1;
-  if (!shipped && !caxpy(sol, c[0] * A(0, 0), res[0], sol)) return 1;
-  for (int k = 1; k < n; k++) {
-    if (!caxpy(res[(size_t)k], -c[(size_t)k - 1], chi[(size_t)k - 1], res[(size_t)k - 1])) return 1;
-    if (!dslash(chi[(size_t)k], res[(size_t)k], g, mp4, tm, QCDGPU_OP_Q, -1)) return 1;
-    // Gram-Schmidt against the orthonormal chi_0 .. chi_{k-1}: the k
-    // projections in one pass, then one batched update (classical form; for
-    // an orthonormal basis its coefficients are modified Gram-Schmidt's,
-    // invert.c:68-79)
-    {
-      std::vector<cplx> t((size_t)k);
-      if (!blas_multi_dot(chi.data(), k, chi[(size_t)k], t.data())) return 1;
-      for (int j = 0; j < k; j++) A(k, j) = -t[(size_t)j];
-      if (!blas_multi_axpy(chi[(size_t)k], chi.data(), &A(k, 0), k)) return 1;
-    }
-    if (!norm(chi[(size_t)k], &nv)) return 1;
-    A(k, k) = 1.0 / nv;
-    if (std::isnan(A(k, k).real())) {
-      set_error("gcr: Krylov space is sick (NaN norm)");
+  // Device scalars: n sums, n reciprocal norms, n x n dots, the coefficients
+  // of one step (and of the solution), then the passes' scratch. The basis
+  // chi stays unnormalised: 1 / |chi_j|^2 goes into the coefficients.
+  const size_t nsum = (size_t)n * sizeof(GsSums) / sizeof(double), ndot = 2 * (size_t)n * n;
+  double *dev = big_partials((int64_t)(nsum + ndot + 3 * (size_t)n) + 2 + gs_scratch_doubles());
+  if (!dev) return 1;
+  GsSums *sums = (GsSums *)dev;
+  double2 *dots = (double2 *)(dev + nsum), *coef = dots + (size_t)n * n;
+  double *inv2 = (double *)(coef + n), *scratch = inv2 + (n + 1) / 2 * 2;
+  if (!gs_init(scratch) || !blas_copy(res[0], src)) return 1;
+  for (int k = 0; k < n; k++) {
+    const size_t K = (size_t)k;
+    if (k > 0 && !blas_axpy_dev(res[K], &sums[K - 1].step, chi[K - 1], res[K - 1])) return 1;
+    if (!dslash(chi[K], res[K], g, mp4, tm, QCDGPU_OP_Q, -1)) return 1;
+    // Gram-Schmidt against chi_0 .. chi_{k-1}: the k projections, then one
+    // batched update (classical form; for an orthogonal basis its coefficients
+    // are modified Gram-Schmidt's, invert.c:68-79) that also sums |chi_k|^2
+    // and <chi_k, src>. No pass waits for the host.
+    if (!gs_dots(chi.data(), k, chi[K], scratch, dots + K * n, inv2, coef) ||
+        !gs_update(chi[K], chi.data(), coef, k, src, scratch, inv2 + k, sums + k))
       return 1;
-    }
-    if (!scale(chi[(size_t)k], A(k, k).real())) return 1;
-    for (int j = 0; j < k; j++) A(k, j) *= A(k, k).real();
+  }
+  std::vector<GsSums> hs((size_t)n);
+  std::vector<cplx> hd((size_t)n * n), a((size_t)n * n), sol_coef((size_t)n);
+  cudaStream_t st = stream();
+  if (!QG_CUDA(cudaMemcpyAsync(hs.data(), sums, sizeof(GsSums) * n, cudaMemcpyDeviceToHost, st)) ||
+      !QG_CUDA(cudaMemcpyAsync(hd.data(), dots, sizeof(double) * ndot, cudaMemcpyDeviceToHost, st)) ||
+      !QG_CUDA(cudaStreamSynchronize(st)))
+    return 1;
+  // sol = sum_k c_k sum_{j <= k} A(k, j) res_j, one pass over the res_j at the end
+  auto A = [&](int i, int j) -> cplx & { return a[(size_t)i * n + j]; };
+  bool sick = false;
+  for (int k = 0; k < n && !sick; k++) {
+    const double inv = 1.0 / sqrt(hs[(size_t)k].n2);
+    sick = k > 0 && std::isnan(inv);
+    if (sick) break;
+    A(k, k) = inv;
+    for (int j = 0; j < k; j++) A(k, j) = -(hd[(size_t)k * n + j] * A(j, j).real()) * inv;
     for (int j = 0; j < k; j++) {
       A(k, j) *= A(j, j).real();
       for (int l = j + 1; l < k; l++) A(k, j) += A(k, l) * A(l, j);
     }
-    if (!dot(chi[(size_t)k], src, &c[(size_t)k])) return 1;
-    {
-      std::vector<cplx> coef((size_t)k + 1);
-      for (int j = 0; j <= k; j++) coef[(size_t)j] = c[(size_t)k] * A(k, j);
-      if (!blas_multi_axpy(sol, res.data(), coef.data(), k + 1)) return 1;
-    }
+    const cplx c = cplx(hs[(size_t)k].dot.x, hs[(size_t)k].dot.y) * inv;
+    if (k > 0 || !shipped)
+      for (int j = 0; j <= k; j++) sol_coef[(size_t)j] += c * A(k, j);
+  }
+  if (!blas_zero(sol) || !QG_CUDA(cudaMemcpyAsync(coef, sol_coef.data(), sizeof(cplx) * n, cudaMemcpyHostToDevice, st)) ||
+      !gs_update(sol, res.data(), coef, n, nullptr, scratch, nullptr, nullptr))
+    return 1;
+  if (sick) {
+    set_error("gcr: Krylov space is sick (NaN norm)");
+    return 1;
   }
   return 0;
 }
