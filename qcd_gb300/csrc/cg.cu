@@ -38,6 +38,7 @@ using namespace qgd;
 bool dslash_partials(qcdgpu_field out, qcdgpu_field in, qcdgpu_gauge g, double mp4, double tm, bool dag,
                      int arith, double *partials, const CgFuse *fuse = nullptr);
 double *big_partials(int64_t n);
+int64_t dslash_df64_blocks(int64_t V);
 
 constexpr int kChunk = 16;
 
@@ -208,7 +209,9 @@ static int cgnr_core(qcdgpu_field y, qcdgpu_field c, double cn, const CgOps &ops
   const int V = (int)rt->V;
   const unsigned nb = (unsigned)((V + 127) / 128);            // operator launches: 128 sites per block
   const unsigned nbr = (unsigned)((V + kCgSites - 1) / kCgSites);  // the fused reductions
-  double *part = big_partials(nb);
+  // one partial per block of the operator: 128 sites, fewer in the float-float kernel
+  const int64_t nff = dslash_df64_blocks(V);
+  double *part = big_partials(prec == QCDGPU_F64 && nff > nb ? nff : nb);
   double *s = reduce_scratch();
   double *h = host_result();
   if (!part || !s || !h) return 3;

@@ -85,7 +85,7 @@ __device__ __forceinline__ void cg_scalars_from(double t, double *s, int mode, i
   }
 }
 
-// Called by every thread of a 128-thread block after block_partial wrote the
+// Called by every thread of a block after block_partial wrote the
 // block's partial: the block that finishes last sums all gridDim.x partials
 // in index order (the same order whichever block is last), updates the
 // scalars and re-arms the counter. No block waits for another.
@@ -100,16 +100,18 @@ __device__ __forceinline__ void cg_last_block(const double *partials, unsigned *
   __syncthreads();
   if (!last) return;
   __threadfence();
-  // eight independent loads in flight per thread, summed in a fixed order
+  // 24 independent loads in flight per thread, summed in a fixed order: one
+  // round of loads for the half-lattice launches of 24^3 x 48 (2,592 partials)
   const int n = (int)gridDim.x;
   double v = 0.0;
   const int nt = (int)blockDim.x;
-  for (int i0 = threadIdx.x; i0 < n; i0 += 8 * nt) {
-    double w[8];
+  constexpr int kLoads = 24;
+  for (int i0 = threadIdx.x; i0 < n; i0 += kLoads * nt) {
+    double w[kLoads];
 #pragma unroll
-    for (int k = 0; k < 8; k++) w[k] = i0 + k * nt < n ? __ldcg(partials + i0 + k * nt) : 0.0;
+    for (int k = 0; k < kLoads; k++) w[k] = i0 + k * nt < n ? __ldcg(partials + i0 + k * nt) : 0.0;
 #pragma unroll
-    for (int k = 0; k < 8; k++) v += w[k];
+    for (int k = 0; k < kLoads; k++) v += w[k];
   }
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;

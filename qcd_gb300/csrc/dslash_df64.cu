@@ -13,10 +13,9 @@
 //     renormalised (Fast2Sum) only when its value is consumed.
 // Every operation uses the explicitly rounded intrinsics, so the compiler can
 // neither contract nor reorder them. The double -> float-pair splits of the
-// spinors (eight per hop and thread) use integer bit operations, because the
-// hardware conversions run on the FP64 pipe; the pair -> double joins of the
-// result (once per output component) use the FP64 pipe. The links come from a copy of the gauge field stored as
-// float pairs, made once per field, with the boundary phase e^{i th/L}
+// spinors (four per hop and thread) and the widenings of the results use
+// integer bit operations, because the hardware conversions run on the FP64
+// pipe. The links come from a copy of the gauge field stored as float pairs, made once per field, with the boundary phase e^{i th/L}
 // multiplied into the links of twisted directions (U' h for the forward hop,
 // U'^+ h = e^{-i th/L} U^+ h for the backward one, as qcd_wilson.c applies it).
 // The result differs from FP64 by a few 2^-46 relative, within the 1e-13
@@ -32,213 +31,195 @@ using namespace qgd;
 struct F2 {  // h + l
   float h, l;
 };
-struct FA {  // accumulator: value s + e, not normalised
-  float s, e;
-};
-struct CF {
-  F2 re, im;
-};
-struct CA {
-  FA re, im;
-};
 
-// out of line, so the common path does not carry its FP64 conversions
-__device__ __noinline__ F2 split_slow(double d)
+// double -> float pair, any value
+__device__ F2 split_any(double d)
 {
+  const unsigned e = ((unsigned)__double2hiint(d) >> 20) & 0x7ffu;
   F2 r;
-  r.h = __double2float_rn(d);
-  r.l = __double2float_rn(__dsub_rn(d, (double)r.h));
-  return r;
-}
-
-// double -> float pair. In range (|d| in [2^-74, 2^127)) with integer bit
-// operations: hi takes the leading 24 significand bits and lo the next 23
-// (both truncated; the pair keeps 47 bits, relative error below 2^-46).
-__device__ __forceinline__ F2 split_d(double d)
-{
-  const unsigned lo32 = (unsigned)__double2loint(d), hi32 = (unsigned)__double2hiint(d);
-  const unsigned e = (hi32 >> 20) & 0x7ffu;
-  F2 r;
-  if (e - 949u <= 201u) {  // e in [949, 1150]
-    // (hi32:lo32) << 3 holds the exponent's low 9 bits and the top 23
-    // significand bits in float position; e - 896 = (e mod 512) - 384 here,
-    // so one subtraction rebiases the exponent, and the sign goes back in
-    const unsigned hb = (__funnelshift_l(lo32, hi32, 3) - (384u << 23)) | (hi32 & 0x80000000u);
-    r.h = __uint_as_float(hb);
-    // the 23 bits below hi as an exact integer-valued float, scaled by
-    // 2^(e - 1069) with hi's sign: hi's sign and exponent field less 46
-    const float f1 = __fsub_rn(__uint_as_float(0x4B000000u | ((lo32 >> 6) & 0x7fffffu)), 8388608.0f);
-    r.l = __fmul_rn(f1, __uint_as_float((hb & 0xff800000u) - (46u << 23)));
-  } else if (e == 0u) {
-    r.h = __uint_as_float(hi32 & 0x80000000u);
+  if (e == 0u) {
+    r.h = __uint_as_float((unsigned)__double2hiint(d) & 0x80000000u);
     r.l = 0.0f;
   } else {
-    r = split_slow(d);
+    r.h = __double2float_rn(d);
+    r.l = __double2float_rn(__dsub_rn(d, (double)r.h));
   }
   return r;
 }
 
-// h + l -> double: two exact widenings and one FP64 add, rounded to nearest.
-// The join runs once per output component, in the epilogue, where the FP64
-// pipe has room; it replaced an integer bit-assembly of the double (~30
-// instructions on the issue-bound side): 0.388 -> 0.372 ms per 24^3x48 apply.
-__device__ __forceinline__ double join_d(F2 x) { return __dadd_rn((double)x.h, (double)x.l); }
-
-__device__ __forceinline__ void two_sum(float a, float b, float &s, float &q)
+// In range (|d| in [2^-74, 2^127)) with integer bit operations: hi takes the
+// leading 24 significand bits and lo the next 23 (both truncated; the pair
+// keeps 47 bits, relative error below 2^-46).
+__device__ __forceinline__ F2 split_d(double d)
 {
-  s = __fadd_rn(a, b);
-  float bb = __fsub_rn(s, a);
-  q = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
-}
-__device__ __forceinline__ F2 neg(F2 a) { return F2{-a.h, -a.l}; }
-// a + b, unnormalised
-__device__ __forceinline__ F2 add(F2 a, F2 b)
-{
+  const unsigned lo32 = (unsigned)__double2loint(d), hi32 = (unsigned)__double2hiint(d);
   F2 r;
-  float q;
-  two_sum(a.h, b.h, r.h, q);
-  r.l = __fadd_rn(q, __fadd_rn(a.l, b.l));
+  // (hi32:lo32) << 3 holds the exponent's low 9 bits and the top 23
+  // significand bits in float position; e - 896 = (e mod 512) - 384 here,
+  // so one subtraction rebiases the exponent, and the sign goes back in
+  const unsigned hb = (__funnelshift_l(lo32, hi32, 3) - (384u << 23)) | (hi32 & 0x80000000u);
+  r.h = __uint_as_float(hb);
+  // the 23 bits below hi as an exact integer-valued float, scaled by
+  // 2^(e - 1069) with hi's sign: hi's sign and exponent field less 46
+  const float f1 = __fsub_rn(__uint_as_float(0x4B000000u | ((lo32 >> 6) & 0x7fffffu)), 8388608.0f);
+  r.l = __fmul_rn(f1, __uint_as_float((hb & 0xff800000u) - (46u << 23)));
   return r;
 }
-__device__ __forceinline__ F2 fin(FA a)
+
+struct F2Quad {
+  F2 ar, ai, br, bi;
+};
+// a zero or a value out of range among the four: out of line
+__device__ __noinline__ F2Quad split_slow(double2 a, double2 b)
 {
-  float s = __fadd_rn(a.s, a.e);
-  return F2{s, __fsub_rn(a.e, __fsub_rn(s, a.s))};
+  auto one = [](double d) {
+    const unsigned e = ((unsigned)__double2hiint(d) >> 20) & 0x7ffu;
+    return e - 949u <= 201u ? split_d(d) : split_any(d);
+  };
+  return F2Quad{one(a.x), one(a.y), one(b.x), one(b.y)};
 }
-// acc += a * b
-__device__ __forceinline__ void mac(FA &acc, F2 a, F2 b)
+// exponent distance above 2^-74 (in units of the exponent field)
+__device__ __forceinline__ unsigned split_range(double d)
 {
-  float p = __fmul_rn(a.h, b.h);
-  float t = __fmaf_rn(a.h, b.h, -p);
-  float s, q;
-  two_sum(acc.s, p, s, q);
-  float e = __fadd_rn(acc.e, __fadd_rn(t, q));
-  e = __fmaf_rn(a.h, b.l, e);
-  acc.e = __fmaf_rn(a.l, b.h, e);
-  acc.s = s;
-}
-// acc += x
-__device__ __forceinline__ void acc_add(FA &acc, F2 x)
-{
-  float s, q;
-  two_sum(acc.s, x.h, s, q);
-  acc.e = __fadd_rn(acc.e, __fadd_rn(q, x.l));
-  acc.s = s;
+  return ((unsigned)__double2hiint(d) & 0x7ff00000u) - (949u << 20);
 }
 
-// acc = a * b into an empty accumulator: no error-free sum needed
-__device__ __forceinline__ FA mac0(F2 a, F2 b)
+// h + l -> double: two exact widenings and one FP64 add, rounded to nearest
+__device__ __forceinline__ double join_d(F2 x) { return __dadd_rn((double)x.h, (double)x.l); }
+// the same with the widenings as integer operations (the conversions run on
+// the FP64 pipe), for normal h and l
+__device__ __forceinline__ double widen(float f)
 {
-  const float p = __fmul_rn(a.h, b.h);
-  float e = __fmaf_rn(a.h, b.h, -p);
-  e = __fmaf_rn(a.h, b.l, e);
-  return FA{p, __fmaf_rn(a.l, b.h, e)};
+  const unsigned b = __float_as_uint(f);
+  return __hiloint2double((int)((((b & 0x7fffffffu) >> 3) + 0x38000000u) | (b & 0x80000000u)), (int)(b << 29));
+}
+__device__ __forceinline__ double join_fast(float h, float l) { return __dadd_rn(widen(h), widen(l)); }
+// below 0x7f000000 for normal f
+__device__ __forceinline__ unsigned widen_range(float f) { return (__float_as_uint(f) & 0x7fffffffu) - 0x00800000u; }
+
+// Two pairs at once, in the halves of sm_103a's packed FP32 operations (one
+// issue slot for two results; each half rounds as the scalar operation does).
+struct F2x2 {
+  float2 h, l;
+};
+struct FAx2 {  // accumulator: values s + e, not normalised
+  float2 s, e;
+};
+struct CAx2 {
+  FAx2 re, im;
+};
+__device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
+// a - b: a multiply-add by -1 rounds the same, and a negated operand of a
+// packed add costs instructions of its own (24^3 x 48: 0.336 against 0.306 ms)
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a); }
+__device__ __forceinline__ float2 dup2(float a) { return make_float2(a, a); }
+__device__ __forceinline__ void two_sum2(float2 a, float2 b, float2 &s, float2 &q)
+{
+  s = __fadd2_rn(a, b);
+  const float2 bb = sub2(s, a);
+  q = __fadd2_rn(sub2(a, sub2(s, bb)), sub2(b, bb));
+}
+// acc += a * b; nah = -a.h (t is the product's error, negated: a negated
+// operand of a packed operation costs an instruction of its own)
+__device__ __forceinline__ void mac2(FAx2 &acc, F2x2 a, float2 nah, F2x2 b)
+{
+  const float2 p = __fmul2_rn(a.h, b.h);
+  const float2 t = __ffma2_rn(nah, b.h, p);
+  float2 s, q;
+  two_sum2(acc.s, p, s, q);
+  float2 e = __fadd2_rn(acc.e, sub2(q, t));
+  e = __ffma2_rn(a.h, b.l, e);
+  acc.e = __ffma2_rn(a.l, b.h, e);
+  acc.s = s;
+}
+// acc = a * b into an empty accumulator: no error-free sum needed
+__device__ __forceinline__ FAx2 mac02(F2x2 a, float2 nah, F2x2 b)
+{
+  const float2 p = __fmul2_rn(a.h, b.h);
+  float2 e = __ffma2_rn(a.h, b.h, __fmul2_rn(nah, b.h));
+  e = __ffma2_rn(a.h, b.l, e);
+  return FAx2{p, __ffma2_rn(a.l, b.h, e)};
 }
 // acc += x for an unnormalised x
-__device__ __forceinline__ void acc_add_fa(FA &acc, FA x)
+__device__ __forceinline__ void acc_add2(FAx2 &acc, FAx2 x)
 {
-  float s, q;
-  two_sum(acc.s, x.s, s, q);
-  acc.e = __fadd_rn(acc.e, __fadd_rn(q, x.e));
+  float2 s, q;
+  two_sum2(acc.s, x.s, s, q);
+  acc.e = __fadd2_rn(acc.e, __fadd2_rn(q, x.e));
   acc.s = s;
 }
-__device__ __forceinline__ FA fneg(FA a) { return FA{-a.s, -a.e}; }
-struct CFA {  // complex accumulator value
-  FA re, im;
-};
-// z -> (i z if ifl) then negated if ng
-__device__ __forceinline__ CFA coefa(CFA z, bool ifl, bool ng)
+// (a, b) and their imaginary parts as pairs: one range test for the four values
+__device__ __forceinline__ void split_pair(double2 a, double2 b, F2x2 &re, F2x2 &im)
 {
-  CFA r = ifl ? CFA{fneg(z.im), z.re} : z;
-  return ng ? CFA{fneg(r.re), fneg(r.im)} : r;
+  F2Quad q;
+  if (max(max(split_range(a.x), split_range(a.y)), max(split_range(b.x), split_range(b.y))) <= (201u << 20))
+    q = F2Quad{split_d(a.x), split_d(a.y), split_d(b.x), split_d(b.y)};
+  else
+    q = split_slow(a, b);
+  re = F2x2{make_float2(q.ar.h, q.br.h), make_float2(q.ar.l, q.br.l)};
+  im = F2x2{make_float2(q.ai.h, q.bi.h), make_float2(q.ai.l, q.bi.l)};
 }
-__device__ __forceinline__ void cacc_fa(CA &acc, CFA x)
+// re + i im of both halves
+__device__ __forceinline__ void join_pair(F2x2 re, F2x2 im, double2 &a, double2 &b)
 {
-  acc_add_fa(acc.re, x.re);
-  acc_add_fa(acc.im, x.im);
+  const unsigned m0 = max(max(widen_range(re.h.x), widen_range(re.l.x)), max(widen_range(im.h.x), widen_range(im.l.x)));
+  const unsigned m1 = max(max(widen_range(re.h.y), widen_range(re.l.y)), max(widen_range(im.h.y), widen_range(im.l.y)));
+  if (max(m0, m1) < 0x7f000000u) {
+    a = make_double2(join_fast(re.h.x, re.l.x), join_fast(im.h.x, im.l.x));
+    b = make_double2(join_fast(re.h.y, re.l.y), join_fast(im.h.y, im.l.y));
+  } else {
+    a = make_double2(join_d(F2{re.h.x, re.l.x}), join_d(F2{im.h.x, im.l.x}));
+    b = make_double2(join_d(F2{re.h.y, re.l.y}), join_d(F2{im.h.y, im.l.y}));
+  }
 }
-
-__device__ __forceinline__ CF cadd(CF a, CF b) { return CF{add(a.re, b.re), add(a.im, b.im)}; }
-__device__ __forceinline__ CF cneg(CF a) { return CF{neg(a.re), neg(a.im)}; }
-__device__ __forceinline__ CF ci(CF a) { return CF{neg(a.im), a.re}; }  // i a
-__device__ __forceinline__ void cacc(CA &acc, CF x)
+// the two halves exchanged
+__device__ __forceinline__ FAx2 flip2(FAx2 v)
 {
-  acc_add(acc.re, x.re);
-  acc_add(acc.im, x.im);
-}
-
-__device__ __forceinline__ CF load_sp(const double2 *base, int64_t stride, int y, int k)
-{
-  double2 v = __ldg(base + (int64_t)k * stride + y);
-  return CF{split_d(v.x), split_d(v.y)};
-}
-__device__ __forceinline__ CF load_link(const float4 *base, int64_t stride, int y, int mu, int k)
-{
-  float4 v = __ldg(base + ((int64_t)mu * 9 + k) * stride + y);
-  return CF{F2{v.x, v.y}, F2{v.z, v.w}};
+  return FAx2{make_float2(v.s.y, v.s.x), make_float2(v.e.y, v.e.x)};
 }
 
-// z -> (i z if ifl) then negated if ng; ifl and ng are warp-uniform
-__device__ __forceinline__ CF coef(CF z, bool ifl, bool ng)
-{
-  CF r = ifl ? CF{neg(z.im), z.re} : z;
-  return ng ? cneg(r) : r;
-}
-
-// Thread layout: a block of 96 * kFFGroups threads covers 32 * kFFGroups
-// sites as groups of three warps; warp w of a group owns colour row i = w for its 32 sites and
-// the four accumulators (spins 0..3) of that colour. Per hop each warp
-// projects the neighbour spinor of its colour, the three warps share the
-// half spinors through shared memory, and each warp multiplies its link row.
-// The eight hops are unrolled (directions and signs compile-time); with S
-// the projector sign,
-// (1 + S g_mu) in the chiral basis is
+// Thread layout: a block of three warps covers 32 sites; warp w owns colour
+// row i = w and the four accumulators (spins 0..3) of that colour. Per hop
+// each warp projects the neighbour spinor of its colour, the three warps share
+// the half spinors through shared memory, and each multiplies its link row.
+// With S the projector sign, (1 + S g_mu) in the chiral basis is
 //   h0 = p0 + c0 p_b0, h1 = p1 + c1 p_b1            (upper half)
 //   b0 = 2 (mu 0,3) or 3 (mu 1,2), b1 = 5 - b0, c = +-1 (mu even) or +-i (odd)
 //   c0 = -S ; c1 = -S (mu 0,1) or +S (mu 2,3)
 // and the lower half rebuilt from v = U h:
 //   r2 = cA v_jA, r3 = cB v_jB ; jA = 1 for mu 1,2 else 0, jB = 1 - jA
 //   cA = -S (mu 0) else +S ; cB = +S (mu 1) else -S ; times i for odd mu
-// (qcd_wilson.h:17-387).
+// (qcd_wilson.h:17-387). The directions run 0, 3, 1, 2: the lower pair is
+// accumulated as (spin 2, spin 3) for the first two and as (3, 2) for the
+// others, so that no hop exchanges the halves of a pair.
 //
-// Each group of three warps synchronises on its own named barrier (ids 1..4,
-// 96 threads), so the four groups of a block never wait for one another.
-//
-// The spin projections (adds of two spinor components) run in native FP64
-// straight after the loads, and only the half spinor is split into float
-// pairs: two double -> pair conversions per half-spinor component instead of
-// four, for four FP64 adds per hop and warp. The FP64 pipe is far too slow
-// for the operator's multiply-adds, but it is otherwise idle here, and the
-// conversions it saves are integer work on the issue-bound FP32 side.
-// Each thread's four spinor components of the next hop are copied into
-// shared memory with cp.async while the current hop computes (two stages,
-// 128 bytes per thread), so the loads hold no registers.
-// (Measured on GB300, 24^3x48: 0.505 -> 0.440 ms per apply; unrolled hops
-// and the 47-bit split: 0.425 ms; staged loads: 0.417 ms. Moving more --
-// the epilogue, whole hops, or whole site groups -- onto the FP64 pipe was
-// slower.)
-// Block geometry, measured on GB300 at 24^3x48 (ms per apply, groups x
-// blocks per SM: registers): 4 x 3: 56 (spills) 0.372; 4 x 2: 80 0.379;
-// 3 x 4: 56 (spills) 0.376; 3 x 3: 72 0.364; 5 x 2: 64 0.391; 6 x 2: 56
-// 0.393; 2 x 5: 64 0.409; 2 x 6: 56 0.434; 1 x 10: 64 0.397; 1 x 12: 56
-// 0.395. The group barrier's id is a register, so ptxas reserves all 16
-// named barriers per block of more than one group, and ncu reports the
-// barriers as a limit of four resident blocks per SM. Immediate ids (a
-// warp-uniform switch over the groups) lift that limit but cost every form
-// 4-11 % (3 x 3: 0.406 ms; the branches sit in the unrolled hop loop).
-constexpr int kFFGroups = 3;       // groups of three warps (32 sites) per block
-constexpr int kFFMinBlocks = 3;    // resident blocks per SM the registers are sized for
-constexpr int kFFSites = 32 * kFFGroups;
-
-__device__ __forceinline__ void group_bar(int grp) { asm volatile("bar.sync %0, 96;" ::"r"(grp + 1) : "memory"); }
+// What bounds it: instruction issue and latency (about half of the issue slots
+// are taken), the FP64 pipe next. So the two spins of a half spinor are the
+// two halves of packed FP32 operations, which halves the issue slots of the
+// products and sums; a link entry is broadcast to both. The FP64 pipe does
+// only the spin projections (four adds per hop and warp: half the conversions
+// of splitting all components first) and one add per joined result. The two
+// hops of a direction are one loop body: four bodies of code stay in the
+// instruction cache, eight did not. Each thread's four spinor components of
+// the next hop are copied into shared memory with cp.async while the current
+// hop computes, so the loads hold no registers.
+// Measured on GB300 at 24^3 x 48, ms per apply: 0.366 with scalar operations
+// (298 M warp instructions), nine warps a block and eight unrolled hops; packed 0.350
+// (214 M); one body per direction 0.330; blocks of three warps 0.306; widening
+// by integer operations in the join 0.302; one range test per four splits and
+// per eight widenings, no negated packed operands and one barrier per hop
+// instead of two 0.275 (209 M, 61 % of the issue slots, FP64 pipe 47 %). One
+// thread per site (no exchange, 184 M warp instructions) holds 15 warps per SM
+// at 128 registers and ran at 0.402.
+constexpr int kFFSites = 32;
+constexpr int kFFThreads = 3 * kFFSites;
+constexpr int kFFMinBlocks = 7;  // resident blocks per SM the registers are sized for (8: 0.285, 9: 0.277, 10: 0.301 ms)
 
 // site of output index e; EO: the site of parity eo_par among full indices
 // 2e, 2e + 1 (even t extent)
 template <bool EO>
-__device__ __forceinline__ int ff_site(const DArgs &a, int e, bool act, int c[4])
+__device__ __forceinline__ int ff_site(const DArgs &a, int e, int c[4])
 {
-  c[0] = c[1] = c[2] = c[3] = 0;
-  if (!act) return e;
   if (EO) {
     coords(a.geo, 2 * e, c);
     const int b = (a.eo_par ^ c[1] ^ c[2] ^ c[3]) & 1;
@@ -284,196 +265,205 @@ __device__ __forceinline__ void cp_async_wait()
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// staging of the four spinor components a thread projects per hop: two
-// hops in flight, [stage][component][thread]
-constexpr int kFFThreads = 96 * kFFGroups;
-constexpr size_t kFFStageBytes = 2 * 4 * kFFThreads * sizeof(double2);
+__device__ __forceinline__ F2x2 fin2(FAx2 a)
+{
+  const float2 s = __fadd2_rn(a.s, a.e);
+  return F2x2{s, sub2(a.e, sub2(s, a.s))};
+}
+__device__ __forceinline__ FAx2 mul2(FAx2 a, float2 b) { return FAx2{__fmul2_rn(a.s, b), __fmul2_rn(a.e, b)}; }
+__device__ __forceinline__ F2x2 neg2(F2x2 a) { return F2x2{neg2(a.h), neg2(a.l)}; }
 
-// the float-float operator for one group's 32 sites; returns the thread's |out|^2.
-// AOS: in and out in the host layout (site-major, 12 double2 per site)
-template <bool DAG, bool EO, bool AOS>
-__device__ __forceinline__ double group_ff(const DArgs &a, int grp, int col, int lane, int e, bool act, int x,
-                                           const int c[4], CF (*hs)[2][3][32], double2 *stage)
+// out = epilogue of the accumulated hopping term, for the spin pair (2 P, 2 P + 1)
+template <int P, bool EO, bool AOS, bool SUMS>
+__device__ __forceinline__ void ff_store(const DArgs &a, int x, int e, int i, CAx2 acc, bool act, double &n2)
+{
+  const F2x2 mp4{dup2(a.mp4_h), dup2(a.mp4_l)};
+  const F2x2 tp{dup2(P ? -a.tm_h : a.tm_h), dup2(P ? -a.tm_l : a.tm_l)};
+  const int k0 = 6 * P + i, k1 = k0 + 3;
+  F2x2 hr = fin2(acc.re), hi = fin2(acc.im), dr, di;
+  if (EO) {
+    if (a.ainv) {  // (ai_r + i ai_i g5) H in
+      const F2x2 air{dup2(a.ai_r_h), dup2(a.ai_r_l)};
+      const F2x2 gi{dup2(P ? -a.ai_i_h : a.ai_i_h), dup2(P ? -a.ai_i_l : a.ai_i_l)};
+      FAx2 re = mac02(air, neg2(air.h), hr), im = mac02(air, neg2(air.h), hi);
+      mac2(re, neg2(gi), gi.h, hi);
+      mac2(im, gi, neg2(gi.h), hr);
+      hr = fin2(re);
+      hi = fin2(im);
+    }
+    const F2x2 ch{dup2(a.ch_h), dup2(a.ch_l)};
+    FAx2 re = mac02(ch, neg2(ch.h), hr), im = mac02(ch, neg2(ch.h), hi);
+    if (a.zmode) {
+      const double2 *z = (const double2 *)a.z;
+      const double2 z0 = __ldg(z + (int64_t)k0 * a.stride + e), z1 = __ldg(z + (int64_t)k1 * a.stride + e);
+      F2x2 zr, zi;
+      split_pair(z0, z1, zr, zi);
+      if (a.zmode == 2) {  // + (m+4) z + i tm g5 z
+        mac2(re, mp4, neg2(mp4.h), zr);
+        mac2(re, neg2(tp), tp.h, zi);
+        mac2(im, mp4, neg2(mp4.h), zi);
+        mac2(im, tp, neg2(tp.h), zr);
+      } else {
+        acc_add2(re, FAx2{zr.h, zr.l});
+        acc_add2(im, FAx2{zi.h, zi.l});
+      }
+    }
+    dr = fin2(re);
+    di = fin2(im);
+  } else {
+    // (m+4) psi + i tm g5 psi - acc / 2
+    const double2 *sp = (const double2 *)a.in;
+    const double2 s0 = __ldg(AOS ? sp + (int64_t)x * 12 + k0 : sp + (int64_t)k0 * a.stride + x);
+    const double2 s1 = __ldg(AOS ? sp + (int64_t)x * 12 + k1 : sp + (int64_t)k1 * a.stride + x);
+    F2x2 sr, si;
+    split_pair(s0, s1, sr, si);
+    FAx2 re = mul2(FAx2{hr.h, hr.l}, dup2(-0.5f)), im = mul2(FAx2{hi.h, hi.l}, dup2(-0.5f));
+    mac2(re, mp4, neg2(mp4.h), sr);
+    mac2(re, neg2(tp), tp.h, si);
+    mac2(im, mp4, neg2(mp4.h), si);
+    mac2(im, tp, neg2(tp.h), sr);
+    dr = fin2(re);
+    di = fin2(im);
+    if (a.op_q) {  // i g5: spins 0, 1 times i, spins 2, 3 times -i
+      const F2x2 t = dr;
+      dr = P ? di : neg2(di);
+      di = P ? neg2(t) : t;
+    }
+  }
+  double2 v0, v1;
+  join_pair(dr, di, v0, v1);
+  if (act) {
+    double2 *out = (double2 *)a.out;
+    const int o = EO ? e : x;
+    out[AOS ? (int64_t)o * 12 + k0 : (int64_t)k0 * a.stride + o] = v0;
+    out[AOS ? (int64_t)o * 12 + k1 : (int64_t)k1 * a.stride + o] = v1;
+    if (SUMS) n2 += v0.x * v0.x + v0.y * v0.y + v1.x * v1.x + v1.y * v1.y;
+  }
+}
+
+// the half spinors the three warps exchange, double-buffered by hop:
+// [hop & 1][colour][re, im][site], a pair's high words, then its low words
+typedef float4 FFShare[2][3][2][kFFSites];
+
+// the two hops of direction MU for one site and colour row col. The staged
+// components of hop (MU, back) are in stage `back`; the next hop's are
+// requested first (NEXT: the direction after MU, 4 when MU is the last).
+template <int MU, int NEXT, bool DAG, bool EO, bool AOS>
+__device__ __forceinline__ void ff_hops(const DArgs &a, int col, int lane, int x, const int c[4], FFShare &hs,
+                                        double2 *stage, CAx2 &up, CAx2 &lo)
 {
   const double2 *sp = (const double2 *)a.in;
-  const float4 *gf = (const float4 *)a.gauge;
-  constexpr int SF = DAG ? +1 : -1;
-  const int tid = threadIdx.x;
-  // the four components hop dd projects, copied into stage st
-  auto issue = [&](int dd, int st) {
-    if (act) {
-      const int mu2 = dd >> 1, y2 = ff_nb(a, x, c, mu2, dd & 1), ys2 = EO ? (y2 >> 1) : y2;
-      const int b02 = (mu2 == 0 || mu2 == 3) ? 2 : 3;
-      const int comp[4] = {col, 3 + col, 3 * b02 + col, 3 * (5 - b02) + col};
+  const float4 *gf = (const float4 *)a.gauge + (int64_t)MU * 9 * a.gstride;
+  constexpr bool odd = MU & 1;
+  constexpr int NB0 = (NEXT == 0 || NEXT == 3) ? 2 : 3, B0 = (MU == 0 || MU == 3) ? 2 : 3;
+#pragma unroll 1
+  for (int back = 0; back < 2; back++) {
+    if (NEXT < 4 || back == 0) {
+      const int yn = back ? ff_nb(a, x, c, NEXT & 3, false) : ff_nb(a, x, c, MU, true), ys = EO ? (yn >> 1) : yn;
+      const int b0 = back ? NB0 : B0;
+      double2 *to = stage + (back ^ 1) * 4 * kFFThreads;
+      const int comp[4] = {col, 3 + col, 3 * b0 + col, 3 * (5 - b0) + col};
 #pragma unroll
       for (int i = 0; i < 4; i++)
-        cp_async16(stage + (st * 4 + i) * kFFThreads + tid,
-                   AOS ? sp + (int64_t)ys2 * 12 + comp[i] : sp + (int64_t)comp[i] * a.stride + ys2);
-    }
-    cp_async_commit();
-  };
-  issue(0, 0);
-  CA acc[4];
-#pragma unroll
-  for (int s = 0; s < 4; s++) acc[s] = CA{{0.f, 0.f}, {0.f, 0.f}};
-#pragma unroll
-  for (int d = 0; d < 8; d++) {
-    // hop d + 1's components start to arrive while hop d computes
-    if (d < 7) {
-      issue(d + 1, (d + 1) & 1);
+        cp_async16(to + i * kFFThreads, AOS ? sp + (int64_t)ys * 12 + comp[i] : sp + (int64_t)comp[i] * a.stride + ys);
+      cp_async_commit();
       cp_async_wait<1>();
     } else {
       cp_async_wait<0>();
     }
-    const int mu = d >> 1;
-    const bool back = d & 1;
-    const int S = back ? -SF : SF;
-    const int y = act ? ff_nb(a, x, c, mu, back) : x;
-    const int ly = back ? y : x;
-    const bool odd = mu & 1;
-    const bool neg0 = S > 0, neg1 = mu < 2 ? S > 0 : S < 0;
-    double2 d0 = make_double2(0.0, 0.0), d1 = d0;
-    if (act) {
-      const double2 *b = stage + (d & 1) * 4 * kFFThreads + tid;  // this thread's own copies
-      const double2 p0 = b[0], p1 = b[kFFThreads], q0 = b[2 * kFFThreads], q1 = b[3 * kFFThreads];
-      d0 = dadd(p0, dcoef(q0, odd, neg0));
-      d1 = dadd(p1, dcoef(q1, odd, neg1));
+    // projector sign S > 0: forward for D^+, backward for D
+    const bool pos = (back != 0) != DAG;
+    const bool neg0 = pos, neg1 = MU < 2 ? pos : !pos;
+    const double2 *b = stage + back * 4 * kFFThreads;  // this thread's own copies
+    {
+      const double2 d0 = dadd(b[0], dcoef(b[2 * kFFThreads], odd, neg0));
+      const double2 d1 = dadd(b[kFFThreads], dcoef(b[3 * kFFThreads], odd, neg1));
+      F2x2 r, i;
+      split_pair(d0, d1, r, i);
+      hs[back][col][0][lane] = make_float4(r.h.x, r.h.y, r.l.x, r.l.y);
+      hs[back][col][1][lane] = make_float4(i.h.x, i.h.y, i.l.x, i.l.y);
     }
-    hs[grp][0][col][lane] = CF{split_d(d0.x), split_d(d0.y)};
-    hs[grp][1][col][lane] = CF{split_d(d1.x), split_d(d1.y)};
-    group_bar(grp);
-    CA u0, u1;
+    // forward: U[col][k] at x; backward: conj(U[k][col]) at the neighbour
+    const int lx = back ? ff_nb(a, x, c, MU, true) : x;
+    const int64_t si = back ? a.gstride : 3 * a.gstride, sk = back ? 3 * a.gstride : a.gstride;
+    const unsigned cj = back ? 0x80000000u : 0u;
+    float4 wl[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) wl[k] = __ldg(gf + lx + col * si + k * sk);
+    __syncthreads();
+    CAx2 u;  // U h for the two half-spinor components
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-      CF g0 = hs[grp][0][k][lane], g1 = hs[grp][1][k][lane];
-      // forward: U[col][k]; backward: conj(U[k][col])
-      CF wl = act ? load_link(gf, a.gstride, ly, mu, back ? 3 * k + col : 3 * col + k) : CF{{0.f, 0.f}, {0.f, 0.f}};
-      F2 wr = wl.re, wi = back ? neg(wl.im) : wl.im, mwi = neg(wi);
+      const float4 gr = hs[back][k][0][lane], gi = hs[back][k][1][lane];
+      const F2x2 hr{make_float2(gr.x, gr.y), make_float2(gr.z, gr.w)}, hi{make_float2(gi.x, gi.y), make_float2(gi.z, gi.w)};
+      float4 w = wl[k];
+      w.z = __uint_as_float(__float_as_uint(w.z) ^ cj);
+      w.w = __uint_as_float(__float_as_uint(w.w) ^ cj);
+      const F2x2 wr{dup2(w.x), dup2(w.y)}, wp{dup2(w.z), dup2(w.w)}, wm{dup2(-w.z), dup2(-w.w)};
+      const float2 nwr = dup2(-w.x);
       if (k == 0) {
-        u0.re = mac0(wr, g0.re);
-        u0.im = mac0(wr, g0.im);
-        u1.re = mac0(wr, g1.re);
-        u1.im = mac0(wr, g1.im);
+        u.re = mac02(wr, nwr, hr);
+        u.im = mac02(wr, nwr, hi);
       } else {
-        mac(u0.re, wr, g0.re);
-        mac(u0.im, wr, g0.im);
-        mac(u1.re, wr, g1.re);
-        mac(u1.im, wr, g1.im);
+        mac2(u.re, wr, nwr, hr);
+        mac2(u.im, wr, nwr, hi);
       }
-      mac(u0.re, mwi, g0.im);
-      mac(u0.im, wi, g0.re);
-      mac(u1.re, mwi, g1.im);
-      mac(u1.im, wi, g1.re);
+      mac2(u.re, wm, wp.h, hi);
+      mac2(u.im, wp, wm.h, hr);
     }
-    // the products enter the spinor accumulators unnormalised (the first
-    // hop assigns them)
-    const CFA v0{u0.re, u0.im}, v1{u1.re, u1.im};
-    const bool jA = (mu == 1 || mu == 2);
-    const bool negA = mu == 0 ? S > 0 : S < 0, negB = mu == 1 ? S < 0 : S > 0;
-    const CFA l2 = coefa(jA ? v1 : v0, odd, negA), l3 = coefa(jA ? v0 : v1, odd, negB);
-    if (d == 0) {
-      acc[0] = CA{v0.re, v0.im};
-      acc[1] = CA{v1.re, v1.im};
-      acc[2] = CA{l2.re, l2.im};
-      acc[3] = CA{l3.re, l3.im};
+    // the products enter the spinor accumulators unnormalised. Lower spins:
+    // sign pairs of (spin 2, spin 3) for MU 0, 3; (3, 2) for 1, 2
+    const float S = pos ? 1.f : -1.f;
+    const float2 sg = MU == 0 ? make_float2(-S, -S) : MU == 1 ? make_float2(S, S) : MU == 2 ? make_float2(-S, S)
+                                                                                            : make_float2(S, -S);
+    acc_add2(up.re, u.re);
+    acc_add2(up.im, u.im);
+    if (odd) {  // times i
+      acc_add2(lo.re, mul2(u.im, neg2(sg)));
+      acc_add2(lo.im, mul2(u.re, sg));
     } else {
-      cacc_fa(acc[0], v0);
-      cacc_fa(acc[1], v1);
-      cacc_fa(acc[2], l2);
-      cacc_fa(acc[3], l3);
-    }
-    group_bar(grp);  // hs is rewritten by the next hop
-  }
-  if (!act) return 0.0;
-  double n2 = 0.0;
-  if (EO) {
-    double2 *out = (double2 *)a.out;
-    const F2 mp4{a.mp4_h, a.mp4_l}, tm{a.tm_h, a.tm_l}, ch{a.ch_h, a.ch_l};
-    const F2 air{a.ai_r_h, a.ai_r_l}, aii{a.ai_i_h, a.ai_i_l};
-#pragma unroll
-    for (int s = 0; s < 4; s++) {
-      const int k = 3 * s + col;
-      F2 hr = fin(acc[s].re), hi = fin(acc[s].im);
-      if (a.ainv) {  // (ai_r + i ai_i g5) H in
-        const F2 gi = s < 2 ? aii : neg(aii);
-        FA re{0.f, 0.f}, im{0.f, 0.f};
-        mac(re, air, hr);
-        mac(re, neg(gi), hi);
-        mac(im, air, hi);
-        mac(im, gi, hr);
-        hr = fin(re);
-        hi = fin(im);
-      }
-      FA re{0.f, 0.f}, im{0.f, 0.f};
-      mac(re, ch, hr);
-      mac(im, ch, hi);
-      if (a.zmode) {
-        const CF zv = load_sp((const double2 *)a.z, a.stride, e, k);
-        if (a.zmode == 2) {  // + (m+4) z + i tm g5 z
-          const F2 g5tm = s < 2 ? tm : neg(tm);
-          mac(re, mp4, zv.re);
-          mac(re, neg(g5tm), zv.im);
-          mac(im, mp4, zv.im);
-          mac(im, g5tm, zv.re);
-        } else {
-          acc_add(re, zv.re);
-          acc_add(im, zv.im);
-        }
-      }
-      const double vr = join_d(fin(re)), vi = join_d(fin(im));
-      out[(int64_t)k * a.stride + e] = make_double2(vr, vi);
-      n2 += vr * vr + vi * vi;
-    }
-  } else {
-    double2 *out = (double2 *)a.out;
-    const F2 mp4{a.mp4_h, a.mp4_l}, tm{a.tm_h, a.tm_l};
-#pragma unroll
-    for (int s = 0; s < 4; s++) {
-      // (m+4) psi + i tm g5 psi - acc/2 for component (spin s, colour col)
-      const int k = 3 * s + col;
-      CF sv = AOS ? load_sp(sp + (int64_t)x * 12, 1, 0, k) : load_sp(sp, a.stride, x, k);
-      F2 g5tm = s < 2 ? tm : neg(tm), mg5tm = neg(g5tm);
-      F2 ar = fin(acc[s].re), ai = fin(acc[s].im);
-      FA re{__fmul_rn(ar.h, -0.5f), __fmul_rn(ar.l, -0.5f)};
-      FA im{__fmul_rn(ai.h, -0.5f), __fmul_rn(ai.l, -0.5f)};
-      mac(re, mp4, sv.re);
-      mac(re, mg5tm, sv.im);
-      mac(im, mp4, sv.im);
-      mac(im, g5tm, sv.re);
-      F2 dr = fin(re), di = fin(im);
-      if (a.op_q) {  // i g5: spins 0,1 times i, spins 2,3 times -i
-        F2 t = dr;
-        if (s < 2) {
-          dr = neg(di);
-          di = t;
-        } else {
-          dr = di;
-          di = neg(t);
-        }
-      }
-      double vr = join_d(dr), vi = join_d(di);
-      out[AOS ? (int64_t)x * 12 + k : (int64_t)k * a.stride + x] = make_double2(vr, vi);
-      n2 += vr * vr + vi * vi;
+      acc_add2(lo.re, mul2(u.re, sg));
+      acc_add2(lo.im, mul2(u.im, sg));
     }
   }
-  return n2;
 }
 
 // EO: even/odd kernel on half fields (sites of parity a.eo_par; neighbours
-// read at (full index) >> 1) with the epilogue ch * [A^{-1}] H in + {z | A z}
-template <bool DAG, bool EO, bool AOS>
+// read at (full index) >> 1) with the epilogue ch * [A^{-1}] H in + {z | A z};
+// SUMS: with the block sums of |out|^2 (a.partials)
+template <bool DAG, bool EO, bool AOS, bool SUMS>
 __global__ void __launch_bounds__(kFFThreads, kFFMinBlocks) k_wilson_ff(const DArgs a)
 {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int grp = w / 3, col = w - 3 * grp;
-  const int e = a.x0 + blockIdx.x * kFFSites + grp * 32 + lane;  // output index
-  const bool act = e < a.V;
-  __shared__ CF hs[kFFGroups][2][3][32];
+  const int lane = threadIdx.x & 31, col = threadIdx.x >> 5;
+  const int id = a.x0 + blockIdx.x * kFFSites + lane;  // output index
+  const bool act = id < a.V;
+  const int e = act ? id : a.V - 1;  // idle lanes repeat the last site
+  __shared__ FFShare hs;
+  __shared__ double2 staging[2 * 4 * kFFThreads];  // [hop & 1][component][thread]
   int c[4];
-  const int x = ff_site<EO>(a, e, act, c);
-  extern __shared__ double2 ff_stage[];
-  const double n2 = group_ff<DAG, EO, AOS>(a, grp, col, lane, e, act, x, c, hs, ff_stage);
-  if (a.partials) block_partial_cg(n2, a);
+  const int x = ff_site<EO>(a, e, c);
+  double2 *stage = staging + threadIdx.x;
+  {
+    const double2 *sp = (const double2 *)a.in;
+    const int y = ff_nb(a, x, c, 0, false), ys = EO ? (y >> 1) : y;
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+      cp_async16(stage + i * kFFThreads,
+                 AOS ? sp + (int64_t)ys * 12 + 3 * i + col : sp + (int64_t)(3 * i + col) * a.stride + ys);
+    cp_async_commit();
+  }
+  const float2 z = make_float2(0.f, 0.f);
+  CAx2 up{FAx2{z, z}, FAx2{z, z}}, lo = up;
+  ff_hops<0, 3, DAG, EO, AOS>(a, col, lane, x, c, hs, stage, up, lo);
+  ff_hops<3, 1, DAG, EO, AOS>(a, col, lane, x, c, hs, stage, up, lo);
+  lo = CAx2{flip2(lo.re), flip2(lo.im)};
+  ff_hops<1, 2, DAG, EO, AOS>(a, col, lane, x, c, hs, stage, up, lo);
+  ff_hops<2, 4, DAG, EO, AOS>(a, col, lane, x, c, hs, stage, up, lo);
+  lo = CAx2{flip2(lo.re), flip2(lo.im)};
+  double n2 = 0.0;
+  ff_store<0, EO, AOS, SUMS>(a, x, e, col, up, act, n2);
+  ff_store<1, EO, AOS, SUMS>(a, x, e, col, lo, act, n2);
+  if (SUMS) block_partial_cg(n2, a);
 }
 
 // ------------------------------------------------------ float-pair links
@@ -524,32 +514,29 @@ bool gauge_to_ff(qcdgpu_gauge d, qcdgpu_gauge s)
   return QG_LAUNCHED("gauge_to_ff");
 }
 
-// the staging buffer is dynamic shared memory (36 KB for three groups; the
-// attribute lifts the 48 KB default limit for larger blocks): opted in once
-// per instantiation
-template <bool D, bool E, bool A = false>
-static void launch_ff(const DArgs &a, unsigned grid)
+template <bool D, bool E, bool A, bool P>
+static void launch_ff(const DArgs &a)
 {
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(k_wilson_ff<D, E, A>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFFStageBytes);
-    attr = true;
-  }
-  k_wilson_ff<D, E, A><<<grid, kFFThreads, kFFStageBytes, stream()>>>(a);
+  k_wilson_ff<D, E, A, P><<<(unsigned)((a.V - a.x0 + kFFSites - 1) / kFFSites), kFFThreads, 0, stream()>>>(a);
 }
+
+int64_t dslash_df64_blocks(int64_t V) { return (V + kFFSites - 1) / kFFSites; }
 
 bool dslash_df64(const DArgs &a, bool dag, bool eo)
 {
-  unsigned grid = (unsigned)((a.V - a.x0 + kFFSites - 1) / kFFSites);
-  if (eo) {
-    if (dag) launch_ff<true, true>(a, grid);
-    else launch_ff<false, true>(a, grid);
-  } else if (a.aos) {
-    if (dag) launch_ff<true, false, true>(a, grid);
-    else launch_ff<false, false, true>(a, grid);
+  if (a.aos) {
+    if (dag) launch_ff<true, false, true, false>(a);
+    else launch_ff<false, false, true, false>(a);
+  } else if (a.partials) {
+    if (dag && eo) launch_ff<true, true, false, true>(a);
+    else if (dag) launch_ff<true, false, false, true>(a);
+    else if (eo) launch_ff<false, true, false, true>(a);
+    else launch_ff<false, false, false, true>(a);
   } else {
-    if (dag) launch_ff<true, false>(a, grid);
-    else launch_ff<false, false>(a, grid);
+    if (dag && eo) launch_ff<true, true, false, false>(a);
+    else if (dag) launch_ff<true, false, false, false>(a);
+    else if (eo) launch_ff<false, true, false, false>(a);
+    else launch_ff<false, false, false, false>(a);
   }
   return QG_LAUNCHED("wilson_df64");
 }
