@@ -78,6 +78,10 @@ __device__ __noinline__ F2Quad split_slow(double2 a, double2 b)
   };
   return F2Quad{one(a.x), one(a.y), one(b.x), one(b.y)};
 }
+__device__ __forceinline__ bool is_zero(double2 a)
+{
+  return (((__double2hiint(a.x) | __double2hiint(a.y)) & 0x7fffffff) | __double2loint(a.x) | __double2loint(a.y)) == 0;
+}
 // exponent distance above 2^-74 (in units of the exponent field)
 __device__ __forceinline__ unsigned split_range(double d)
 {
@@ -154,6 +158,8 @@ __device__ __forceinline__ void split_pair(double2 a, double2 b, F2x2 &re, F2x2 
   F2Quad q;
   if (max(max(split_range(a.x), split_range(a.y)), max(split_range(b.x), split_range(b.y))) <= (201u << 20))
     q = F2Quad{split_d(a.x), split_d(a.y), split_d(b.x), split_d(b.y)};
+  else if (is_zero(a) && is_zero(b))  // empty sites of sources and first iterates
+    q = F2Quad{};
   else
     q = split_slow(a, b);
   re = F2x2{make_float2(q.ar.h, q.br.h), make_float2(q.ar.l, q.br.l)};
