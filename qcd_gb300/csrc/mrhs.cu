@@ -1,12 +1,11 @@
 // mrhs.cu -- many right-hand sides sharing one gauge-field read.
 //
 // A multi-RHS field holds N spinors in FP16 with one float norm per
-// (site, RHS), laid out [component 0..11][site][rhs] as half2 (re, im), so
-// the RHS of one site and component are contiguous.
+// (site, RHS), slot after slot in the layout of an FP16 field (mrhs.h).
 //
-// Operator: three kernels, picked per (volume, slot count) by timing. SIMT:
-// one thread per site and one or two slots, links shared through L1.
-// tcgen05: one FP16 GEMM per site with the eight hops concatenated along K
+// Operator: three kernels. SIMT, the one that runs unless another is asked
+// for: one thread per site and two slots, links shared through L1, its block
+// size picked per (volume, slot count) by timing. tcgen05: one FP16 GEMM per site with the eight hops concatenated along K
 // (see k_wilson_mrhs_tc). mma.sync (below): one warp per site. For each of
 // the eight hops the warp builds, for 16 RHS at a time, the matrix A (16 RHS x 12 reals of the
 // projected half spinor, padded to 16) and multiplies it with
@@ -39,6 +38,7 @@ struct MArgs {
   const float2 *gauge;  // FP32, 4 mu x 9 float2 blocks
   Geom geo;
   int V, N, nact;
+  int64_t stride;  // block stride of the fields
   int64_t gstride;
   float phr[4], phi[4];
   int twist_mask;
@@ -56,10 +56,10 @@ struct MArgs {
   float ch;
 };
 
-__device__ __forceinline__ float2 mload(const __half2 *d, const float *nrm, int V, int N, int k, int site, int r)
+__device__ __forceinline__ float2 mload(const __half2 *d, const float *nrm, int64_t S, int k, int site, int r)
 {
-  float2 f = __half22float2(d[mhalf2_index(V, N, k, site, r)]);
-  float s = nrm[(int64_t)site * N + r];
+  float2 f = __half22float2(d[mhalf2_index(S, k, site, r)]);
+  float s = nrm[mnorm_at(S, site, r)];
   return make_float2(f.x * s, f.y * s);
 }
 
@@ -174,8 +174,8 @@ __global__ void __launch_bounds__(128) k_wilson_mrhs(const MArgs a)
           const int kk = t + 4 * q, j = kk / 6, cc = (kk % 6) >> 1;
           float val = 0.f;
           if (r < a.nact) {
-            float2 p = mload(a.in, a.in_norm, a.V, a.N, 3 * j + cc, y, r);
-            float2 pb = mload(a.in, a.in_norm, a.V, a.N, 3 * (j == 0 ? b0 : b1) + cc, y, r);
+            float2 p = mload(a.in, a.in_norm, a.stride, 3 * j + cc, y, r);
+            float2 pb = mload(a.in, a.in_norm, a.stride, 3 * (j == 0 ? b0 : b1) + cc, y, r);
             if (odd) pb = make_float2(-pb.y, pb.x);
             if (j == 0 ? neg0 : neg1) pb = make_float2(-pb.x, -pb.y);
             val = (t & 1) ? p.y + pb.y : p.x + pb.x;
@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(128) k_wilson_mrhs(const MArgs a)
       for (int nt = 0; nt < 3; nt++) {
         const int q = 4 * nt + t, s = q / 3;
         float2 cq = make_float2(acc[m][nt][2 * row], acc[m][nt][2 * row + 1]);
-        float2 ps = live ? mload(a.in, a.in_norm, a.V, a.N, q, x, r) : make_float2(0.f, 0.f);
+        float2 ps = live ? mload(a.in, a.in_norm, a.stride, q, x, r) : make_float2(0.f, 0.f);
         const float g5tm = s < 2 ? tmr : -tmr;
         o[nt] = make_float2(mp4r * ps.x - g5tm * ps.y - 0.5f * cq.x, mp4r * ps.y + g5tm * ps.x - 0.5f * cq.y);
         mx = fmaxf(mx, fmaxf(fabsf(o[nt].x), fabsf(o[nt].y)));
@@ -221,40 +221,35 @@ __global__ void __launch_bounds__(128) k_wilson_mrhs(const MArgs a)
 #pragma unroll
         for (int nt = 0; nt < 3; nt++) {
           const int q = 4 * nt + t;
-          a.out[mhalf2_index(a.V, a.N, q, x, r)] = __floats2half2_rn(o[nt].x * inv, o[nt].y * inv);
+          a.out[mhalf2_index(a.stride, q, x, r)] = __floats2half2_rn(o[nt].x * inv, o[nt].y * inv);
         }
-        if (t == 0) a.out_norm[(int64_t)x * a.N + r] = mx;
+        if (t == 0) a.out_norm[mnorm_at(a.stride, x, r)] = mx;
       }
     }
 }
 
 // ------------------------------------------------ SIMT variant (FP32 cores)
-// One thread per site and RP adjacent RHS slots, block (N / RP threads, SB
-// sites): the threads of one site read the same links (L1 broadcast), so
-// the gauge field is fetched once per site for all RHS, while the per-RHS
-// spin projection, link products and reconstruction run as FP32 FMAs. With
-// RP = 2 a thread loads the two slots' half2 values of a component as one
-// 8-byte word and applies each link it loads to both. With `partials` the
-// epilogue also writes, per block and slot, the sum of |out|^2 over the
-// block's sites (partials[block * N + slot]) in a fixed order.
-template <int RP>
-__device__ __forceinline__ void mload_rp(const MArgs &a, const __half2 *d, const float *dn, int y, int r0,
-                                         C<float> s[RP][12], float nrm[RP])
+// One thread per site and two adjacent RHS slots; a warp takes 32 consecutive
+// sites of a slot pair, the warps of a block the same sites of several pairs:
+// each link a thread loads serves two slots, and the block's pairs meet in L1
+// for it, while the per-RHS spin projection, link products and reconstruction
+// run as FP32 FMAs. With `partials` the epilogue also writes, per 32 sites
+// (blockIdx.x) and slot, the sum of |out|^2 (partials[block * N + slot]) in a
+// fixed order that does not depend on the occupied slots.
+// Bound by instruction issue and FP32 arithmetic like the single-RHS FP16
+// kernel: 24^3 x 48, 16 slots, 0.637 ms (39.8 us a slot against 47.1). Packed
+// FP32 operations over the two slots (links stored twice, since a broadcast
+// costs two moves) needed more registers than they freed and took 0.74 ms.
+
+// spinor and norm of slot r at y
+__device__ __forceinline__ void mload_slot(const MArgs &a, const __half2 *d, const float *dn, int y, int r,
+                                           C<float> s[12], float &nrm)
 {
-  if (RP == 2) {
-    const float2 n2 = *(const float2 *)(dn + (int64_t)y * a.N + r0);
-    nrm[0] = n2.x;
-    nrm[RP - 1] = n2.y;
-  } else {
-    nrm[0] = dn[(int64_t)y * a.N + r0];
-  }
+  nrm = dn[mnorm_at(a.stride, y, r)];
+  float2 v[12];
+  mload_raw(d, a.stride, y, r, v);
 #pragma unroll
-  for (int q = 0; q < RP; q++) {
-    float2 v[12];
-    mload_raw(d, a.V, a.N, y, r0 + q, v);
-#pragma unroll
-    for (int k = 0; k < 12; k++) s[q][k] = C<float>{v[k].x, v[k].y};
-  }
+  for (int k = 0; k < 12; k++) s[k] = C<float>{v[k].x, v[k].y};
 }
 
 // h = upper half of (1 + S g_mu) s for the spinor s held as its three
@@ -276,74 +271,54 @@ __device__ __forceinline__ void project_words(const uint4 w[3], C<float> h[6])
   }
 }
 
-// the same for slot r of the multi-RHS spinor at y
-template <int MU, int S>
-__device__ __forceinline__ void mload_project(const __half2 *d, int64_t V, int N, int y, int r, C<float> h[6])
-{
-  const uint4 *p = (const uint4 *)d;
-  uint4 w[3];
-#pragma unroll
-  for (int j = 0; j < 3; j++) w[j] = p[((int64_t)j * V + y) * N + r];
-  project_words<MU, S>(w, h);
-}
+// two adjacent slots of a field: the first one's words and norms, and how far
+// the second one's lie (in words; four floats each)
+struct SlotPair {
+  const uint4 *w;
+  const float *n;
+  int64_t next;
+};
 
-template <int MU, bool DAG, int RP, bool EO>
-__device__ __forceinline__ void mhop_pair(const MArgs &a, int x, const int c[4], int r0, C<float> acc[RP][12])
+template <int MU, bool BACK, bool DAG, bool EO>
+__device__ __forceinline__ void mhop(const MArgs &a, const SlotPair &in, int x, const int c[4], C<float> acc[2][12])
 {
-  constexpr int SF = DAG ? +1 : -1;
-  const bool twisted = (a.twist_mask >> MU) & 1;
+  constexpr int S = (DAG ? 1 : -1) * (BACK ? -1 : 1);  // projector sign
+  const int y = BACK ? bwd(a.geo, x, c, MU) : fwd(a.geo, x, c, MU);
+  const int ys = EO ? (y >> 1) : y;
+  C<float> U[9];
+  Link<QCDGPU_F32, 18, float>::load(a.gauge, a.gstride, BACK ? y : x, MU, U);
 #pragma unroll
-  for (int dir = 0; dir < 2; dir++) {
-    const bool back = dir == 1;
-    const int y = back ? bwd(a.geo, x, c, MU) : fwd(a.geo, x, c, MU);
-    C<float> U[9];
-    const int ys = EO ? (y >> 1) : y;
-    float nrm[RP];
-    if (RP == 2) {
-      const float2 n2 = *(const float2 *)(a.in_norm + (int64_t)ys * a.N + r0);
-      nrm[0] = n2.x;
-      nrm[RP - 1] = n2.y;
-    } else {
-      nrm[0] = a.in_norm[(int64_t)ys * a.N + r0];
-    }
-    Link<QCDGPU_F32, 18, float>::load(a.gauge, a.gstride, back ? y : x, MU, U);
+  for (int q = 0; q < 2; q++) {
+    // the projection adds the stored half pairs, then the six projected
+    // components are converted; the slot's site norm scales the accumulation
+    const uint4 *p = in.w + q * in.next + ys;
+    const float nrm = __ldg(in.n + q * 4 * in.next + ys);
+    uint4 w[3];
 #pragma unroll
-    for (int q = 0; q < RP; q++) {
-      C<float> h[6], uh[6];
-      // the projection adds the stored half pairs, then the six projected
-      // components are converted; the slot's site norm scales the accumulation
-      if (back) mload_project<MU, -SF>(a.in, a.V, a.N, ys, r0 + q, h);
-      else mload_project<MU, SF>(a.in, a.V, a.N, ys, r0 + q, h);
+    for (int j = 0; j < 3; j++) w[j] = __ldg(p + j * a.stride);
+    C<float> h[6], uh[6];
+    project_words<MU, S>(w, h);
 #pragma unroll
-      for (int j = 0; j < 2; j++)
+    for (int j = 0; j < 2; j++)
 #pragma unroll
-        for (int i = 0; i < 3; i++)
-          uh[3 * j + i] =
-              back ? cmadd_conj(U[6 + i], h[3 * j + 2], cmadd_conj(U[3 + i], h[3 * j + 1], cdot(U[i], h[3 * j])))
-                   : cmadd(U[3 * i + 2], h[3 * j + 2], cmadd(U[3 * i + 1], h[3 * j + 1], U[3 * i] * h[3 * j]));
-      if (twisted) {
-        C<float> ph{a.phr[MU], back ? -a.phi[MU] : a.phi[MU]};
-#pragma unroll
-        for (int k = 0; k < 6; k++) uh[k] = uh[k] * ph;
-      }
-      if (back) accumulate_scaled<MU, -SF>(acc[q], uh, nrm[q]);
-      else accumulate_scaled<MU, SF>(acc[q], uh, nrm[q]);
-    }
+      for (int i = 0; i < 3; i++)
+        uh[3 * j + i] =
+            BACK ? cmadd_conj(U[6 + i], h[3 * j + 2], cmadd_conj(U[3 + i], h[3 * j + 1], cdot(U[i], h[3 * j])))
+                 : cmadd(U[3 * i + 2], h[3 * j + 2], cmadd(U[3 * i + 1], h[3 * j + 1], U[3 * i] * h[3 * j]));
+    accumulate_scaled<MU, S>(acc[q], uh, nrm);
   }
 }
 
 // MODE 0: full lattice, out = A in - H in / 2. Even/odd (half fields): MODE 1
 // out = A^{-1} H in; MODE 2 out = A z - H in / 4 (the two halves of the Schur
 // complement). The epilogue is fixed at compile time for each mode.
-template <bool DAG, int RP, int MODE>
+template <bool DAG, int MODE>
 __global__ void __launch_bounds__(256, 2) k_wilson_mrhs_simt(const MArgs a, double *partials)
 {
   constexpr bool EO = MODE != 0;
-  const int r0 = threadIdx.x * RP;
-  const int e = blockIdx.x * blockDim.y + threadIdx.y;  // output index
-  double n2[RP];
-#pragma unroll
-  for (int q = 0; q < RP; q++) n2[q] = 0.0;
+  const int r0 = 2 * (blockIdx.y * blockDim.y + threadIdx.y);
+  const int e = blockIdx.x * 32 + threadIdx.x;  // output index
+  double n2[2] = {0.0, 0.0};
   if (r0 < a.nact && e < a.V) {
     int c[4], x = e;
     if (EO) {  // the site of parity eo_par among full indices 2e, 2e + 1 (even t extent)
@@ -354,23 +329,25 @@ __global__ void __launch_bounds__(256, 2) k_wilson_mrhs_simt(const MArgs a, doub
     } else {
       coords(a.geo, x, c);
     }
-    C<float> acc[RP][12];
+    const SlotPair in{(const uint4 *)a.in + mword(a.stride, 0, 0, r0), a.in_norm + mnorm_at(a.stride, 0, r0),
+                      mword(a.stride, 0, 0, 1)};
+    C<float> acc[2][12];
 #pragma unroll
-    for (int q = 0; q < RP; q++)
+    for (int q = 0; q < 2; q++)
 #pragma unroll
       for (int k = 0; k < 12; k++) acc[q][k] = C<float>{0.f, 0.f};
-    mhop_pair<0, DAG, RP, EO>(a, x, c, r0, acc);
-    mhop_pair<1, DAG, RP, EO>(a, x, c, r0, acc);
-    mhop_pair<2, DAG, RP, EO>(a, x, c, r0, acc);
-    mhop_pair<3, DAG, RP, EO>(a, x, c, r0, acc);
-    constexpr int zmode = MODE == 1 ? 0 : 2;
+    mhop<0, false, DAG, EO>(a, in, x, c, acc);
+    mhop<0, true, DAG, EO>(a, in, x, c, acc);
+    mhop<1, false, DAG, EO>(a, in, x, c, acc);
+    mhop<1, true, DAG, EO>(a, in, x, c, acc);
+    mhop<2, false, DAG, EO>(a, in, x, c, acc);
+    mhop<2, true, DAG, EO>(a, in, x, c, acc);
+    mhop<3, false, DAG, EO>(a, in, x, c, acc);
+    mhop<3, true, DAG, EO>(a, in, x, c, acc);
     constexpr bool ainv = MODE == 1;
     constexpr float ch = MODE == 0 ? -0.5f : MODE == 1 ? 1.0f : -0.25f;
-    C<float> s[RP][12];
-    float nrm[RP];
-    if (zmode) mload_rp<RP>(a, EO ? a.z : a.in, EO ? a.z_norm : a.in_norm, e, r0, s, nrm);
 #pragma unroll
-    for (int q = 0; q < RP; q++) {
+    for (int q = 0; q < 2; q++) {
       const int r = r0 + q;
       // slots past nact hold zeros; their results are not stored
       const float mp4r = a.mp4s ? a.mp4s[r] : a.mp4;
@@ -385,12 +362,14 @@ __global__ void __launch_bounds__(256, 2) k_wilson_mrhs_simt(const MArgs a, doub
           mx = fmaxf(mx, fmaxf(fabsf(acc[q][k].re), fabsf(acc[q][k].im)));
         }
       } else {  // ch H in + A z
-        const float zs = nrm[q];
-        const float zm = zmode == 2 ? mp4r * zs : zs, zt = zmode == 2 ? tmr * zs : 0.f;
+        C<float> s[12];
+        float zs;
+        mload_slot(a, EO ? a.z : a.in, EO ? a.z_norm : a.in_norm, e, r, s, zs);
+        const float zm = mp4r * zs, zt = tmr * zs;
 #pragma unroll
         for (int k = 0; k < 12; k++) {
           const float g5tm = k < 6 ? zt : -zt;
-          const C<float> zk = s[q][k];
+          const C<float> zk = s[k];
           acc[q][k] = C<float>{qfma(ch, acc[q][k].re, qfma(-g5tm, zk.im, zm * zk.re)),
                                qfma(ch, acc[q][k].im, qfma(g5tm, zk.re, zm * zk.im))};
           mx = fmaxf(mx, fmaxf(fabsf(acc[q][k].re), fabsf(acc[q][k].im)));
@@ -402,7 +381,7 @@ __global__ void __launch_bounds__(256, 2) k_wilson_mrhs_simt(const MArgs a, doub
         float2 o[12];
 #pragma unroll
         for (int k = 0; k < 12; k++) o[k] = make_float2(acc[q][k].re, acc[q][k].im);
-        mstore_raw(a.out, a.V, a.N, e, r, o, inv);
+        mstore_raw(a.out, a.stride, e, r, o, inv);
         float s2 = 0.f;
         if (partials) {  // |out|^2 of the stored (rounded) values
 #pragma unroll
@@ -411,26 +390,18 @@ __global__ void __launch_bounds__(256, 2) k_wilson_mrhs_simt(const MArgs a, doub
             s2 += f.x * f.x + f.y * f.y;
           }
         }
-        a.out_norm[(int64_t)e * a.N + r] = mx;
+        a.out_norm[mnorm_at(a.stride, e, r)] = mx;
         n2[q] = (double)(s2 * mx * mx);  // per-site sum in FP32, block sum in double
       }
     }
   }
   if (partials) {
-    // the block covers slots 0 .. NS-1 (the occupied ones); partials keep
-    // the field's slot stride N
-    extern __shared__ double sh[];
-    const int N = a.N, y = threadIdx.y, NS = min(N, (int)blockDim.x * RP);
 #pragma unroll
-    for (int q = 0; q < RP; q++)
-      if (threadIdx.x * RP + q < NS) sh[y * NS + threadIdx.x * RP + q] = n2[q];
-    __syncthreads();
-    for (int r = threadIdx.x; r < NS; r += blockDim.x)
-      if (y == 0) {
-        double t = 0.0;
-        for (int i = 0; i < (int)blockDim.y; i++) t += sh[i * NS + r];
-        partials[(int64_t)blockIdx.x * N + r] = t;
-      }
+    for (int q = 0; q < 2; q++) {
+      double t = n2[q];
+      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if (threadIdx.x == 0 && r0 + q < a.N) partials[(int64_t)blockIdx.x * a.N + r0 + q] = t;
+    }
   }
 }
 
@@ -443,18 +414,21 @@ qcdgpu_mfield mfield_new(const int L[4], int N)
   }
   qcdgpu_field probe = field_new(L, QCDGPU_F16);  // validates L and the volume
   if (!probe) return nullptr;
+  const size_t slot = probe->bytes;
   field_free(probe);
   auto *m = new qcdgpu_mfield_s();
   memcpy(m->L, L, sizeof(m->L));
   m->V = (int64_t)L[0] * L[1] * L[2] * L[3];
+  m->stride = pad_stride(m->V);
   m->N = N;
-  size_t nd = (size_t)12 * m->V * N * sizeof(__half2), nn = (size_t)m->V * N * sizeof(float);
-  m->bytes = nd + nn;
+  // the operator's threads hold two slots: an odd count has a spare one, which
+  // is read (as zeros) and never written
+  m->bytes = slot * (size_t)(N + N % 2);
   if (!QG_CUDA(cudaMalloc(&m->data, m->bytes))) {
     delete m;
     return nullptr;
   }
-  m->norm = (float *)((char *)m->data + nd);
+  m->norm = (float *)m->data + 12 * m->stride;
   if (!QG_CUDA(cudaMemsetAsync(m->data, 0, m->bytes, stream()))) {
     cudaFree(m->data);
     delete m;
@@ -472,7 +446,7 @@ void mfield_free(qcdgpu_mfield m)
 
 // slot r of m <- f (f in any storage precision)
 template <int P>
-__global__ void k_pack(__half2 *d, float *dn, int V, int N, int r, const void *f, const float *fn, int64_t stride)
+__global__ void k_pack(__half2 *d, float *dn, int64_t S, int V, int r, const void *f, const float *fn, int64_t stride)
 {
   int x = (int)(blockIdx.x * blockDim.x + threadIdx.x);
   if (x >= V) return;
@@ -486,23 +460,23 @@ __global__ void k_pack(__half2 *d, float *dn, int V, int N, int r, const void *f
   float2 v[12];
 #pragma unroll
   for (int k = 0; k < 12; k++) v[k] = make_float2(s[k].re, s[k].im);
-  mstore_raw(d, V, N, x, r, v, inv);
-  dn[(int64_t)x * N + r] = mx;
+  mstore_raw(d, S, x, r, v, inv);
+  dn[mnorm_at(S, x, r)] = mx;
 }
 
-// f <- slot r of m
+// f <- slot r of m, in the slots' own FP32 arithmetic
 template <int P>
-__global__ void k_unpack(void *f, float *fn, int64_t stride, const __half2 *d, const float *dn, int V, int N, int r)
+__global__ void k_unpack(void *f, float *fn, int64_t stride, const __half2 *d, const float *dn, int64_t S, int V, int r)
 {
   int x = (int)(blockIdx.x * blockDim.x + threadIdx.x);
   if (x >= V) return;
-  C<double> s[12];
+  const float n = dn[mnorm_at(S, x, r)];
+  float2 v[12];
+  mload_raw(d, S, x, r, v);
+  C<float> s[12];
 #pragma unroll
-  for (int k = 0; k < 12; k++) {
-    float2 v = mload(d, dn, V, N, k, x, r);
-    s[k] = C<double>{(double)v.x, (double)v.y};
-  }
-  Spinor<P, double>::store(f, fn, stride, x, s);
+  for (int k = 0; k < 12; k++) s[k] = C<float>{v[k].x * n, v[k].y * n};
+  Spinor<P, float>::store(f, fn, stride, x, s);
 }
 
 bool mfield_set(qcdgpu_mfield m, int r, qcdgpu_field f)
@@ -511,11 +485,13 @@ bool mfield_set(qcdgpu_mfield m, int r, qcdgpu_field f)
     set_error("multi-RHS set: bad slot or shape");
     return false;
   }
-  unsigned g = (unsigned)((m->V + 127) / 128);
+  const unsigned g = (unsigned)((m->V + 127) / 128);
   __half2 *d = (__half2 *)m->data;
-  if (f->prec == QCDGPU_F64) k_pack<QCDGPU_F64><<<g, 128, 0, stream()>>>(d, m->norm, (int)m->V, m->N, r, f->data, f->norm, f->stride);
-  else if (f->prec == QCDGPU_F32) k_pack<QCDGPU_F32><<<g, 128, 0, stream()>>>(d, m->norm, (int)m->V, m->N, r, f->data, f->norm, f->stride);
-  else k_pack<QCDGPU_F16><<<g, 128, 0, stream()>>>(d, m->norm, (int)m->V, m->N, r, f->data, f->norm, f->stride);
+  if (f->prec == QCDGPU_F16)
+    return QG_CUDA(cudaMemcpyAsync((char *)m->data + (size_t)r * f->bytes, f->data, f->bytes, cudaMemcpyDeviceToDevice,
+                                   stream()));
+  if (f->prec == QCDGPU_F64) k_pack<QCDGPU_F64><<<g, 128, 0, stream()>>>(d, m->norm, m->stride, (int)m->V, r, f->data, f->norm, f->stride);
+  else k_pack<QCDGPU_F32><<<g, 128, 0, stream()>>>(d, m->norm, m->stride, (int)m->V, r, f->data, f->norm, f->stride);
   return QG_LAUNCHED("mrhs_pack");
 }
 
@@ -525,11 +501,13 @@ bool mfield_get(qcdgpu_field f, qcdgpu_mfield m, int r)
     set_error("multi-RHS get: bad slot or shape");
     return false;
   }
-  unsigned g = (unsigned)((m->V + 127) / 128);
+  const unsigned g = (unsigned)((m->V + 127) / 128);
   const __half2 *d = (const __half2 *)m->data;
-  if (f->prec == QCDGPU_F64) k_unpack<QCDGPU_F64><<<g, 128, 0, stream()>>>(f->data, f->norm, f->stride, d, m->norm, (int)m->V, m->N, r);
-  else if (f->prec == QCDGPU_F32) k_unpack<QCDGPU_F32><<<g, 128, 0, stream()>>>(f->data, f->norm, f->stride, d, m->norm, (int)m->V, m->N, r);
-  else k_unpack<QCDGPU_F16><<<g, 128, 0, stream()>>>(f->data, f->norm, f->stride, d, m->norm, (int)m->V, m->N, r);
+  if (f->prec == QCDGPU_F16)
+    return QG_CUDA(cudaMemcpyAsync(f->data, (const char *)m->data + (size_t)r * f->bytes, f->bytes,
+                                   cudaMemcpyDeviceToDevice, stream()));
+  if (f->prec == QCDGPU_F64) k_unpack<QCDGPU_F64><<<g, 128, 0, stream()>>>(f->data, f->norm, f->stride, d, m->norm, m->stride, (int)m->V, r);
+  else k_unpack<QCDGPU_F32><<<g, 128, 0, stream()>>>(f->data, f->norm, f->stride, d, m->norm, m->stride, (int)m->V, r);
   return QG_LAUNCHED("mrhs_unpack");
 }
 
@@ -538,16 +516,16 @@ bool mfield_get(qcdgpu_field f, qcdgpu_mfield m, int r)
 // ------------------------------------------------------------ launch + tuner
 // per-slot sum of |v|^2 over the block's sites (for the tensor-core variant,
 // whose epilogue has no reduction); block (N, SB) like the SIMT variant
-__global__ void k_mnorm(const __half2 *d, const float *dn, int V, int N, int nact, double *partials)
+__global__ void k_mnorm(const __half2 *d, const float *dn, int64_t S, int V, int N, int nact, double *partials)
 {
   const int r = threadIdx.x, x = blockIdx.x * blockDim.y + threadIdx.y;
   double n2 = 0.0;
   if (r < nact && x < V) {
-    const float s = dn[(int64_t)x * N + r];
+    const float s = dn[mnorm_at(S, x, r)];
     float s2 = 0.f;  // per-site sum in FP32, block sum in double
 #pragma unroll
     for (int k = 0; k < 12; k++) {
-      float2 f = __half22float2(d[mhalf2_index(V, N, k, x, r)]);
+      float2 f = __half22float2(d[mhalf2_index(S, k, x, r)]);
       s2 += (f.x * s) * (f.x * s) + (f.y * s) * (f.y * s);
     }
     n2 = (double)s2;
@@ -862,7 +840,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_wilson_mrhs_tc(const MArgs a,
 #pragma unroll
           for (int dd = 0; dd < 8; dd++) {
             const int y = nb[hs * 9 + dd];
-            nr[dd] = a.in_norm[(int64_t)(EO ? (y >> 1) : y) * a.N + r];
+            nr[dd] = a.in_norm[mnorm_at(a.stride, EO ? (y >> 1) : y, r)];
           }
           const uint4 *p = (const uint4 *)a.in;
 #pragma unroll
@@ -870,7 +848,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_wilson_mrhs_tc(const MArgs a,
             const int y = nb[hs * 9 + 4 * hh + q];
             const int64_t ys = EO ? (y >> 1) : y;
 #pragma unroll
-            for (int j = 0; j < 3; j++) w[q][j] = p[((int64_t)j * a.V + ys) * a.N + r];
+            for (int j = 0; j < 3; j++) w[q][j] = p[mword(a.stride, j, ys, r)];
           }
         }
         if (n >= 2) tc_wait(bdone + 8 * b, ((n >> 1) & 1) ^ 1, ctl, failed);  // the MMAs of item n - 2
@@ -996,9 +974,9 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_wilson_mrhs_tc(const MArgs a,
       for (int g = 0; g < G; g++, n++) {
         const int b = n & 1, r = g * 16 + rl;
         // the diagonal term does not wait for the tensor cores
-        C<float> zs[1][12];
-        float znrm[1] = {0.f};
-        if (zmode && act) mload_rp<1>(a, EO ? a.z : a.in, EO ? a.z_norm : a.in_norm, e, r, zs, znrm);
+        C<float> zs[12];
+        float znrm = 0.f;
+        if (zmode && act) mload_slot(a, EO ? a.z : a.in, EO ? a.z_norm : a.in_norm, e, r, zs, znrm);
         tc_wait(bdone + 8 * b, (n >> 1) & 1, ctl, failed);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         tc_wait(bsready + 8 * b, (n >> 1) & 1, ctl, failed);
@@ -1047,13 +1025,13 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_wilson_mrhs_tc(const MArgs a,
               acc[k] = C<float>{ar * acc[k].re - g5ai * acc[k].im, ar * acc[k].im + g5ai * acc[k].re};
             }
           }
-          const float zsc = zmode ? znrm[0] : 0.f;
+          const float zsc = zmode ? znrm : 0.f;
           const float zm = zmode == 2 ? mp4r * zsc : zsc, zt = zmode == 2 ? tmr * zsc : 0.f;
           float mx = 0.f;
 #pragma unroll
           for (int k = 0; k < 12; k++) {
             const float g5tm = k < 6 ? zt : -zt;
-            const C<float> zk = zmode ? zs[0][k] : C<float>{0.f, 0.f};
+            const C<float> zk = zmode ? zs[k] : C<float>{0.f, 0.f};
             acc[k] = C<float>{zm * zk.re - g5tm * zk.im + ch * acc[k].re, zm * zk.im + g5tm * zk.re + ch * acc[k].im};
             mx = fmaxf(mx, fmaxf(fabsf(acc[k].re), fabsf(acc[k].im)));
           }
@@ -1063,8 +1041,8 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_wilson_mrhs_tc(const MArgs a,
             float2 o[12];
 #pragma unroll
             for (int k = 0; k < 12; k++) o[k] = make_float2(acc[k].re, acc[k].im);
-            mstore_raw(a.out, a.V, a.N, e, r, o, inv);
-            a.out_norm[(int64_t)e * a.N + r] = mx;
+            mstore_raw(a.out, a.stride, e, r, o, inv);
+            a.out_norm[mnorm_at(a.stride, e, r)] = mx;
             if (partials) {  // |out|^2 of the stored (rounded) values
               float s2 = 0.f;
 #pragma unroll
@@ -1156,50 +1134,20 @@ bool mrhs_tc_failed() { return g_tc_fail_host && *g_tc_fail_host; }
 
 struct MrhsTune {
   int variant;  // MRHS_SIMT, MRHS_MMA or MRHS_TC
-  int threads;  // SIMT: N x (sites per block) target, 64, 128 or 256
-  int rp;       // SIMT: RHS slots per thread (1, or 2 when N is even)
+  int threads;  // SIMT: threads per block, 64, 128 or 256
 };
 
 static int g_mrhs_variant = MRHS_AUTO;
 static std::map<std::pair<int64_t, int>, MrhsTune> g_mrhs_tuned;
 
-// block (N / rp slot threads, sites per block). `threads` / N sites is the
-// target; of the counts from half to twice that (at least up to 4, at most
-// 256 threads) the one that leaves the fewest idle lanes in the block's last
-// warp is taken, the nearest to the target on a tie (48 slots at two per
-// thread: 4 sites of 24 threads fill three warps, where 1 site leaves a
-// quarter of its warp idle)
-static dim3 simt_block(int N, int threads, int rp = 1)
-{
-  const int x = (N + rp - 1) / rp;  // threads per site
-  const int sb = threads / N > 0 ? threads / N : 1;
-  const int hi = 2 * sb > 4 ? 2 * sb : 4;
-  int best = sb;
-  int best_idle = 1 << 30, best_warps = 1;
-  for (int c = sb / 2 > 1 ? sb / 2 : 1; c <= hi && x * c <= 256; c++) {
-    const int t = x * c, warps = (t + 31) / 32, idle = warps * 32 - t;
-    // idle / (32 warps) compared exactly: fewer idle lanes per lane, then nearer the target
-    const long long lhs = (long long)idle * best_warps, rhs = (long long)best_idle * warps;
-    if (best_idle == 1 << 30 || lhs < rhs || (lhs == rhs && abs(c - sb) < abs(best - sb))) {
-      best = c;
-      best_idle = idle;
-      best_warps = warps;
-    }
-  }
-  return dim3((unsigned)x, (unsigned)best);
-}
+// (slot, site) block of the mma.sync variant's norm kernel
+static dim3 mnorm_block(int N) { return dim3((unsigned)N, (unsigned)(256 / N)); }
 
-// the largest block count of any shape that writes per-slot partial sums
+// the largest block count of any launch that writes per-slot partial sums
 unsigned mrhs_max_blocks(int64_t V, int N)
 {
-  unsigned m = 0;
-  for (int threads : {64, 128, 256})
-    for (int rp : {1, 2}) {
-      const dim3 b = simt_block(N, threads, rp);
-      const unsigned nb = (unsigned)((V + b.y - 1) / b.y);
-      if (nb > m) m = nb;
-    }
-  return m;
+  const unsigned simt = (unsigned)((V + 31) / 32), y = mnorm_block(N).y, mma = (unsigned)((V + y - 1) / y);
+  return simt > mma ? simt : mma;
 }
 
 static bool launch_mrhs(const MArgs &a, bool dag, MrhsTune t, double *partials, unsigned *nblocks)
@@ -1233,40 +1181,27 @@ static bool launch_mrhs(const MArgs &a, bool dag, MrhsTune t, double *partials, 
     return true;
   }
   const bool simt = t.variant == MRHS_SIMT;
-  // threads for the occupied slots only (the tuned block size holds more
-  // sites when fewer slots are occupied), except when the launch writes
-  // per-slot partial sums: their grouping into blocks, and so their summation
-  // order, must not depend on which other slots are occupied
-  const dim3 blk = simt_block(simt && !partials ? a.nact : a.N, simt ? t.threads : 256, simt ? t.rp : 1);
-  const unsigned nb = (unsigned)((a.V + blk.y - 1) / blk.y);
-  const size_t shm = sizeof(double) * a.N * blk.y;
   if (simt) {
-    const int ns = (int)blk.x * t.rp < a.N ? (int)blk.x * t.rp : a.N;
-    const size_t sm = partials ? sizeof(double) * ns * blk.y : 0;
+    // warps: 32 sites of one slot pair; a block holds several pairs of the
+    // same sites (their links meet in L1). The grouping of a slot's partial
+    // sums does not depend on the occupied slots.
+    const int pairs = (a.nact + 1) / 2, pb = pairs < t.threads / 32 ? pairs : t.threads / 32;
+    const dim3 grid((unsigned)((a.V + 31) / 32), (unsigned)((pairs + pb - 1) / pb)), blk(32, (unsigned)pb);
     // kernel mode from the epilogue (see k_wilson_mrhs_simt)
     const int mode = a.eo_par < 0 ? 0 : a.ainv ? 1 : 2;
-#define QG_SIMT(RP, MODE)                                                           \
-  if (dag) k_wilson_mrhs_simt<true, RP, MODE><<<nb, blk, sm, s>>>(a, partials);     \
-  else k_wilson_mrhs_simt<false, RP, MODE><<<nb, blk, sm, s>>>(a, partials);
-    if (t.rp == 2) {
-      if (mode == 0) {
-        QG_SIMT(2, 0)
-      } else if (mode == 1) {
-        QG_SIMT(2, 1)
-      } else {
-        QG_SIMT(2, 2)
-      }
+#define QG_SIMT(MODE)                                                            \
+  if (dag) k_wilson_mrhs_simt<true, MODE><<<grid, blk, 0, s>>>(a, partials);     \
+  else k_wilson_mrhs_simt<false, MODE><<<grid, blk, 0, s>>>(a, partials);
+    if (mode == 0) {
+      QG_SIMT(0)
+    } else if (mode == 1) {
+      QG_SIMT(1)
     } else {
-      if (mode == 0) {
-        QG_SIMT(1, 0)
-      } else if (mode == 1) {
-        QG_SIMT(1, 1)
-      } else {
-        QG_SIMT(1, 2)
-      }
+      QG_SIMT(2)
     }
 #undef QG_SIMT
-    if (!QG_LAUNCHED("wilson_mrhs_simt")) return false;
+    if (nblocks) *nblocks = grid.x;
+    return QG_LAUNCHED("wilson_mrhs_simt");
   } else {
     unsigned grid = (unsigned)((a.V + 3) / 4);
     int mt = (a.nact + 15) / 16;
@@ -1282,38 +1217,37 @@ static bool launch_mrhs(const MArgs &a, bool dag, MrhsTune t, double *partials, 
 #undef QG_MRHS
     if (!QG_LAUNCHED("wilson_mrhs")) return false;
     if (partials) {
-      k_mnorm<<<nb, simt_block(a.N, 256), shm, s>>>(a.out, a.out_norm, a.V, a.N, a.nact, partials);
+      const dim3 blk = mnorm_block(a.N);
+      const unsigned nb = (unsigned)((a.V + blk.y - 1) / blk.y);
+      const size_t shm = sizeof(double) * a.N * blk.y;
+      if (nblocks) *nblocks = nb;
+      k_mnorm<<<nb, blk, shm, s>>>(a.out, a.out_norm, a.stride, a.V, a.N, a.nact, partials);
       if (!QG_LAUNCHED("mrhs_norm")) return false;
     }
   }
-  if (nblocks) *nblocks = nb;
   return true;
 }
 
-// Pick the variant and block shape for (V, N) by timing each candidate
-// three times on the caller's fields (the output is overwritten with the
-// same result). Not while the stream is being captured: then the SIMT
-// variant with 256-thread blocks runs until a tuned choice exists.
+// Pick the SIMT kernel's block size for (V, N) by timing each candidate three
+// times on the caller's fields (the output is overwritten with the same
+// result). Not while the stream is being captured: then 64-thread blocks run
+// until a tuned choice exists. The tensor-core kernels have lost to SIMT at
+// every volume and slot count measured (by factors of 2 and 9): they run when
+// asked for, and a first apply does not spend its time on them.
 static MrhsTune mrhs_tune(const MArgs &a, bool dag)
 {
-  if (g_mrhs_variant == MRHS_MMA) return MrhsTune{MRHS_MMA, 256, 1};
-  if (g_mrhs_variant == MRHS_TC) return MrhsTune{MRHS_TC, kTcThreads, 1};
-  if (g_mrhs_variant >= 64) {  // forced block size; +1: two slots per thread
-    const int rp = (g_mrhs_variant & 1) && a.N % 2 == 0 ? 2 : 1;
-    return MrhsTune{MRHS_SIMT, g_mrhs_variant & ~1, rp};
-  }
+  if (g_mrhs_variant == MRHS_MMA) return MrhsTune{MRHS_MMA, 256};
+  if (g_mrhs_variant == MRHS_TC) return MrhsTune{MRHS_TC, kTcThreads};
+  if (g_mrhs_variant >= 64) return MrhsTune{MRHS_SIMT, g_mrhs_variant & ~1};  // forced block size
   // even/odd kernels are tuned separately (key: minus the half volume)
   const auto key = std::make_pair(a.eo_par < 0 ? (int64_t)a.V : -(int64_t)a.V, a.N);
   auto it = g_mrhs_tuned.find(key);
   if (it != g_mrhs_tuned.end()) return it->second;
-  const MrhsTune fallback{MRHS_SIMT, 128, 1};
+  const MrhsTune fallback{MRHS_SIMT, 64};
   cudaStream_t s = stream();
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return fallback;
-  const MrhsTune cands[] = {{MRHS_SIMT, 64, 1},  {MRHS_SIMT, 128, 1}, {MRHS_SIMT, 256, 1},
-                            {MRHS_SIMT, 64, 2},  {MRHS_SIMT, 128, 2}, {MRHS_SIMT, 256, 2},
-                            {MRHS_TC, kTcThreads, 1}, {MRHS_MMA, 256, 1}};
-  const int ncand = a.eo_par < 0 ? 8 : 7;  // the mma.sync kernel has no even/odd mode
+  const MrhsTune cands[] = {{MRHS_SIMT, 64}, {MRHS_SIMT, 128}, {MRHS_SIMT, 256}};
   cudaEvent_t e0, e1;
   if (cudaEventCreate(&e0) != cudaSuccess) return fallback;
   if (cudaEventCreate(&e1) != cudaSuccess) {
@@ -1322,10 +1256,7 @@ static MrhsTune mrhs_tune(const MArgs &a, bool dag)
   }
   MrhsTune best = fallback;
   float best_ms = 1e30f;
-  for (int ic = 0; ic < ncand; ic++) {
-    const MrhsTune &c = cands[ic];
-    if (c.variant == MRHS_SIMT && (c.threads < a.N || (c.rp == 2 && a.N % 2 != 0))) continue;
-    if (c.variant == MRHS_TC && a.N % 16 != 0) continue;
+  for (const MrhsTune &c : cands) {
     if (!launch_mrhs(a, dag, c, nullptr, nullptr)) break;  // warm-up
     cudaEventRecord(e0, s);
     bool ok = true;
@@ -1376,6 +1307,7 @@ bool dslash_mrhs(qcdgpu_mfield out, qcdgpu_mfield in, qcdgpu_gauge g, double mp4
   a.geo.st[3] = in->L[0] * in->L[1] * in->L[2];
   a.V = (int)in->V;
   a.N = in->N;
+  a.stride = in->stride;
   a.nact = nact;
   a.gstride = g32->stride;
   // the FP32 copy holds the boundary phases folded into its links
@@ -1434,6 +1366,7 @@ bool dslash_mrhs_eo(qcdgpu_mfield out, qcdgpu_mfield in, qcdgpu_mfield z, qcdgpu
   a.geo.st[3] = g->L[0] * g->L[1] * g->L[2];
   a.V = (int)in->V;
   a.N = in->N;
+  a.stride = in->stride;
   a.nact = nact;
   a.gstride = g32->stride;
   // the FP32 copy holds the boundary phases folded into its links
@@ -1521,7 +1454,7 @@ int qcdgpu_mrhs_tuned(const int L[4], int nrhs, int *variant, int *threads)
   auto it = qg::g_mrhs_tuned.find(std::make_pair(V, nrhs));
   if (it == qg::g_mrhs_tuned.end()) return 1;
   *variant = it->second.variant;
-  *threads = it->second.threads + (it->second.rp == 2 ? 1 : 0);
+  *threads = it->second.threads + 1;  // two slots per thread
   return 0;
 }
 

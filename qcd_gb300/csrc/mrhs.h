@@ -4,30 +4,39 @@
 
 #include "internal.h"
 
-// N spinors in FP16 with one float norm per (site, RHS). The 12 complex
-// components of a spinor form three groups of four; group j of slot r at
-// site x is one 16-byte word (8 halves: re, im of components 4j..4j+3) at
-// uint4 index (j * V + x) * N + r. A thread reads a whole spinor with three
-// 128-bit loads, and the threads of consecutive (site, slot) pairs read
-// consecutive words. Norms are [site][slot] floats.
+// N spinors in FP16 with one float norm per (site, RHS), slot after slot, each
+// slot exactly as an FP16 field lies in memory (internal.h): three blocks of
+// 16-byte words (8 halves: re, im of components 4j..4j+3), then the norms, with
+// the field's block stride. A warp takes 32 consecutive sites of a slot (pair),
+// so every access is a run of consecutive words, and a slot moves in and out as
+// a plain copy. (With all slots of a site adjacent the operator took the same
+// time, but one of 16 slots of 24^3 x 48 took 50 us to read out, against 12.)
 struct qcdgpu_mfield_s {
   int L[4];
   int64_t V;
-  int N;  // RHS slots
+  int64_t stride;  // block stride, as of a field
+  int N;           // RHS slots
   void *data;
-  float *norm;
+  float *norm;     // of slot 0; slot r's lie 13 r stride floats further
   size_t bytes;
 };
 
 namespace qg {
 
+// indexes of slot r in blocks of stride S: word j (uint4) and norm (float) of site x
+__host__ __device__ __forceinline__ int64_t mword(int64_t S, int j, int64_t x, int r)
+{
+  return r * (S / 4 * 13) + j * S + x;
+}
+__host__ __device__ __forceinline__ int64_t mnorm_at(int64_t S, int64_t x, int r) { return r * (13 * S) + x; }
+
 // spinor (x, r) of a multi-RHS field as 12 float2 (without the norm)
-__device__ __forceinline__ void mload_raw(const __half2 *d, int64_t V, int N, int x, int r, float2 v[12])
+__device__ __forceinline__ void mload_raw(const __half2 *d, int64_t S, int x, int r, float2 v[12])
 {
   const uint4 *p = (const uint4 *)d;
 #pragma unroll
   for (int j = 0; j < 3; j++) {
-    const uint4 w = p[((int64_t)j * V + x) * N + r];
+    const uint4 w = p[mword(S, j, x, r)];
     v[4 * j + 0] = __half22float2(*(const __half2 *)&w.x);
     v[4 * j + 1] = __half22float2(*(const __half2 *)&w.y);
     v[4 * j + 2] = __half22float2(*(const __half2 *)&w.z);
@@ -36,7 +45,7 @@ __device__ __forceinline__ void mload_raw(const __half2 *d, int64_t V, int N, in
 }
 
 // spinor (x, r) <- 12 float2 multiplied by inv, rounded to FP16
-__device__ __forceinline__ void mstore_raw(__half2 *d, int64_t V, int N, int x, int r, const float2 v[12], float inv)
+__device__ __forceinline__ void mstore_raw(__half2 *d, int64_t S, int x, int r, const float2 v[12], float inv)
 {
   uint4 *p = (uint4 *)d;
 #pragma unroll
@@ -49,14 +58,14 @@ __device__ __forceinline__ void mstore_raw(__half2 *d, int64_t V, int N, int x, 
     w.y = *(const unsigned *)&h[1];
     w.z = *(const unsigned *)&h[2];
     w.w = *(const unsigned *)&h[3];
-    p[((int64_t)j * V + x) * N + r] = w;
+    p[mword(S, j, x, r)] = w;
   }
 }
 
 // component k of spinor (x, r) as one half2
-__device__ __forceinline__ int64_t mhalf2_index(int64_t V, int N, int k, int x, int r)
+__device__ __forceinline__ int64_t mhalf2_index(int64_t S, int k, int x, int r)
 {
-  return (((int64_t)(k >> 2) * V + x) * N + r) * 4 + (k & 3);
+  return mword(S, k >> 2, x, r) * 4 + (k & 3);
 }
 
 qcdgpu_mfield mfield_new(const int L[4], int N);

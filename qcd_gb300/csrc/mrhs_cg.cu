@@ -32,14 +32,15 @@ using namespace qgd;
 struct MV {
   __half2 *d;
   float *n;
-  int V, N;
+  int64_t S;  // block stride
+  int V;
 };
-static MV mv(qcdgpu_mfield m) { return MV{(__half2 *)m->data, m->norm, (int)m->V, m->N}; }
+static MV mv(qcdgpu_mfield m) { return MV{(__half2 *)m->data, m->norm, m->stride, (int)m->V}; }
 
 __device__ __forceinline__ void mv_load(const MV &m, int x, int r, float2 v[12])
 {
-  const float s = m.n[(int64_t)x * m.N + r];
-  mload_raw(m.d, m.V, m.N, x, r, v);
+  const float s = m.n[mnorm_at(m.S, x, r)];
+  mload_raw(m.d, m.S, x, r, v);
 #pragma unroll
   for (int k = 0; k < 12; k++) v[k] = make_float2(v[k].x * s, v[k].y * s);
 }
@@ -50,51 +51,39 @@ __device__ __forceinline__ void mv_store(const MV &m, int x, int r, const float2
   for (int k = 0; k < 12; k++) mx = fmaxf(mx, fmaxf(fabsf(v[k].x), fabsf(v[k].y)));
   if (!(mx >= 1.17549435e-38f)) mx = 0.f;
   const float inv = mx > 0.f ? 1.0f / mx : 0.f;
-  mstore_raw(m.d, m.V, m.N, x, r, v, inv);
-  m.n[(int64_t)x * m.N + r] = mx;
+  mstore_raw(m.d, m.S, x, r, v, inv);
+  m.n[mnorm_at(m.S, x, r)] = mx;
 }
 
-// Launch shape of the per-(site, slot) kernels: block (N, SB) -- x = slot,
-// y = site within the block -- so a warp reads the slots of one site
-// contiguously; partials[block * N + slot] receives the block's sum for each
-// slot in a fixed order.
-static dim3 mblock(int N) { return dim3((unsigned)N, (unsigned)(256 / N > 0 ? 256 / N : 1)); }
-static unsigned mgrid(int V, int N) { return (unsigned)((V + mblock(N).y - 1) / mblock(N).y); }
+// Launch shape of the per-(site, slot) kernels: blocks of kMSites sites of one
+// slot (blockIdx.y); partials[block * N + slot] receives the block's sum in a
+// fixed order that no other slot enters.
+constexpr int kMSites = 256;
+static dim3 mgrid(int64_t V, int n) { return dim3((unsigned)((V + kMSites - 1) / kMSites), (unsigned)n); }
 
-// block partials of the blockDim.x occupied slots, at slot stride N
-__device__ __forceinline__ void slot_partial(double v, double *partials, int N)
-{
-  extern __shared__ double sh[];
-  const int NS = blockDim.x, r = threadIdx.x, y = threadIdx.y;
-  sh[y * NS + r] = v;
-  __syncthreads();
-  if (y == 0) {
-    double s = 0.0;
-    for (int i = 0; i < (int)blockDim.y; i++) s += sh[i * NS + r];
-    partials[(int64_t)blockIdx.x * N + r] = s;
-  }
-}
-
-// FP32 solution increments of the slots: components 2j, 2j+1 of slot r at
-// site x form the float4 at index (j * V + x) * N + r, j = 0..5. FP16 would
-// round every increment to 11 bits and cost iterations.
+// FP32 solution increments of the slots, each laid out as an FP32 field
+// (components 2j, 2j+1 form one float4, j = 0..5). FP16 would round every
+// increment to 11 bits and cost iterations.
 struct MX {
   float4 *d;
-  int V, N;
+  int64_t S;
+  int V;
+  __device__ __forceinline__ float4 &at(int j, int x, int r) const { return d[(r * 6 + j) * S + x]; }
 };
 
 // xs += alpha p ; rs -= alpha Ap ; partials <- |rs|^2 per slot
-__global__ void k_mupdate(MX xs, MV ps, MV rs, MV aps, int nact, const double *alpha, double *partials)
+__global__ void __launch_bounds__(kMSites) k_mupdate(MX xs, MV ps, MV rs, MV aps, const double *alpha,
+                                                     double *partials, int N)
 {
-  const int r = threadIdx.x, x = blockIdx.x * blockDim.y + threadIdx.y;
+  const int r = blockIdx.y, x = blockIdx.x * kMSites + threadIdx.x;
   double n2 = 0.0;
-  if (r < nact && x < xs.V) {
+  if (x < xs.V) {
     const float al = (float)alpha[r];
     float2 a[12], b[12];
     mv_load(ps, x, r, b);
 #pragma unroll
     for (int j = 0; j < 6; j++) {
-      float4 &v = xs.d[((int64_t)j * xs.V + x) * xs.N + r];
+      float4 &v = xs.at(j, x, r);
       const float4 w = v;
       v = make_float4(__fmaf_rn(al, b[2 * j].x, w.x), __fmaf_rn(al, b[2 * j].y, w.y),
                       __fmaf_rn(al, b[2 * j + 1].x, w.z), __fmaf_rn(al, b[2 * j + 1].y, w.w));
@@ -110,7 +99,15 @@ __global__ void k_mupdate(MX xs, MV ps, MV rs, MV aps, int nact, const double *a
     mv_store(rs, x, r, a);
     n2 = (double)s2;
   }
-  slot_partial(n2, partials, xs.N);
+  for (int o = 16; o > 0; o >>= 1) n2 += __shfl_xor_sync(0xffffffffu, n2, o);
+  __shared__ double sh[kMSites / 32];
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = n2;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double s = 0.0;
+    for (int i = 0; i < kMSites / 32; i++) s += sh[i];
+    partials[(int64_t)blockIdx.x * N + r] = s;
+  }
 }
 
 // f (FP64 field) += slot r of xs, then slot r of xs <- 0
@@ -120,7 +117,7 @@ __global__ void k_mx_flush(double2 *f, int64_t fstride, MX xs, int r)
   if (x >= xs.V) return;
 #pragma unroll
   for (int j = 0; j < 6; j++) {
-    float4 &v = xs.d[((int64_t)j * xs.V + x) * xs.N + r];
+    float4 &v = xs.at(j, x, r);
     double2 &o0 = f[(int64_t)(2 * j) * fstride + x];
     double2 &o1 = f[(int64_t)(2 * j + 1) * fstride + x];
     const float4 w = v;
@@ -139,15 +136,15 @@ __global__ void k_mx_copy(MX xs, int from, int to, int zero)
   if (x >= xs.V) return;
 #pragma unroll
   for (int j = 0; j < 6; j++)
-    xs.d[((int64_t)j * xs.V + x) * xs.N + to] =
-        zero ? make_float4(0.f, 0.f, 0.f, 0.f) : xs.d[((int64_t)j * xs.V + x) * xs.N + from];
+    xs.at(j, x, to) =
+        zero ? make_float4(0.f, 0.f, 0.f, 0.f) : xs.at(j, x, from);
 }
 
 // ps = rs + beta ps
-__global__ void k_mp(MV ps, MV rs, int nact, const double *beta)
+__global__ void __launch_bounds__(kMSites) k_mp(MV ps, MV rs, const double *beta)
 {
-  const int r = threadIdx.x, x = blockIdx.x * blockDim.y + threadIdx.y;
-  if (r >= nact || x >= ps.V) return;
+  const int r = blockIdx.y, x = blockIdx.x * kMSites + threadIdx.x;
+  if (x >= ps.V) return;
   const float be = (float)beta[r];
   float2 p[12], q[12];
   mv_load(ps, x, r, p);
@@ -165,8 +162,8 @@ __global__ void k_mcopy(MV m, int from, int to, int zero)
   uint4 *p = (uint4 *)m.d;
 #pragma unroll
   for (int j = 0; j < 3; j++)
-    p[((int64_t)j * m.V + x) * m.N + to] = zero ? make_uint4(0u, 0u, 0u, 0u) : p[((int64_t)j * m.V + x) * m.N + from];
-  m.n[(int64_t)x * m.N + to] = zero ? 0.f : m.n[(int64_t)x * m.N + from];
+    p[mword(m.S, j, x, to)] = zero ? make_uint4(0u, 0u, 0u, 0u) : p[mword(m.S, j, x, from)];
+  m.n[mnorm_at(m.S, x, to)] = zero ? 0.f : m.n[mnorm_at(m.S, x, from)];
 }
 
 // scalar layout, per slot r of N: rr, pAp, alpha, beta, then history[j]
@@ -294,7 +291,7 @@ struct qcdgpu_batch_s {
 
 namespace qg {
 
-static MX mx(qcdgpu_batch B) { return MX{B->xs, (int)B->Vs, B->cap}; }
+static MX mx(qcdgpu_batch B) { return MX{B->xs, pad_stride(B->Vs), (int)B->Vs}; }
 
 static void batch_free(qcdgpu_batch b)
 {
@@ -363,11 +360,11 @@ static qcdgpu_batch batch_new(qcdgpu_gauge g, int cap, bool eo)
     }
   }
   size_t ns = (size_t)(M_HIST + kMChunk) * cap;
-  unsigned nb = mgrid((int)b->Vs, cap);
+  unsigned nb = mgrid(b->Vs, 1).x;
   if (mrhs_max_blocks(b->Vs, cap) > nb) nb = mrhs_max_blocks(b->Vs, cap);
-  ok = ok && QG_CUDA(cudaMalloc(&b->xs, (size_t)12 * b->Vs * cap * sizeof(float2))) &&
-            QG_CUDA(cudaMalloc(&b->s, ns * sizeof(double))) && QG_CUDA(cudaMalloc(&b->mp4s, cap * sizeof(float))) &&
-            QG_CUDA(cudaMalloc(&b->tms, cap * sizeof(float))) &&
+  ok = ok && QG_CUDA(cudaMalloc(&b->xs, (size_t)12 * pad_stride(b->Vs) * cap * sizeof(float2))) &&
+            QG_CUDA(cudaMalloc(&b->s, ns * sizeof(double))) && QG_CUDA(cudaMalloc(&b->mp4s, (cap + 1) * sizeof(float))) &&
+            QG_CUDA(cudaMalloc(&b->tms, (cap + 1) * sizeof(float))) &&
             QG_CUDA(cudaMalloc(&b->part, (size_t)nb * cap * sizeof(double))) &&
             QG_CUDA(cudaMalloc(&b->l1, (size_t)kMSGroups * cap * sizeof(double) + 256)) &&
             QG_CUDA(cudaMalloc(&b->rudev, (size_t)4 * cap * sizeof(double))) &&
@@ -601,16 +598,11 @@ static bool chunk_enqueue(qcdgpu_batch B, int n)
 {
   const int cap = B->cap;
   const int V = (int)B->Vs;
-  // the update writes per-slot partial sums: its block shape follows the
-  // capacity, so their summation order does not depend on the mix; the
-  // direction update uses threads for the n occupied slots only
-  const dim3 blk = mblock(cap), blkp = mblock(n);
-  const unsigned nb = mgrid(V, cap), nbp = mgrid(V, n);
-  const size_t shm = sizeof(double) * blk.x * blk.y;
+  const dim3 grid = mgrid(V, n);
   cudaStream_t st = stream();
   for (int j = 0; j < kMChunk; j++) {
     // p = r + beta p (beta = 0 keeps a fresh slot's p = r)
-    k_mp<<<nbp, blkp, 0, st>>>(mv(B->ps), mv(B->rs), n, B->s + M_BETA * cap);
+    k_mp<<<grid, kMSites, 0, st>>>(mv(B->ps), mv(B->rs), B->s + M_BETA * cap);
     if (!QG_LAUNCHED("mrhs_p")) return false;
     // p^+ A^+ A p = |A p|^2, summed per slot in the epilogue of t = A p
     // (A = D, or the Schur complement M = A_ee - H_eo A_oo^{-1} H_oe / 4 as
@@ -632,9 +624,9 @@ static bool chunk_enqueue(qcdgpu_batch B, int n)
     } else if (!dslash_mrhs(B->aps, B->t, B->g, 4.0, 0.0, true, n, B->mp4s, B->tms)) {
       return false;
     }
-    k_mupdate<<<nb, blk, shm, st>>>(mx(B), mv(B->ps), mv(B->rs), mv(B->aps), n, B->s + M_ALPHA * cap, B->part);
+    k_mupdate<<<grid, kMSites, 0, st>>>(mx(B), mv(B->ps), mv(B->rs), mv(B->aps), B->s + M_ALPHA * cap, B->part, cap);
     if (!QG_LAUNCHED("mrhs_update")) return false;
-    k_mscalars2<<<kMSGroups, 256, 0, st>>>(B->part, (int)nb, cap, n, B->s, 1, j, B->l1, B->msdone);
+    k_mscalars2<<<kMSGroups, 256, 0, st>>>(B->part, (int)grid.x, cap, n, B->s, 1, j, B->l1, B->msdone);
     if (!QG_LAUNCHED("mrhs_scalars")) return false;
   }
   return QG_CUDA(cudaMemcpyAsync(B->hs, B->s, sizeof(double) * (M_HIST + kMChunk) * cap, cudaMemcpyDeviceToHost, st));
@@ -840,7 +832,7 @@ int qcdgpu_batch_poll(qcdgpu_batch b, int *tags, int *status, int *iters, double
 size_t qcdgpu_batch_bytes(qcdgpu_batch b)
 {
   if (!b) return 0;
-  size_t n = 4 * b->rs->bytes + (size_t)12 * b->Vs * b->cap * sizeof(float2) + 3 * b->rt->bytes + b->bd->bytes;
+  size_t n = 4 * b->rs->bytes + (size_t)12 * qg::pad_stride(b->Vs) * b->cap * sizeof(float2) + 3 * b->rt->bytes + b->bd->bytes;
   if (b->eo) n += b->u->bytes + b->u64->bytes + 3 * b->r32->bytes + (size_t)b->cap * b->rt->bytes;
   for (const auto &sl : b->slots)  // c_e, A^{-1} b_o outside x (x too small for both)
     for (auto f : {sl.ce, sl.to})

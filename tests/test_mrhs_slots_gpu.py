@@ -1,0 +1,64 @@
+"""Multi-RHS fields and batches where slots and sites do not fill the kernels'
+pairs and warps: odd slot counts (a spare slot pads the last pair), odd
+occupied counts, site counts off 32. The operator against the oracle (4e-3 per
+RHS, the FP16 bar of test_mrhs_gpu.py); FP16 fields go in and come out
+unchanged; odd-capacity batches reach their tolerance."""
+import numpy as np
+import pytest
+
+import qcd_gb300 as q
+from tests.conftest import EPS_PLAQ_060
+
+pytestmark = pytest.mark.gpu
+TH = (np.pi, 0.0, 0.0, 0.0)
+
+
+@pytest.mark.parametrize("nrhs,nact", [(1, 1), (3, 3), (7, 6), (8, 5)])
+@pytest.mark.parametrize("L", [(2, 2, 2, 2), (3, 5, 2, 7)])
+def test_odd_slots_and_sites(gpu, orc, L, nrhs, nact):
+    u = orc.gauge_synthetic(L, 71, EPS_PLAQ_060)
+    g = q.Gauge(L, TH).load(u)
+    mi, mo, f = q.MField(L, nrhs), q.MField(L, nrhs), q.Field(L)
+    src = [orc.gaussian_spinor(L, 700 + r) for r in range(nrhs)]
+    for r in range(nrhs):
+        mi.set(r, f.load(src[r]))
+    q.dslash_mrhs(mo, mi, g, 0.15, 0.03, q.OP_D, nact)
+    for r in range(nact):
+        ref = orc.dslash(src[r], u, L, TH, kappa=0.15, tm=0.03)
+        assert np.linalg.norm(mo.get(r, f).store() - ref) <= 4e-3 * np.linalg.norm(ref)
+    for r in range(nact, nrhs):  # slots that were not asked for stay empty
+        assert not mo.get(r, f).store().any()
+    for o in (g, mi, mo, f):
+        o.close()
+
+
+@pytest.mark.parametrize("L", [(3, 5, 2, 7), (4, 4, 4, 4)])
+def test_fp16_fields_pass_unchanged(gpu, orc, L):
+    m, a, b = q.MField(L, 3), q.Field(L, q.F16), q.Field(L, q.F16)
+    for r in range(3):
+        m.set(r, a.load(orc.gaussian_spinor(L, 720 + r) * 10.0 ** (3 * r)))
+        assert np.array_equal(m.get(r, b).store(), a.store())
+    for o in (m, a, b):
+        o.close()
+
+
+@pytest.mark.parametrize("cap,n", [(1, 2), (3, 4)])
+@pytest.mark.parametrize("eo", [False, True])
+def test_odd_capacity_batches(gpu, orc, cap, n, eo):
+    L = (8, 4, 4, 4)
+    u = orc.gauge_synthetic(L, 73, EPS_PLAQ_060)
+    g = q.Gauge(L, TH).load(u)
+    batch = q.Batch(g, cap, eo=eo)
+    src = [orc.gaussian_spinor(L, 730 + r) for r in range(n)]
+    fb, fx = [q.Field(L).load(v) for v in src], [q.Field(L) for _ in range(n)]
+    nxt = 0
+    while nxt < n or batch.active:
+        while nxt < n and batch.add(fx[nxt], fb[nxt], 0.14, 0.01, tol=1e-10, tag=nxt) >= 0:
+            nxt += 1
+        batch.step(16)
+    assert sorted(t for t, st, _, _ in batch.poll() if st == 0) == list(range(n))
+    for v, x in zip(src, fx):
+        assert orc.true_residual(x.store(), v, u, L, TH, 0.14, 0.01) <= 1e-10
+    batch.close()
+    for o in fb + fx + [g]:
+        o.close()
