@@ -353,8 +353,9 @@ typedef float4 FFShare[2][3][2][kFFSites];
 
 // the two hops of direction MU for one site and colour row col. The staged
 // components of hop (MU, back) are in stage `back`; the next hop's are
-// requested first (NEXT: the direction after MU, 4 when MU is the last).
-template <int MU, int NEXT, bool DAG, bool EO, bool AOS>
+// requested first (NEXT: the direction after MU, 4 when MU is the last). BAR:
+// the barrier of the three warps.
+template <int MU, int NEXT, int BAR, bool DAG, bool EO, bool AOS>
 __device__ __forceinline__ void ff_hops(const DArgs &a, int col, int lane, int x, const int c[4], FFShare &hs,
                                         double2 *stage, CAx2 &up, CAx2 &lo)
 {
@@ -396,7 +397,7 @@ __device__ __forceinline__ void ff_hops(const DArgs &a, int col, int lane, int x
     float4 wl[3];
 #pragma unroll
     for (int k = 0; k < 3; k++) wl[k] = __ldg(gf + lx + col * si + k * sk);
-    __syncthreads();
+    asm volatile("bar.sync %0, %1;" ::"n"(BAR), "n"(kFFThreads) : "memory");
     CAx2 u;  // U h for the two half-spinor components
 #pragma unroll
     for (int k = 0; k < 3; k++) {
@@ -434,6 +435,20 @@ __device__ __forceinline__ void ff_hops(const DArgs &a, int col, int lane, int x
   }
 }
 
+// the components of the forward hop of direction mu into stage 0
+template <bool EO, bool AOS>
+__device__ __forceinline__ void ff_first(const DArgs &a, int mu, int col, int x, const int c[4], double2 *stage)
+{
+  const double2 *sp = (const double2 *)a.in;
+  const int y = ff_nb(a, x, c, mu, false), ys = EO ? (y >> 1) : y;
+  const int b0 = (mu == 0 || mu == 3) ? 2 : 3;
+  const int comp[4] = {col, 3 + col, 3 * b0 + col, 3 * (5 - b0) + col};
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+    cp_async16(stage + i * kFFThreads, AOS ? sp + (int64_t)ys * 12 + comp[i] : sp + (int64_t)comp[i] * a.stride + ys);
+  cp_async_commit();
+}
+
 // EO: even/odd kernel on half fields (sites of parity a.eo_par; neighbours
 // read at (full index) >> 1) with the epilogue ch * [A^{-1}] H in + {z | A z};
 // SUMS: with the block sums of |out|^2 (a.partials)
@@ -449,28 +464,74 @@ __global__ void __launch_bounds__(kFFThreads, kFFMinBlocks) k_wilson_ff(const DA
   int c[4];
   const int x = ff_site<EO>(a, e, c);
   double2 *stage = staging + threadIdx.x;
-  {
-    const double2 *sp = (const double2 *)a.in;
-    const int y = ff_nb(a, x, c, 0, false), ys = EO ? (y >> 1) : y;
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-      cp_async16(stage + i * kFFThreads,
-                 AOS ? sp + (int64_t)ys * 12 + 3 * i + col : sp + (int64_t)(3 * i + col) * a.stride + ys);
-    cp_async_commit();
-  }
+  ff_first<EO, AOS>(a, 0, col, x, c, stage);
   const float2 z = make_float2(0.f, 0.f);
   CAx2 up{FAx2{z, z}, FAx2{z, z}}, lo = up;
-  ff_hops<0, 3, DAG, EO, AOS>(a, col, lane, x, c, hs, stage, up, lo);
-  ff_hops<3, 1, DAG, EO, AOS>(a, col, lane, x, c, hs, stage, up, lo);
+  ff_hops<0, 3, 0, DAG, EO, AOS>(a, col, lane, x, c, hs, stage, up, lo);
+  ff_hops<3, 1, 0, DAG, EO, AOS>(a, col, lane, x, c, hs, stage, up, lo);
   lo = CAx2{flip2(lo.re), flip2(lo.im)};
-  ff_hops<1, 2, DAG, EO, AOS>(a, col, lane, x, c, hs, stage, up, lo);
-  ff_hops<2, 4, DAG, EO, AOS>(a, col, lane, x, c, hs, stage, up, lo);
+  ff_hops<1, 2, 0, DAG, EO, AOS>(a, col, lane, x, c, hs, stage, up, lo);
+  ff_hops<2, 4, 0, DAG, EO, AOS>(a, col, lane, x, c, hs, stage, up, lo);
   lo = CAx2{flip2(lo.re), flip2(lo.im)};
   double n2 = 0.0;
   ff_store<0, EO, AOS, SUMS>(a, x, e, col, up, act, n2);
   ff_store<1, EO, AOS, SUMS>(a, x, e, col, lo, act, n2);
   if (SUMS) block_partial_cg(n2, a);
 }
+
+// The same for small lattices: four groups of three warps per 32 sites, one
+// direction each, whose sums meet in shared memory (the upper spins' in group
+// 0, the lower ones' in group 1, which store them). A lattice of a few hundred
+// blocks leaves the SMs nearly empty and its time is the chain of the eight
+// hops, here four chains of two (kernel times in a graph, one group against
+// four): 2,048 sites 7.6 and 5.0 us, 8^3 x 16 9.1 and 7.4, 16,384 sites 12.0 and
+// 13.3, 27,648 sites 16.5 and 19.6. The line lies where two blocks of four
+// groups per SM hold the lattice at once.
+constexpr int kFFGroups = 4;
+constexpr int kFFSmall = 2 * 152 * kFFSites;
+constexpr size_t kFF4Shared = kFFGroups * (sizeof(FFShare) + sizeof(double2) * 8 * kFFThreads);
+
+template <bool DAG, bool EO, bool AOS, bool SUMS>
+__global__ void __launch_bounds__(kFFGroups * kFFThreads, 2) k_wilson_ff4(const DArgs a)
+{
+  extern __shared__ __align__(16) char ff4_shared[];
+  const int grp = threadIdx.x / kFFThreads, t = threadIdx.x - grp * kFFThreads;
+  const int lane = t & 31, col = t >> 5;
+  const int id = a.x0 + blockIdx.x * kFFSites + lane;  // output index
+  const bool act = id < a.V;
+  const int e = act ? id : a.V - 1;  // idle lanes repeat the last site
+  FFShare &hs = ((FFShare *)ff4_shared)[grp];
+  double2 *stage = (double2 *)(ff4_shared + kFFGroups * sizeof(FFShare)) + grp * 8 * kFFThreads + t;
+  int c[4];
+  const int x = ff_site<EO>(a, e, c);
+  ff_first<EO, AOS>(a, grp, col, x, c, stage);
+  const float2 z = make_float2(0.f, 0.f);
+  CAx2 up{FAx2{z, z}, FAx2{z, z}}, lo = up;
+  if (grp == 0) ff_hops<0, 4, 1, DAG, EO, AOS>(a, col, lane, x, c, hs, stage, up, lo);
+  else if (grp == 1) ff_hops<1, 4, 2, DAG, EO, AOS>(a, col, lane, x, c, hs, stage, up, lo);
+  else if (grp == 2) ff_hops<2, 4, 3, DAG, EO, AOS>(a, col, lane, x, c, hs, stage, up, lo);
+  else ff_hops<3, 4, 4, DAG, EO, AOS>(a, col, lane, x, c, hs, stage, up, lo);
+  if (grp == 1 || grp == 2) lo = CAx2{flip2(lo.re), flip2(lo.im)};
+  __syncthreads();
+  CAx2 *sums = (CAx2 *)ff4_shared + t;  // [group][upper, lower][thread]: the exchange is done
+  sums[(2 * grp) * kFFThreads] = up;
+  sums[(2 * grp + 1) * kFFThreads] = lo;
+  __syncthreads();
+  double n2 = 0.0;
+  if (grp < 2) {
+    CAx2 s = sums[grp * kFFThreads];
+#pragma unroll
+    for (int g = 1; g < kFFGroups; g++) {
+      const CAx2 v = sums[(2 * g + grp) * kFFThreads];
+      acc_add2(s.re, v.re);
+      acc_add2(s.im, v.im);
+    }
+    if (grp == 0) ff_store<0, EO, AOS, SUMS>(a, x, e, col, s, act, n2);
+    else ff_store<1, EO, AOS, SUMS>(a, x, e, col, s, act, n2);
+  }
+  if (SUMS) block_partial_cg(n2, a);
+}
+static_assert(kFF4Shared >= sizeof(CAx2) * 2 * kFFGroups * kFFThreads, "the sums replace the exchange");
 
 // ------------------------------------------------------ float-pair links
 __global__ void k_gauge_to_ff(float4 *dst, int64_t dstride, const double2 *src, int64_t sstride, int64_t V,
@@ -520,10 +581,20 @@ bool gauge_to_ff(qcdgpu_gauge d, qcdgpu_gauge s)
   return QG_LAUNCHED("gauge_to_ff");
 }
 
+// the dynamic shared memory (73 KB) is opted in once per instantiation
 template <bool D, bool E, bool A, bool P>
 static void launch_ff(const DArgs &a)
 {
-  k_wilson_ff<D, E, A, P><<<(unsigned)((a.V - a.x0 + kFFSites - 1) / kFFSites), kFFThreads, 0, stream()>>>(a);
+  const int n = a.V - a.x0;
+  const unsigned grid = (unsigned)((n + kFFSites - 1) / kFFSites);
+  if (n > kFFSmall) {
+    k_wilson_ff<D, E, A, P><<<grid, kFFThreads, 0, stream()>>>(a);
+    return;
+  }
+  static const cudaError_t opted = cudaFuncSetAttribute(
+      k_wilson_ff4<D, E, A, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFF4Shared);
+  (void)opted;  // a failure shows in the launch
+  k_wilson_ff4<D, E, A, P><<<grid, kFFGroups * kFFThreads, kFF4Shared, stream()>>>(a);
 }
 
 int64_t dslash_df64_blocks(int64_t V) { return (V + kFFSites - 1) / kFFSites; }
