@@ -87,6 +87,22 @@ __global__ void __launch_bounds__(kCgThreads) k_cg_update(void *xs, float *xsn, 
   cg_last_block(partials, done, s, 1, hist);
 }
 
+// y += xs, xs = 0: the FP32 increment into the FP64 solution
+__global__ void __launch_bounds__(128) k_cg_flush(double2 *y, int64_t ystride, float4 *xs, int64_t stride, int V)
+{
+  const int x = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  if (x >= V) return;
+#pragma unroll
+  for (int j = 0; j < 6; j++) {
+    float4 &v = xs[j * stride + x];
+    double2 &a = y[(2 * j) * ystride + x], &b = y[(2 * j + 1) * ystride + x];
+    const float4 w = v;
+    a = make_double2(a.x + (double)w.x, a.y + (double)w.y);
+    b = make_double2(b.x + (double)w.z, b.y + (double)w.w);
+    v = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+}
+
 template <int P, typename R>
 __global__ void __launch_bounds__(128) k_cg_p(void *ps, float *psn, const void *rs, const float *rsn, int64_t stride,
                                               int V, const double *s)
@@ -125,10 +141,13 @@ struct CgOps {
   std::function<bool(qcdgpu_field, qcdgpu_field)> opdag;
   // FP64 storage (accurate arithmetic): out = A in, out = A^+ in
   std::function<bool(qcdgpu_field, qcdgpu_field)> op64, opdag64;
-  // optional: rs = A^+ rt in the inner precision with |rs|^2 (instead of
-  // opdag64 + conversion): the true residual rt is FP64-accurate, and its
-  // image only seeds the low-precision iteration
-  std::function<bool(qcdgpu_field, qcdgpu_field, double *)> restart;
+  // optional: a reliable update without the host in between. residual: rt = c -
+  // A y with |rt|^2 on the device at *res (partials in part); restart: rs = A^+
+  // rt in the inner precision with rr and beta on the device (mode 3 of
+  // cg_scalars_from). The true residual rt is FP64-accurate, and its image
+  // only seeds the low-precision iteration.
+  std::function<bool(qcdgpu_field rt, qcdgpu_field y, double *part, unsigned *done, double *res)> residual;
+  std::function<bool(qcdgpu_field rs, qcdgpu_field rt, double *part, unsigned *done, double *s)> restart;
 };
 
 struct Held {
@@ -211,14 +230,16 @@ static int cgnr_core(qcdgpu_field y, qcdgpu_field c, double cn, const CgOps &ops
   const unsigned nbr = (unsigned)((V + kCgSites - 1) / kCgSites);  // the fused reductions
   // one partial per block of the operator: 128 sites, fewer in the float-float kernel
   const int64_t nff = dslash_df64_blocks(V);
-  double *part = big_partials(prec == QCDGPU_F64 && nff > nb ? nff : nb);
+  double *part = big_partials(nff > nb ? nff : nb);
   double *s = reduce_scratch();
   double *h = host_result();
   if (!part || !s || !h) return 3;
   s += 2 * kMaxPartials + 16;  // 16 + kChunk slots past the blas result words
   unsigned *done = (unsigned *)(s + S_HIST + kChunk);  // block counters of the fused reductions
   cudaStream_t st = stream();
-  if (!QG_CUDA(cudaMemsetAsync(done, 0, 2 * sizeof(unsigned), st))) return 3;
+  if (!QG_CUDA(cudaMemsetAsync(s, 0, sizeof(double) * S_HIST, st)) ||
+      !QG_CUDA(cudaMemsetAsync(done, 0, 4 * sizeof(unsigned), st)))
+    return 3;
   if (!blas_zero(y)) return 3;
   // true residual rt = c - A y (FP64), returns |rt| / cn
   auto true_res = [&](double *rel) -> bool {
@@ -232,10 +253,14 @@ static int cgnr_core(qcdgpu_field y, qcdgpu_field c, double cn, const CgOps &ops
   auto restart_residual = [&](double *rr_out) -> bool {
     double rr;
     if (ops.restart) {
-      if (!ops.restart(rs, rt, &rr)) return false;
-    } else if (!ops.opdag64(r, rt) || !blas_norm2(r, &rr) || !convert_field(rs, r)) {
-      return false;
+      if (!ops.restart(rs, rt, part, done + 2, s) ||
+          !QG_CUDA(cudaMemcpyAsync(h, s + S_RR, sizeof(double), cudaMemcpyDeviceToHost, st)) ||
+          !QG_CUDA(cudaStreamSynchronize(st)))
+        return false;
+      *rr_out = h[0];
+      return true;
     }
+    if (!ops.opdag64(r, rt) || !blas_norm2(r, &rr) || !convert_field(rs, r)) return false;
     h[0] = rr;
     if (!QG_CUDA(cudaMemcpyAsync(s + S_RR, h, sizeof(double), cudaMemcpyHostToDevice, st))) return false;
     if (!QG_CUDA(cudaStreamSynchronize(st))) return false;
@@ -265,7 +290,7 @@ static int cgnr_core(qcdgpu_field y, qcdgpu_field c, double cn, const CgOps &ops
       first = false;
       // p^+ A^+ A p = |A p|^2, summed in the epilogue of the first operator;
       // its last block forms alpha
-      const CgFuse fz{done, s, j};
+      const CgFuse fz{done, s, j, 0};
       if (!ops.op(t, ps, part, &fz) || !ops.opdag(aps, t)) return false;
 #define QG_CG_UPD(P, R)                                                                                           \
   k_cg_update<P, R><<<nbr, kCgThreads, 0, st>>>(xs->data, xs->norm, ps->data, ps->norm, rs->data, rs->norm, aps->data, \
@@ -308,19 +333,30 @@ static int cgnr_core(qcdgpu_field y, qcdgpu_field c, double cn, const CgOps &ops
     bool last = p->iters >= p->maxiter;
     if (update || hinted || last) {
       if (prec == QCDGPU_F64) {
-        if (!blas_axpby(y, 1.0, 0.0, xs, 1.0, 0.0, y)) return 3;
+        if (!blas_axpby(y, 1.0, 0.0, xs, 1.0, 0.0, y) || !blas_zero(xs)) return 3;
       } else {
-        if (!convert_field(up, xs) || !blas_axpby(y, 1.0, 0.0, up, 1.0, 0.0, y)) return 3;
+        k_cg_flush<<<nb, 128, 0, st>>>((double2 *)y->data, y->stride, (float4 *)xs->data, xs->stride, V);
+        if (!QG_LAUNCHED("cg_flush")) return 3;
       }
-      if (!blas_zero(xs)) return 3;
-      double rel;
-      if (!true_res(&rel)) return 3;
-      p->true_residual = rel;
       p->reliable_updates++;
       since_update = 0;
+      if (hinted) hint = rn * 0.3;
+      double rel;
+      if (ops.restart) {  // residual and restart in one go (the restart is not used when converged)
+        if (!ops.residual(rt, y, part, done + 2, s + S_RES) || !ops.restart(rs, rt, part, done + 2, s) ||
+            !QG_CUDA(cudaMemcpyAsync(h, s, sizeof(double) * S_HIST, cudaMemcpyDeviceToHost, st)) ||
+            !QG_CUDA(cudaStreamSynchronize(st)))
+          return 3;
+        rel = p->true_residual = sqrt(h[S_RES]) / cn;
+        if (rel <= p->tol) return 0;
+        if (last) return 1;
+        maxr = sqrt(h[S_RR]);
+        continue;
+      }
+      if (!true_res(&rel)) return 3;
+      p->true_residual = rel;
       if (rel <= p->tol) return 0;
       if (last) return 1;
-      if (hinted) hint = rn * 0.3;
       if (!restart_residual(&rr)) return 3;
       // the next direction p = r_true + beta' p with beta' = |r_true|^2 / |r_prev|^2,
       // where |r_prev|^2 = rr_iter / beta_iter is the residual before the last iteration
@@ -424,10 +460,18 @@ int solve_cgnr_eo(qcdgpu_field x, qcdgpu_field b, qcdgpu_gauge g, double mp4, do
     return dslash_eo(t64, i, nullptr, g, mp4, tm, true, 1, 1.0, true, 0, nullptr, ar) &&
            dslash_eo(o, t64, i, g, mp4, tm, true, 0, -0.25, false, 2, nullptr, ar);
   };
-  if (prec != QCDGPU_F64)
-    ops.restart = [&](qcdgpu_field rs, qcdgpu_field rt, double *rr) {
-      return convert_field(tin, rt) && ops.opdag(rs, tin) && blas_norm2(rs, rr);
+  if (prec != QCDGPU_F64) {
+    ops.residual = [&](qcdgpu_field rt, qcdgpu_field y, double *part, unsigned *done, double *res) {
+      const CgFuse fz{done, res, 0, 2};
+      return dslash_eo(t64, y, nullptr, g, mp4, tm, false, 1, 1.0, true, 0, nullptr, ar) &&
+             dslash_eo(rt, t64, y, g, mp4, tm, false, 0, -0.25, false, 3, part, ar, &fz, ce);
     };
+    ops.restart = [&](qcdgpu_field rs, qcdgpu_field rt, double *part, unsigned *done, double *s) {
+      const CgFuse fz{done, s, 0, 3};
+      return convert_field(tin, rt) && dslash_eo(ti, tin, nullptr, gi, mp4, tm, true, 1, 1.0, true, 0, nullptr, ar) &&
+             dslash_eo(rs, ti, tin, gi, mp4, tm, true, 0, -0.25, false, 2, part, ar, &fz);
+    };
+  }
   const int st = cgnr_core(xe, ce, sqrt(bn2), ops, p);
   if (st == 3) return 3;
   // x_o = A^{-1} b_o + A^{-1} H_oe x_e / 2, then the full true residual

@@ -47,6 +47,7 @@ static bool dslash_once(qcdgpu_field out, qcdgpu_field in, qcdgpu_gauge g, doubl
     a.cg_done = fuse->done;
     a.cg_s = fuse->s;
     a.cg_hist = fuse->hist;
+    a.cg_mode = fuse->mode;
   }
   a.x0 = x0;
   a.out = out->data;
@@ -142,14 +143,17 @@ bool dslash(qcdgpu_field out, qcdgpu_field in, qcdgpu_gauge g, double mp4, doubl
 // Even/odd kernel on half fields (FP64, FP32 or FP16 with a gauge field of
 // the same precision): out (parity par) = ch * [A^{-1}] H in + {0 | z | A z}
 // with A = mp4 + i tm g5 (D^+: tm -> -tm and the hopping term of D^+).
-// in, out, z are fields on the half lattice {L_t / 2, L_x, L_y, L_z}.
+// in, out, z are fields on the half lattice {L_t / 2, L_x, L_y, L_z}. zmode 3
+// (FP64 fields, float-float arithmetic): out = w - (ch H in + A z).
 bool dslash_eo(qcdgpu_field out, qcdgpu_field in, qcdgpu_field z, qcdgpu_gauge g, double mp4, double tm, bool dag,
-               int par, double ch, bool ainv, int zmode, double *partials, int arith, const CgFuse *fuse)
+               int par, double ch, bool ainv, int zmode, double *partials, int arith, const CgFuse *fuse, qcdgpu_field w)
 {
   if (!out || !in || !g || out == in || (zmode && (!z || z == out)) || in->prec != out->prec ||
       in->prec != g->prec || (z && z->prec != in->prec) || !eo_lattice(g->L) || in->L[0] * 2 != g->L[0] ||
       in->L[1] != g->L[1] || in->L[2] != g->L[2] || in->L[3] != g->L[3] || !same_shape(out, in) ||
-      (z && !same_shape(z, in))) {
+      (z && !same_shape(z, in)) ||
+      (zmode == 3 && (!w || !same_shape(w, in) || in->prec != QCDGPU_F64 || w->prec != QCDGPU_F64 ||
+                      arith != QCDGPU_ARITH_DF64 || ainv))) {
     set_error("even/odd operator: half fields of one precision on the gauge field's half lattice (every extent "
               "even)");
     return false;
@@ -160,6 +164,7 @@ bool dslash_eo(qcdgpu_field out, qcdgpu_field in, qcdgpu_field z, qcdgpu_gauge g
     a.cg_done = fuse->done;
     a.cg_s = fuse->s;
     a.cg_hist = fuse->hist;
+    a.cg_mode = fuse->mode;
   }
   a.x0 = 0;
   a.out = out->data;
@@ -168,6 +173,12 @@ bool dslash_eo(qcdgpu_field out, qcdgpu_field in, qcdgpu_field z, qcdgpu_gauge g
   a.in_norm = in->norm;
   a.z = z ? z->data : nullptr;
   a.z_norm = z ? z->norm : nullptr;
+  a.w = w ? w->data : nullptr;
+  if (zmode == 3) {
+    ch = -ch;
+    mp4 = -mp4;
+    tm = -tm;
+  }
   a.gauge = g->data;
   for (int i = 0; i < 4; i++) a.geo.L[i] = g->L[i];
   a.geo.st[0] = 1;

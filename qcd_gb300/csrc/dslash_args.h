@@ -30,7 +30,8 @@ struct DArgs {
   int eo_par;
   const void *z;
   const float *z_norm;
-  int zmode;  // 0: no addend, 1: + z, 2: + A z
+  int zmode;  // 0: no addend, 1: + z, 2: + A z, 3: + A z + w (float-float kernel)
+  const void *w;
   int ainv;   // 1: hopping term multiplied by A^{-1}
   double ch, ai_r, ai_i;  // A^{-1} = ai_r + i ai_i g5
   float ch_h, ch_l, ai_r_h, ai_r_l, ai_i_h, ai_i_l;
@@ -39,17 +40,18 @@ struct DArgs {
   // sites (full-lattice float-float kernel only)
   int aos = 0;
   // non-null (with partials): the CG step alpha = rr / (sum of the partials)
-  // is formed by the block that finishes last (cg_last_block, mode 0)
+  // (or what cg_mode says) is formed by the block that finishes last (cg_last_block)
   unsigned *cg_done = nullptr;
   double *cg_s = nullptr;
-  int cg_hist = 0;
+  int cg_hist = 0, cg_mode = 0;
 };
 
-// the CG scalars a launch of the operator may update at its end
+// the scalars a launch of the operator may update at its end, from the sum of
+// its partials (cg_scalars_from)
 struct CgFuse {
   unsigned *done;  // arrival counter (zero between launches)
-  double *s;       // the solver's scalar slots
-  int hist;
+  double *s;       // the solver's scalar slots; mode 2: where the sum goes
+  int hist, mode = 0;
 };
 
 // |v|^2 summed over the block into partials[blockIdx.x]; every thread of the
@@ -68,20 +70,27 @@ __device__ __forceinline__ void block_partial(double v, double *partials)
 }
 
 // scalar slots
-enum { S_RR = 0, S_PAP = 1, S_RRNEW = 2, S_ALPHA = 3, S_BETA = 4, S_HIST = 8 };
+enum { S_RR = 0, S_PAP = 1, S_RRNEW = 2, S_ALPHA = 3, S_BETA = 4, S_RES = 5, S_HIST = 8 };
 
 // the CG scalars from a reduced total: mode 0 t = p^+ A p -> alpha;
-// mode 1 t = |r|^2 -> beta and the residual history
+// mode 1 t = |r|^2 -> beta and the residual history; mode 2 the total itself;
+// mode 3 t = |r|^2 of a restarted residual: beta' = t / |r_prev|^2 with
+// |r_prev|^2 = rr / beta, the residual before the last iteration
 __device__ __forceinline__ void cg_scalars_from(double t, double *s, int mode, int hist)
 {
   if (mode == 0) {
     s[S_PAP] = t;
     s[S_ALPHA] = t > 0.0 ? s[S_RR] / t : nan("");  // p^+ A p <= 0: breakdown
-  } else {
+  } else if (mode == 1) {
     s[S_RRNEW] = t;
     s[S_BETA] = t / s[S_RR];
     s[S_RR] = t;
     s[S_HIST + hist] = t;
+  } else if (mode == 2) {
+    s[0] = t;
+  } else {
+    s[S_BETA] = s[S_BETA] > 0.0 && s[S_RR] > 0.0 ? t * s[S_BETA] / s[S_RR] : 0.0;
+    s[S_RR] = t;
   }
 }
 
@@ -129,7 +138,7 @@ __device__ __forceinline__ void cg_last_block(const double *partials, unsigned *
 __device__ __forceinline__ void block_partial_cg(double v, const DArgs &a)
 {
   block_partial(v, a.partials);
-  if (a.cg_done) cg_last_block(a.partials, a.cg_done, a.cg_s, 0, a.cg_hist);
+  if (a.cg_done) cg_last_block(a.partials, a.cg_done, a.cg_s, a.cg_mode, a.cg_hist);
 }
 
 // a launch scalar in the kernel's arithmetic type R

@@ -304,7 +304,7 @@ __device__ __forceinline__ void ff_store(const DArgs &a, int x, int e, int i, CA
       const double2 z0 = __ldg(z + (int64_t)k0 * a.stride + e), z1 = __ldg(z + (int64_t)k1 * a.stride + e);
       F2x2 zr, zi;
       split_pair(z0, z1, zr, zi);
-      if (a.zmode == 2) {  // + (m+4) z + i tm g5 z
+      if (a.zmode >= 2) {  // + (m+4) z + i tm g5 z
         mac2(re, mp4, neg2(mp4.h), zr);
         mac2(re, neg2(tp), tp.h, zi);
         mac2(im, mp4, neg2(mp4.h), zi);
@@ -312,6 +312,13 @@ __device__ __forceinline__ void ff_store(const DArgs &a, int x, int e, int i, CA
       } else {
         acc_add2(re, FAx2{zr.h, zr.l});
         acc_add2(im, FAx2{zi.h, zi.l});
+      }
+      if (a.zmode == 3) {
+        const double2 *w = (const double2 *)a.w;
+        F2x2 wr, wi;
+        split_pair(__ldg(w + (int64_t)k0 * a.stride + e), __ldg(w + (int64_t)k1 * a.stride + e), wr, wi);
+        acc_add2(re, FAx2{wr.h, wr.l});
+        acc_add2(im, FAx2{wi.h, wi.l});
       }
     }
     dr = fin2(re);

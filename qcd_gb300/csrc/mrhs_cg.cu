@@ -23,6 +23,7 @@
 
 #include <vector>
 
+#include "dslash_args.h"
 #include "mrhs.h"
 
 namespace qg {
@@ -400,13 +401,15 @@ static bool slot_residual(qcdgpu_batch B, int k, const BSlot &sl, double *res)
   if (B->eo) {
     qcdgpu_gauge g32 = gauge_at(B->g, QCDGPU_F32);
     const int ar = QCDGPU_ARITH_DF64;
+    // the norms come with the residual and the restart residual
+    const CgFuse f0{B->msdone + 1, res, 0, 2}, f1{B->msdone + 1, res + 2, 0, 2};
     return g32 && dslash_eo(B->u64, sl.xe, nullptr, B->g, sl.mp4, sl.tm, false, 1, 1.0, true, 0, nullptr, ar) &&
-           dslash_eo(B->rt, B->u64, sl.xe, B->g, sl.mp4, sl.tm, false, 0, -0.25, false, 2, nullptr, ar) &&
-           blas_axpby(B->rt, 1.0, 0.0, sl.ce, -1.0, 0.0, B->rt) && blas_norm2_dev(B->rt, res) &&
+           dslash_eo(B->rt, B->u64, sl.xe, B->g, sl.mp4, sl.tm, false, 0, -0.25, false, 3, B->part, ar, &f0, sl.ce) &&
            convert_field(B->r32, B->rt) &&
            dslash_eo(B->u32, B->r32, nullptr, g32, sl.mp4, sl.tm, true, 1, 1.0, true, 0, nullptr) &&
-           dslash_eo(B->s32, B->u32, B->r32, g32, sl.mp4, sl.tm, true, 0, -0.25, false, 2, nullptr) &&
-           blas_norm2_dev(B->s32, res + 2) && mfield_set(B->rs, k, B->s32);
+           dslash_eo(B->s32, B->u32, B->r32, g32, sl.mp4, sl.tm, true, 0, -0.25, false, 2, B->part, QCDGPU_ARITH_F64,
+                     &f1) &&
+           mfield_set(B->rs, k, B->s32);
   }
   return slot_bd(B, sl) && dslash(B->rt, sl.x, B->g, sl.mp4, sl.tm, QCDGPU_OP_D, QCDGPU_ARITH_DF64) &&
          blas_axpby(B->rt, 1.0, 0.0, B->bd, -1.0, 0.0, B->rt) && blas_norm2_dev(B->rt, res) &&
