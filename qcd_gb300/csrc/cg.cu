@@ -7,9 +7,9 @@
 // for the even/odd operator, whose A is two hops) and no host
 // synchronisation:
 //   1. t = A p            (operator kernel; its epilogue also sums |t|^2 =
-//                          p^+ A^+ A p per block, and the block that
-//                          finishes last forms alpha = rr / pAp)
-//   2. Ap = A^+ t         (operator kernel)
+//                          p^+ A^+ A p per block)
+//   2. Ap = A^+ t         (operator kernel; one block of its first launch adds
+//                          those sums up and forms alpha = rr / pAp)
 //   3. update kernel:     x' += alpha p, r -= alpha Ap, per-block |r|^2; its
 //                          last block forms rr', beta = rr'/rr, history[i]
 //   4. p = r + beta p     (reads beta from device memory)
@@ -36,7 +36,7 @@ namespace qg {
 using namespace qgd;
 
 bool dslash_partials(qcdgpu_field out, qcdgpu_field in, qcdgpu_gauge g, double mp4, double tm, bool dag,
-                     int arith, double *partials, const CgFuse *fuse = nullptr);
+                     int arith, double *partials, const CgReduce *red = nullptr);
 double *big_partials(int64_t n);
 int64_t dslash_df64_blocks(int64_t V);
 
@@ -132,22 +132,37 @@ __global__ void __launch_bounds__(128) k_cg_p(void *ps, float *psn, const void *
   } while (0)
 
 
+__global__ void __launch_bounds__(512) k_cg_total(CgReduce r) { cg_sum(r); }
+
+bool cg_total(const CgReduce &r)
+{
+  k_cg_total<<<1, 512, 0, stream()>>>(r);
+  return QG_LAUNCHED("cg_total");
+}
+
+// partials an operator launch over V sites leaves, by storage and FP64 arithmetic
+static int64_t partial_blocks(int64_t V, int prec, int arith)
+{
+  return prec == QCDGPU_F64 && arith == QCDGPU_ARITH_DF64 ? dslash_df64_blocks(V) : (V + 127) / 128;
+}
+
 // Operators of the system A y = c that cgnr_core solves through A^+ A.
 struct CgOps {
   int L[4];  // lattice of the system's fields (the half lattice for even/odd)
-  // inner precision: t = A p (with partials: |t|^2 per 128-site block, and
-  // with fuse the CG step from them), aps = A^+ t
-  std::function<bool(qcdgpu_field, qcdgpu_field, double *, const CgFuse *)> op;
-  std::function<bool(qcdgpu_field, qcdgpu_field)> opdag;
+  // inner precision: t = A p (with |t|^2 per block in the partials, `parts` of
+  // them), aps = A^+ t (red: partials its first launch adds up)
+  std::function<bool(qcdgpu_field, qcdgpu_field, double *)> op;
+  std::function<bool(qcdgpu_field, qcdgpu_field, const CgReduce *)> opdag;
+  int64_t parts;
   // FP64 storage (accurate arithmetic): out = A in, out = A^+ in
   std::function<bool(qcdgpu_field, qcdgpu_field)> op64, opdag64;
   // optional: a reliable update without the host in between. residual: rt = c -
-  // A y with |rt|^2 on the device at *res (partials in part); restart: rs = A^+
-  // rt in the inner precision with rr and beta on the device (mode 3 of
-  // cg_scalars_from). The true residual rt is FP64-accurate, and its image
-  // only seeds the low-precision iteration.
-  std::function<bool(qcdgpu_field rt, qcdgpu_field y, double *part, unsigned *done, double *res)> residual;
-  std::function<bool(qcdgpu_field rs, qcdgpu_field rt, double *part, unsigned *done, double *s)> restart;
+  // A y with |rt|^2 in the partials; restart: rs = A^+ rt in the inner precision
+  // (red: as for opdag), with rr and beta in s (mode 3 of cg_scalars_from). The
+  // true residual rt is FP64-accurate, and its image only seeds the
+  // low-precision iteration.
+  std::function<bool(qcdgpu_field rt, qcdgpu_field y, double *part)> residual;
+  std::function<bool(qcdgpu_field rs, qcdgpu_field rt, double *part, const CgReduce *red, double *s)> restart;
 };
 
 struct Held {
@@ -235,10 +250,10 @@ static int cgnr_core(qcdgpu_field y, qcdgpu_field c, double cn, const CgOps &ops
   double *h = host_result();
   if (!part || !s || !h) return 3;
   s += 2 * kMaxPartials + 16;  // 16 + kChunk slots past the blas result words
-  unsigned *done = (unsigned *)(s + S_HIST + kChunk);  // block counters of the fused reductions
+  unsigned *done = (unsigned *)(s + S_HIST + kChunk);  // block counter of the update's reduction
   cudaStream_t st = stream();
   if (!QG_CUDA(cudaMemsetAsync(s, 0, sizeof(double) * S_HIST, st)) ||
-      !QG_CUDA(cudaMemsetAsync(done, 0, 4 * sizeof(unsigned), st)))
+      !QG_CUDA(cudaMemsetAsync(done, 0, sizeof(unsigned), st)))
     return 3;
   if (!blas_zero(y)) return 3;
   // true residual rt = c - A y (FP64), returns |rt| / cn
@@ -253,7 +268,7 @@ static int cgnr_core(qcdgpu_field y, qcdgpu_field c, double cn, const CgOps &ops
   auto restart_residual = [&](double *rr_out) -> bool {
     double rr;
     if (ops.restart) {
-      if (!ops.restart(rs, rt, part, done + 2, s) ||
+      if (!ops.restart(rs, rt, part, nullptr, s) ||
           !QG_CUDA(cudaMemcpyAsync(h, s + S_RR, sizeof(double), cudaMemcpyDeviceToHost, st)) ||
           !QG_CUDA(cudaStreamSynchronize(st)))
         return false;
@@ -288,13 +303,13 @@ static int cgnr_core(qcdgpu_field y, qcdgpu_field c, double cn, const CgOps &ops
         if (!QG_LAUNCHED("cg_p")) return false;
       }
       first = false;
-      // p^+ A^+ A p = |A p|^2, summed in the epilogue of the first operator;
-      // its last block forms alpha
-      const CgFuse fz{done, s, j, 0};
-      if (!ops.op(t, ps, part, &fz) || !ops.opdag(aps, t)) return false;
+      // p^+ A^+ A p = |A p|^2, summed in the epilogue of the first operator and
+      // added up beside the second
+      const CgReduce pap{part, (int)ops.parts, s, 0, j};
+      if (!ops.op(t, ps, part) || !ops.opdag(aps, t, &pap)) return false;
 #define QG_CG_UPD(P, R)                                                                                           \
   k_cg_update<P, R><<<nbr, kCgThreads, 0, st>>>(xs->data, xs->norm, ps->data, ps->norm, rs->data, rs->norm, aps->data, \
-                                                aps->norm, xs->stride, V, s, part, done + 1, j)
+                                                aps->norm, xs->stride, V, s, part, done, j)
       // x += alpha p, r -= alpha A p, with |r|^2 and beta
       if (prec == QCDGPU_F64) QG_CG_UPD(QCDGPU_F64, double);
       else if (prec == QCDGPU_F32) QG_CG_UPD(QCDGPU_F32, float);
@@ -343,7 +358,8 @@ static int cgnr_core(qcdgpu_field y, qcdgpu_field c, double cn, const CgOps &ops
       if (hinted) hint = rn * 0.3;
       double rel;
       if (ops.restart) {  // residual and restart in one go (the restart is not used when converged)
-        if (!ops.residual(rt, y, part, done + 2, s + S_RES) || !ops.restart(rs, rt, part, done + 2, s) ||
+        const CgReduce res{part, (int)nff, s + S_RES, 2, 0};
+        if (!ops.residual(rt, y, part) || !ops.restart(rs, rt, part, &res, s) ||
             !QG_CUDA(cudaMemcpyAsync(h, s, sizeof(double) * S_HIST, cudaMemcpyDeviceToHost, st)) ||
             !QG_CUDA(cudaStreamSynchronize(st)))
           return 3;
@@ -395,10 +411,13 @@ int solve_cgnr_engine(qcdgpu_field x, qcdgpu_field b, qcdgpu_gauge g, double mp4
   if (!bd || !gi) return 3;
   CgOps ops;
   memcpy(ops.L, b->L, sizeof(ops.L));
-  ops.op = [&](qcdgpu_field o, qcdgpu_field i, double *part, const CgFuse *fuse) {
-    return dslash_partials(o, i, gi, mp4, tm, false, -1, part, fuse);
+  ops.op = [&](qcdgpu_field o, qcdgpu_field i, double *part) {
+    return dslash_partials(o, i, gi, mp4, tm, false, -1, part);
   };
-  ops.opdag = [&](qcdgpu_field o, qcdgpu_field i) { return dslash_partials(o, i, gi, mp4, tm, true, -1, nullptr); };
+  ops.opdag = [&](qcdgpu_field o, qcdgpu_field i, const CgReduce *red) {
+    return dslash_partials(o, i, gi, mp4, tm, true, -1, nullptr, red);
+  };
+  ops.parts = partial_blocks(b->V, p->inner_prec, g_f64_arith);
   ops.op64 = [&](qcdgpu_field o, qcdgpu_field i) { return dslash(o, i, g, mp4, tm, QCDGPU_OP_D, QCDGPU_ARITH_DF64); };
   ops.opdag64 = [&](qcdgpu_field o, qcdgpu_field i) {
     return dslash(o, i, g, mp4, tm, QCDGPU_OP_DDAG, QCDGPU_ARITH_DF64);
@@ -444,12 +463,13 @@ int solve_cgnr_eo(qcdgpu_field x, qcdgpu_field b, qcdgpu_gauge g, double mp4, do
   CgOps ops;
   memcpy(ops.L, Lh, sizeof(ops.L));
   const int ar = QCDGPU_ARITH_DF64;  // FP64 fields: float-float arithmetic
-  ops.op = [&](qcdgpu_field o, qcdgpu_field i, double *part, const CgFuse *fuse) {
+  ops.op = [&](qcdgpu_field o, qcdgpu_field i, double *part) {
     return dslash_eo(ti, i, nullptr, gi, mp4, tm, false, 1, 1.0, true, 0, nullptr, ar) &&
-           dslash_eo(o, ti, i, gi, mp4, tm, false, 0, -0.25, false, 2, part, ar, fuse);
+           dslash_eo(o, ti, i, gi, mp4, tm, false, 0, -0.25, false, 2, part, ar);
   };
-  ops.opdag = [&](qcdgpu_field o, qcdgpu_field i) {
-    return dslash_eo(ti, i, nullptr, gi, mp4, tm, true, 1, 1.0, true, 0, nullptr, ar) &&
+  ops.parts = partial_blocks(be->V, prec, ar);
+  ops.opdag = [&](qcdgpu_field o, qcdgpu_field i, const CgReduce *red) {
+    return dslash_eo(ti, i, nullptr, gi, mp4, tm, true, 1, 1.0, true, 0, nullptr, ar, red) &&
            dslash_eo(o, ti, i, gi, mp4, tm, true, 0, -0.25, false, 2, nullptr, ar);
   };
   ops.op64 = [&](qcdgpu_field o, qcdgpu_field i) {
@@ -461,15 +481,15 @@ int solve_cgnr_eo(qcdgpu_field x, qcdgpu_field b, qcdgpu_gauge g, double mp4, do
            dslash_eo(o, t64, i, g, mp4, tm, true, 0, -0.25, false, 2, nullptr, ar);
   };
   if (prec != QCDGPU_F64) {
-    ops.residual = [&](qcdgpu_field rt, qcdgpu_field y, double *part, unsigned *done, double *res) {
-      const CgFuse fz{done, res, 0, 2};
+    ops.residual = [&](qcdgpu_field rt, qcdgpu_field y, double *part) {
       return dslash_eo(t64, y, nullptr, g, mp4, tm, false, 1, 1.0, true, 0, nullptr, ar) &&
-             dslash_eo(rt, t64, y, g, mp4, tm, false, 0, -0.25, false, 3, part, ar, &fz, ce);
+             dslash_eo(rt, t64, y, g, mp4, tm, false, 0, -0.25, false, 3, part, ar, nullptr, ce);
     };
-    ops.restart = [&](qcdgpu_field rs, qcdgpu_field rt, double *part, unsigned *done, double *s) {
-      const CgFuse fz{done, s, 0, 3};
-      return convert_field(tin, rt) && dslash_eo(ti, tin, nullptr, gi, mp4, tm, true, 1, 1.0, true, 0, nullptr, ar) &&
-             dslash_eo(rs, ti, tin, gi, mp4, tm, true, 0, -0.25, false, 2, part, ar, &fz);
+    ops.restart = [&](qcdgpu_field rs, qcdgpu_field rt, double *part, const CgReduce *red, double *s) {
+      return convert_field(tin, rt) &&
+             dslash_eo(ti, tin, nullptr, gi, mp4, tm, true, 1, 1.0, true, 0, nullptr, ar, red) &&
+             dslash_eo(rs, ti, tin, gi, mp4, tm, true, 0, -0.25, false, 2, part, ar) &&
+             cg_total(CgReduce{part, (int)ops.parts, s, 3, 0});
     };
   }
   const int st = cgnr_core(xe, ce, sqrt(bn2), ops, p);

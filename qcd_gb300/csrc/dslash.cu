@@ -21,17 +21,34 @@ using namespace qgd;
 // float-float kernel for FP64 storage (dslash_df64.cu)
 bool dslash_df64(const DArgs &a, bool dag, bool eo = false);
 
+// the kernel's mode (wilson_kernel.cuh) from the launch's reductions
+template <bool DAG, int SP, int RECON, typename R>
+static void launch_full(const DArgs &a, unsigned grid)
+{
+  cudaStream_t s = stream();
+  if (a.partials) k_wilson<DAG, SP, RECON, R, 1><<<grid, 128, 0, s>>>(a);
+  else if (a.red.n) k_wilson<DAG, SP, RECON, R, 2><<<grid + 1, 128, 0, s>>>(a);
+  else k_wilson<DAG, SP, RECON, R, 0><<<grid, 128, 0, s>>>(a);
+}
+template <bool DAG, int SP, int RECON, typename R>
+static void launch_half(const DArgs &a, unsigned grid)
+{
+  cudaStream_t s = stream();
+  if (a.partials) k_wilson_eo<DAG, SP, RECON, R, 1><<<grid, 128, 0, s>>>(a);
+  else if (a.red.n) k_wilson_eo<DAG, SP, RECON, R, 2><<<grid + 1, 128, 0, s>>>(a);
+  else k_wilson_eo<DAG, SP, RECON, R, 0><<<grid, 128, 0, s>>>(a);
+}
+
 template <bool DAG>
 static bool launch_native(const DArgs &a, int prec, int recon)
 {
-  unsigned grid = (unsigned)((a.V - a.x0 + 127) / 128);
-  cudaStream_t s = stream();
+  const unsigned grid = (unsigned)((a.V - a.x0 + 127) / 128);
   // FP64 arithmetic is the bottleneck of the native FP64 kernel (GB300 runs
   // DFMA at ~1/60 of the FP32 rate): read all 18 link reals, no rebuild
-  if (prec == QCDGPU_F64) k_wilson<DAG, QCDGPU_F64, QCDGPU_F64, 18, double><<<grid, 128, 0, s>>>(a);
-  else if (prec == QCDGPU_F32 && recon == 12) k_wilson<DAG, QCDGPU_F32, QCDGPU_F32, 12, float><<<grid, 128, 0, s>>>(a);
-  else if (prec == QCDGPU_F32) k_wilson<DAG, QCDGPU_F32, QCDGPU_F32, 18, float><<<grid, 128, 0, s>>>(a);
-  else k_wilson<DAG, QCDGPU_F16, QCDGPU_F16, 12, float><<<grid, 128, 0, s>>>(a);
+  if (prec == QCDGPU_F64) launch_full<DAG, QCDGPU_F64, 18, double>(a, grid);
+  else if (prec == QCDGPU_F32 && recon == 12) launch_full<DAG, QCDGPU_F32, 12, float>(a, grid);
+  else if (prec == QCDGPU_F32) launch_full<DAG, QCDGPU_F32, 18, float>(a, grid);
+  else launch_full<DAG, QCDGPU_F16, 12, float>(a, grid);
   return QG_LAUNCHED("wilson");
 }
 
@@ -39,16 +56,11 @@ static bool launch_native(const DArgs &a, int prec, int recon)
 // the host layout at these device addresses instead of in / out's data
 static bool dslash_once(qcdgpu_field out, qcdgpu_field in, qcdgpu_gauge g, double mp4, double tm,
                         bool dag, bool q, int arith, double *partials = nullptr, int x0 = 0, int x1 = -1,
-                        const void *in_aos = nullptr, void *out_aos = nullptr, const CgFuse *fuse = nullptr)
+                        const void *in_aos = nullptr, void *out_aos = nullptr, const CgReduce *red = nullptr)
 {
   DArgs a;
   a.partials = partials;
-  if (partials && fuse) {
-    a.cg_done = fuse->done;
-    a.cg_s = fuse->s;
-    a.cg_hist = fuse->hist;
-    a.cg_mode = fuse->mode;
-  }
+  if (red) a.red = *red;
   a.x0 = x0;
   a.out = out->data;
   a.out_norm = out->norm;
@@ -146,7 +158,7 @@ bool dslash(qcdgpu_field out, qcdgpu_field in, qcdgpu_gauge g, double mp4, doubl
 // in, out, z are fields on the half lattice {L_t / 2, L_x, L_y, L_z}. zmode 3
 // (FP64 fields, float-float arithmetic): out = w - (ch H in + A z).
 bool dslash_eo(qcdgpu_field out, qcdgpu_field in, qcdgpu_field z, qcdgpu_gauge g, double mp4, double tm, bool dag,
-               int par, double ch, bool ainv, int zmode, double *partials, int arith, const CgFuse *fuse, qcdgpu_field w)
+               int par, double ch, bool ainv, int zmode, double *partials, int arith, const CgReduce *red, qcdgpu_field w)
 {
   if (!out || !in || !g || out == in || (zmode && (!z || z == out)) || in->prec != out->prec ||
       in->prec != g->prec || (z && z->prec != in->prec) || !eo_lattice(g->L) || in->L[0] * 2 != g->L[0] ||
@@ -160,12 +172,7 @@ bool dslash_eo(qcdgpu_field out, qcdgpu_field in, qcdgpu_field z, qcdgpu_gauge g
   }
   DArgs a;
   a.partials = partials;
-  if (partials && fuse) {
-    a.cg_done = fuse->done;
-    a.cg_s = fuse->s;
-    a.cg_hist = fuse->hist;
-    a.cg_mode = fuse->mode;
-  }
+  if (red) a.red = *red;
   a.x0 = 0;
   a.out = out->data;
   a.out_norm = out->norm;
@@ -224,10 +231,9 @@ bool dslash_eo(qcdgpu_field out, qcdgpu_field in, qcdgpu_field z, qcdgpu_gauge g
     return dslash_df64(a, dag, true);
   }
   const unsigned grid = (unsigned)((a.V + 127) / 128);
-  cudaStream_t s = stream();
-#define QG_EO(SP, RECON, R)                                                        \
-  if (dag) k_wilson_eo<true, SP, SP, RECON, R><<<grid, 128, 0, s>>>(a);            \
-  else k_wilson_eo<false, SP, SP, RECON, R><<<grid, 128, 0, s>>>(a);
+#define QG_EO(SP, RECON, R)                            \
+  if (dag) launch_half<true, SP, RECON, R>(a, grid);   \
+  else launch_half<false, SP, RECON, R>(a, grid);
   if (in->prec == QCDGPU_F64) {
     QG_EO(QCDGPU_F64, 18, double)
   } else if (in->prec == QCDGPU_F32 && g->recon == 12) {
@@ -272,14 +278,13 @@ bool dslash_sites_aos(void *out_aos, const void *in_aos, qcdgpu_field shape, qcd
 }
 
 // out = D in (dag: D^+ in) on fields checked by the caller; when partials is
-// non-null, block b of the launch (128 sites each) also writes the sum of
-// |out|^2 over its sites to partials[b], and with fuse the block that
-// finishes last forms the CG step from them
+// non-null, block b of the launch also writes the sum of |out|^2 over its sites
+// to partials[b]; red: partials of an earlier launch to add up meanwhile
 bool dslash_partials(qcdgpu_field out, qcdgpu_field in, qcdgpu_gauge g, double mp4, double tm, bool dag,
-                     int arith, double *partials, const CgFuse *fuse)
+                     int arith, double *partials, const CgReduce *red)
 {
   if (arith < 0) arith = g_f64_arith;
-  return dslash_once(out, in, g, mp4, tm, dag, false, arith, partials, 0, -1, nullptr, nullptr, fuse);
+  return dslash_once(out, in, g, mp4, tm, dag, false, arith, partials, 0, -1, nullptr, nullptr, red);
 }
 
 // float-float by default: GB300 runs FP64 at ~1/58 of its FP32 rate, and

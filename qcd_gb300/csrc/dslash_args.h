@@ -5,6 +5,18 @@
 
 namespace qg {
 
+// Partial sums that an operator launch adds up beside its own work, in a block
+// of its own (block 0, before the others' blocks), and the scalars it forms from
+// the total (cg_scalars_from; mode 2: the total goes to s[0]). The block sums
+// that an earlier launch left: no launch counts its blocks, which held every
+// block for a fence and an atomic and the last one for the sum.
+struct CgReduce {
+  const double *part = nullptr;
+  int n = 0;
+  double *s = nullptr;
+  int mode = 0, hist = 0;
+};
+
 struct DArgs {
   void *out;
   float *out_norm;
@@ -39,19 +51,7 @@ struct DArgs {
   // double (12 double2 per site), instead of component blocks of `stride`
   // sites (full-lattice float-float kernel only)
   int aos = 0;
-  // non-null (with partials): the CG step alpha = rr / (sum of the partials)
-  // (or what cg_mode says) is formed by the block that finishes last (cg_last_block)
-  unsigned *cg_done = nullptr;
-  double *cg_s = nullptr;
-  int cg_hist = 0, cg_mode = 0;
-};
-
-// the scalars a launch of the operator may update at its end, from the sum of
-// its partials (cg_scalars_from)
-struct CgFuse {
-  unsigned *done;  // arrival counter (zero between launches)
-  double *s;       // the solver's scalar slots; mode 2: where the sum goes
-  int hist, mode = 0;
+  CgReduce red;  // not with partials
 };
 
 // |v|^2 summed over the block into partials[blockIdx.x]; every thread of the
@@ -94,31 +94,19 @@ __device__ __forceinline__ void cg_scalars_from(double t, double *s, int mode, i
   }
 }
 
-// Called by every thread of a block after block_partial wrote the
-// block's partial: the block that finishes last sums all gridDim.x partials
-// in index order (the same order whichever block is last), updates the
-// scalars and re-arms the counter. No block waits for another.
-__device__ __forceinline__ void cg_last_block(const double *partials, unsigned *done, double *s, int mode, int hist)
+// every thread of a block: the sum of r.n partials in a fixed order (the same
+// for one block size) and the scalars from it; 24 independent loads in flight
+// per thread
+__device__ __forceinline__ void cg_sum(const CgReduce &r)
 {
-  __shared__ unsigned last;
   __shared__ double sh[32];
-  if (threadIdx.x == 0) {
-    __threadfence();  // this block's partial before its count
-    last = atomicAdd(done, 1u) == gridDim.x - 1 ? 1u : 0u;
-  }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  // 24 independent loads in flight per thread, summed in a fixed order: one
-  // round of loads for the half-lattice launches of 24^3 x 48 (2,592 partials)
-  const int n = (int)gridDim.x;
   double v = 0.0;
   const int nt = (int)blockDim.x;
   constexpr int kLoads = 24;
-  for (int i0 = threadIdx.x; i0 < n; i0 += kLoads * nt) {
+  for (int i0 = threadIdx.x; i0 < r.n; i0 += kLoads * nt) {
     double w[kLoads];
 #pragma unroll
-    for (int k = 0; k < kLoads; k++) w[k] = i0 + k * nt < n ? __ldcg(partials + i0 + k * nt) : 0.0;
+    for (int k = 0; k < kLoads; k++) w[k] = i0 + k * nt < r.n ? __ldcg(r.part + i0 + k * nt) : 0.0;
 #pragma unroll
     for (int k = 0; k < kLoads; k++) v += w[k];
   }
@@ -128,17 +116,38 @@ __device__ __forceinline__ void cg_last_block(const double *partials, unsigned *
   if (threadIdx.x == 0) {
     double t = 0.0;
     for (int i = 0; i < nt >> 5; i++) t += sh[i];
-    cg_scalars_from(t, s, mode, hist);
-    *done = 0u;
+    cg_scalars_from(t, r.s, r.mode, r.hist);
   }
 }
 
-// the kernels' end with partials: the block partial, then (cg_done) the CG
-// step from all of them
-__device__ __forceinline__ void block_partial_cg(double v, const DArgs &a)
+// the sum and its scalars in a launch of its own (cg.cu)
+bool cg_total(const CgReduce &r);
+
+// this block's index among the blocks of the operator's own work; block 0 of
+// a launch with partials to add adds them and returns -1
+__device__ __forceinline__ int work_block(const CgReduce &r)
 {
-  block_partial(v, a.partials);
-  if (a.cg_done) cg_last_block(a.partials, a.cg_done, a.cg_s, a.cg_mode, a.cg_hist);
+  if (r.n == 0) return (int)blockIdx.x;
+  if (blockIdx.x == 0) cg_sum(r);
+  return (int)blockIdx.x - 1;
+}
+
+// Called by every thread of a block after block_partial wrote the
+// block's partial: the block that finishes last sums all gridDim.x partials
+// in index order (the same order whichever block is last), updates the
+// scalars and re-arms the counter. No block waits for another.
+__device__ __forceinline__ void cg_last_block(const double *partials, unsigned *done, double *s, int mode, int hist)
+{
+  __shared__ unsigned last;
+  if (threadIdx.x == 0) {
+    __threadfence();  // this block's partial before its count
+    last = atomicAdd(done, 1u) == gridDim.x - 1 ? 1u : 0u;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  cg_sum(CgReduce{partials, (int)gridDim.x, s, mode, hist});
+  if (threadIdx.x == 0) *done = 0u;
 }
 
 // a launch scalar in the kernel's arithmetic type R

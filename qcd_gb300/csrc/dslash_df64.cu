@@ -462,8 +462,10 @@ __device__ __forceinline__ void ff_first(const DArgs &a, int mu, int col, int x,
 template <bool DAG, bool EO, bool AOS, bool SUMS>
 __global__ void __launch_bounds__(kFFThreads, kFFMinBlocks) k_wilson_ff(const DArgs a)
 {
+  const int block = SUMS ? (int)blockIdx.x : work_block(a.red);
+  if (block < 0) return;
   const int lane = threadIdx.x & 31, col = threadIdx.x >> 5;
-  const int id = a.x0 + blockIdx.x * kFFSites + lane;  // output index
+  const int id = a.x0 + block * kFFSites + lane;  // output index
   const bool act = id < a.V;
   const int e = act ? id : a.V - 1;  // idle lanes repeat the last site
   __shared__ FFShare hs;
@@ -483,7 +485,7 @@ __global__ void __launch_bounds__(kFFThreads, kFFMinBlocks) k_wilson_ff(const DA
   double n2 = 0.0;
   ff_store<0, EO, AOS, SUMS>(a, x, e, col, up, act, n2);
   ff_store<1, EO, AOS, SUMS>(a, x, e, col, lo, act, n2);
-  if (SUMS) block_partial_cg(n2, a);
+  if (SUMS) block_partial(n2, a.partials);
 }
 
 // The same for small lattices: four groups of three warps per 32 sites, one
@@ -501,10 +503,12 @@ constexpr size_t kFF4Shared = kFFGroups * (sizeof(FFShare) + sizeof(double2) * 8
 template <bool DAG, bool EO, bool AOS, bool SUMS>
 __global__ void __launch_bounds__(kFFGroups * kFFThreads, 2) k_wilson_ff4(const DArgs a)
 {
+  const int block = SUMS ? (int)blockIdx.x : work_block(a.red);
+  if (block < 0) return;
   extern __shared__ __align__(16) char ff4_shared[];
   const int grp = threadIdx.x / kFFThreads, t = threadIdx.x - grp * kFFThreads;
   const int lane = t & 31, col = t >> 5;
-  const int id = a.x0 + blockIdx.x * kFFSites + lane;  // output index
+  const int id = a.x0 + block * kFFSites + lane;  // output index
   const bool act = id < a.V;
   const int e = act ? id : a.V - 1;  // idle lanes repeat the last site
   FFShare &hs = ((FFShare *)ff4_shared)[grp];
@@ -536,7 +540,7 @@ __global__ void __launch_bounds__(kFFGroups * kFFThreads, 2) k_wilson_ff4(const 
     if (grp == 0) ff_store<0, EO, AOS, SUMS>(a, x, e, col, s, act, n2);
     else ff_store<1, EO, AOS, SUMS>(a, x, e, col, s, act, n2);
   }
-  if (SUMS) block_partial_cg(n2, a);
+  if (SUMS) block_partial(n2, a.partials);
 }
 static_assert(kFF4Shared >= sizeof(CAx2) * 2 * kFFGroups * kFFThreads, "the sums replace the exchange");
 
@@ -593,7 +597,7 @@ template <bool D, bool E, bool A, bool P>
 static void launch_ff(const DArgs &a)
 {
   const int n = a.V - a.x0;
-  const unsigned grid = (unsigned)((n + kFFSites - 1) / kFFSites);
+  const unsigned grid = (unsigned)((n + kFFSites - 1) / kFFSites) + (a.red.n ? 1 : 0);
   if (n > kFFSmall) {
     k_wilson_ff<D, E, A, P><<<grid, kFFThreads, 0, stream()>>>(a);
     return;

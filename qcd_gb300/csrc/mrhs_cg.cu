@@ -30,6 +30,8 @@ namespace qg {
 
 using namespace qgd;
 
+int64_t dslash_df64_blocks(int64_t V);
+
 struct MV {
   __half2 *d;
   float *n;
@@ -401,14 +403,15 @@ static bool slot_residual(qcdgpu_batch B, int k, const BSlot &sl, double *res)
   if (B->eo) {
     qcdgpu_gauge g32 = gauge_at(B->g, QCDGPU_F32);
     const int ar = QCDGPU_ARITH_DF64;
-    // the norms come with the residual and the restart residual
-    const CgFuse f0{B->msdone + 1, res, 0, 2}, f1{B->msdone + 1, res + 2, 0, 2};
+    // |rt|^2 comes in the residual's partials, which the next hop adds up
+    const CgReduce r0{B->part, (int)dslash_df64_blocks(B->Vs), res, 2, 0};
+    const CgReduce r1{B->part, (int)((B->Vs + 127) / 128), res + 2, 2, 0};
     return g32 && dslash_eo(B->u64, sl.xe, nullptr, B->g, sl.mp4, sl.tm, false, 1, 1.0, true, 0, nullptr, ar) &&
-           dslash_eo(B->rt, B->u64, sl.xe, B->g, sl.mp4, sl.tm, false, 0, -0.25, false, 3, B->part, ar, &f0, sl.ce) &&
+           dslash_eo(B->rt, B->u64, sl.xe, B->g, sl.mp4, sl.tm, false, 0, -0.25, false, 3, B->part, ar, nullptr, sl.ce) &&
            convert_field(B->r32, B->rt) &&
-           dslash_eo(B->u32, B->r32, nullptr, g32, sl.mp4, sl.tm, true, 1, 1.0, true, 0, nullptr) &&
-           dslash_eo(B->s32, B->u32, B->r32, g32, sl.mp4, sl.tm, true, 0, -0.25, false, 2, B->part, QCDGPU_ARITH_F64,
-                     &f1) &&
+           dslash_eo(B->u32, B->r32, nullptr, g32, sl.mp4, sl.tm, true, 1, 1.0, true, 0, nullptr, QCDGPU_ARITH_F64,
+                     &r0) &&
+           dslash_eo(B->s32, B->u32, B->r32, g32, sl.mp4, sl.tm, true, 0, -0.25, false, 2, B->part) && cg_total(r1) &&
            mfield_set(B->rs, k, B->s32);
   }
   return slot_bd(B, sl) && dslash(B->rt, sl.x, B->g, sl.mp4, sl.tm, QCDGPU_OP_D, QCDGPU_ARITH_DF64) &&

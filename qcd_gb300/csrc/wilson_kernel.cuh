@@ -193,14 +193,25 @@ __device__ __forceinline__ void hop_pair(const DArgs &a, int x, const int c[4], 
   }
 }
 
+// MODE 0: the operator alone; 1: with the block sums of |out|^2 (a.partials);
+// 2: with an earlier launch's partials added up in a block of its own (a.red).
+// Compiled apart: the code of an unused reduction costs a plain FP16 apply up
+// to 3 %. The FP32 kernel keeps its sums behind a test in mode 0 all the same:
+// compiled without them it runs 8 % slower (45 x 31 x 29 x 33: 104.5 against
+// 113 us), a matter of the compiler's schedule.
+//
 // FP32 / FP16 storage: registers capped for seven blocks per SM (72; 80
-// uncapped), measured at 24^3x48: FP16 48.9 -> 47.1 us, FP32 57.3 -> 55.3 us
-// per apply (a cap of 64 spills and loses). The even/odd kernel below keeps
-// the uncapped form, which solves 0.7 % faster.
-template <bool DAG, int SP, int GP, int RECON, typename R>
-__global__ void __launch_bounds__(128, SP != QCDGPU_F64 ? 7 : 1) k_wilson(const DArgs a)
+// uncapped; FP16 alone eight, 64). Measured at 24^3 x 48, uncapped against seven
+// blocks: FP16 48.9 -> 47.1 us, FP32 57.3 -> 55.3 us per apply; at 32^3 x 64,
+// seven against eight: FP16 133.3 -> 131.9 us, FP32 loses. The even/odd kernel
+// below keeps the uncapped form, which solves 0.7 % faster.
+template <bool DAG, int SP, int RECON, typename R, int MODE>
+__global__ void __launch_bounds__(128, SP == QCDGPU_F64 ? 1 : SP == QCDGPU_F16 && MODE == 0 ? 8 : 7) k_wilson(const DArgs a)
 {
-  int x = a.x0 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  constexpr bool SUMS = MODE == 1 || (MODE == 0 && SP == QCDGPU_F32);
+  const int block = MODE == 2 ? work_block(a.red) : (int)blockIdx.x;
+  if (block < 0) return;
+  int x = a.x0 + (int)(block * blockDim.x + threadIdx.x);
   double n2 = 0.0;
   if (x < a.V) {
     int c[4];
@@ -209,10 +220,10 @@ __global__ void __launch_bounds__(128, SP != QCDGPU_F64 ? 7 : 1) k_wilson(const 
     const R zero = Scalar<R>::get(0.0, 0.0f, 0.0f);
 #pragma unroll
     for (int k = 0; k < 12; k++) acc[k] = C<R>{zero, zero};
-    hop_pair<0, DAG, SP, GP, RECON, R>(a, x, c, acc);
-    hop_pair<1, DAG, SP, GP, RECON, R>(a, x, c, acc);
-    hop_pair<2, DAG, SP, GP, RECON, R>(a, x, c, acc);
-    hop_pair<3, DAG, SP, GP, RECON, R>(a, x, c, acc);
+    hop_pair<0, DAG, SP, SP, RECON, R>(a, x, c, acc);
+    hop_pair<1, DAG, SP, SP, RECON, R>(a, x, c, acc);
+    hop_pair<2, DAG, SP, SP, RECON, R>(a, x, c, acc);
+    hop_pair<3, DAG, SP, SP, RECON, R>(a, x, c, acc);
     C<R> s[12];
     Spinor<SP, R>::load(a.in, a.in_norm, a.stride, x, s);
     const R mp4 = Scalar<R>::get(a.mp4, a.mp4_h, a.mp4_l), tm = Scalar<R>::get(a.tm, a.tm_h, a.tm_l);
@@ -227,7 +238,7 @@ __global__ void __launch_bounds__(128, SP != QCDGPU_F64 ? 7 : 1) k_wilson(const 
       acc[k] = d;
     }
     Spinor<SP, R>::store(a.out, a.out_norm, a.stride, x, acc);
-    if (a.partials) {
+    if (SUMS && a.partials) {
       // per-site sum in the working precision (FP64 arithmetic is scarce on
       // this part); the block sum is double
       R s2 = acc[0].re * acc[0].re + acc[0].im * acc[0].im;
@@ -236,17 +247,20 @@ __global__ void __launch_bounds__(128, SP != QCDGPU_F64 ? 7 : 1) k_wilson(const 
       n2 = (double)s2;
     }
   }
-  if (a.partials) block_partial_cg(n2, a);
+  if (SUMS && a.partials) block_partial(n2, a.partials);
 }
 
 // Even/odd kernel: thread e handles the site of parity a.eo_par whose full
 // index is 2e or 2e + 1 (the t extent is even, so the two sites 2e, 2e + 1
 // of a t-row have opposite parities); neighbours are read from the half
 // field of the other parity at (full index) >> 1.
-template <bool DAG, int SP, int GP, int RECON, typename R>
+template <bool DAG, int SP, int RECON, typename R, int MODE>
 __global__ void __launch_bounds__(128) k_wilson_eo(const DArgs a)
 {
-  const int e = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  constexpr bool SUMS = MODE == 1 || (MODE == 0 && SP == QCDGPU_F32);
+  const int block = MODE == 2 ? work_block(a.red) : (int)blockIdx.x;
+  if (block < 0) return;
+  const int e = (int)(block * blockDim.x + threadIdx.x);
   double n2 = 0.0;
   if (e < a.V) {
     int c[4];
@@ -258,10 +272,10 @@ __global__ void __launch_bounds__(128) k_wilson_eo(const DArgs a)
     const R zero = Scalar<R>::get(0.0, 0.0f, 0.0f);
 #pragma unroll
     for (int k = 0; k < 12; k++) acc[k] = C<R>{zero, zero};
-    hop_pair<0, DAG, SP, GP, RECON, R, true>(a, x, c, acc);
-    hop_pair<1, DAG, SP, GP, RECON, R, true>(a, x, c, acc);
-    hop_pair<2, DAG, SP, GP, RECON, R, true>(a, x, c, acc);
-    hop_pair<3, DAG, SP, GP, RECON, R, true>(a, x, c, acc);
+    hop_pair<0, DAG, SP, SP, RECON, R, true>(a, x, c, acc);
+    hop_pair<1, DAG, SP, SP, RECON, R, true>(a, x, c, acc);
+    hop_pair<2, DAG, SP, SP, RECON, R, true>(a, x, c, acc);
+    hop_pair<3, DAG, SP, SP, RECON, R, true>(a, x, c, acc);
     const R ch = Scalar<R>::get(a.ch, a.ch_h, a.ch_l);
     if (a.ainv) {  // ch A^{-1}: the scale folded into the coefficients
       const R ar = ch * Scalar<R>::get(a.ai_r, a.ai_r_h, a.ai_r_l), ai = ch * Scalar<R>::get(a.ai_i, a.ai_i_h, a.ai_i_l);
@@ -294,14 +308,14 @@ __global__ void __launch_bounds__(128) k_wilson_eo(const DArgs a)
       }
     }
     Spinor<SP, R>::store(a.out, a.out_norm, a.stride, e, acc);
-    if (a.partials) {
+    if (SUMS && a.partials) {
       R s2 = acc[0].re * acc[0].re + acc[0].im * acc[0].im;
 #pragma unroll
       for (int k = 1; k < 12; k++) s2 = s2 + acc[k].re * acc[k].re + acc[k].im * acc[k].im;
       n2 = (double)s2;
     }
   }
-  if (a.partials) block_partial_cg(n2, a);
+  if (SUMS && a.partials) block_partial(n2, a.partials);
 }
 
 }  // namespace qg
