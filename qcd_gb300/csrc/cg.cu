@@ -10,9 +10,10 @@
 //                          p^+ A^+ A p per block)
 //   2. Ap = A^+ t         (operator kernel; one block of its first launch adds
 //                          those sums up and forms alpha = rr / pAp)
-//   3. update kernel:     x' += alpha p, r -= alpha Ap, per-block |r|^2; its
-//                          last block forms rr', beta = rr'/rr, history[i]
-//   4. p = r + beta p     (reads beta from device memory)
+//   3. update kernel:     r -= alpha Ap, per-block |r|^2; its last block forms
+//                          rr', beta = rr'/rr, history[i]
+//   4. p = r + beta p     (reads beta from device memory), and every second
+//                          time x' += alpha p for the last two directions
 // The host enqueues a chunk of iterations, then reads the residual history
 // once and decides. Reliable updates (Sleijpen & van der Vorst, Computing 56
 // (1996) 141; Clark et al., Comput. Phys. Commun. 181 (2010) 1517): when the
@@ -42,95 +43,120 @@ int64_t dslash_df64_blocks(int64_t V);
 
 constexpr int kChunk = 16;
 
-// The two fused reductions run kCgSpt sites per thread in blocks of
+// The update with its reduction runs kCgSpt sites per thread in blocks of
 // kCgThreads: fewer blocks, so the last block sums fewer partials.
 constexpr int kCgThreads = 256, kCgSpt = 2, kCgSites = kCgThreads * kCgSpt;
 
 template <int P, typename R>
-__global__ void __launch_bounds__(kCgThreads) k_cg_update(void *xs, float *xsn, const void *ps, const float *psn,
-                                                          void *rs, float *rsn, const void *aps, const float *apsn,
+__global__ void __launch_bounds__(kCgThreads) k_cg_update(void *rs, float *rsn, const void *aps, const float *apsn,
                                                           int64_t stride, int V, double *s, double *partials,
                                                           unsigned *done, int hist)
 {
   double n2 = 0.0;
 #pragma unroll
   for (int i = 0; i < kCgSpt; i++) {
-  const int x = (int)(blockIdx.x * kCgSites + i * kCgThreads + threadIdx.x);
-  if (x < V) {
-    // FP16 iterations keep the solution increment in FP32: rounding every
-    // increment to 11 bits would cost iterations
-    constexpr int PX = P == QCDGPU_F16 ? QCDGPU_F32 : P;
-    const R alpha = (R)s[S_ALPHA];
-    C<R> vx[12], vp[12];
-    Spinor<PX, R>::load(xs, xsn, stride, x, vx);
-    Spinor<P, R>::load(ps, psn, stride, x, vp);
+    const int x = (int)(blockIdx.x * kCgSites + i * kCgThreads + threadIdx.x);
+    if (x < V) {
+      const R alpha = (R)s[S_ALPHA];
+      C<R> vr[12], va[12];
+      Spinor<P, R>::load(rs, rsn, stride, x, vr);
+      Spinor<P, R>::load(aps, apsn, stride, x, va);
+      R s2 = (R)0;  // per-site sum in the working precision, block sum in double
 #pragma unroll
-    for (int k = 0; k < 12; k++) {
-      vx[k].re = qfma(alpha, vp[k].re, vx[k].re);
-      vx[k].im = qfma(alpha, vp[k].im, vx[k].im);
+      for (int k = 0; k < 12; k++) {
+        vr[k].re = qfma(-alpha, va[k].re, vr[k].re);
+        vr[k].im = qfma(-alpha, va[k].im, vr[k].im);
+        s2 = s2 + vr[k].re * vr[k].re + vr[k].im * vr[k].im;
+      }
+      n2 += (double)s2;
+      Spinor<P, R>::store(rs, rsn, stride, x, vr);
     }
-    Spinor<PX, R>::store(xs, xsn, stride, x, vx);
-    Spinor<P, R>::load(rs, rsn, stride, x, vx);
-    Spinor<P, R>::load(aps, apsn, stride, x, vp);
-    R s2 = (R)0;  // per-site sum in the working precision, block sum in double
-#pragma unroll
-    for (int k = 0; k < 12; k++) {
-      vx[k].re = qfma(-alpha, vp[k].re, vx[k].re);
-      vx[k].im = qfma(-alpha, vp[k].im, vx[k].im);
-      s2 = s2 + vx[k].re * vx[k].re + vx[k].im * vx[k].im;
-    }
-    n2 += (double)s2;
-    Spinor<P, R>::store(rs, rsn, stride, x, vx);
-  }
   }
   block_partial(n2, partials);
   cg_last_block(partials, done, s, 1, hist);
 }
 
-// y += xs, xs = 0: the FP32 increment into the FP64 solution
-__global__ void __launch_bounds__(128) k_cg_flush(double2 *y, int64_t ystride, float4 *xs, int64_t stride, int V)
+// FP16 iterations keep the solution increment in FP32: rounding every
+// increment to 11 bits would cost iterations
+template <int P>
+constexpr int kIncPrec = P == QCDGPU_F16 ? QCDGPU_F32 : P;
+
+// v += a p at site x
+template <int P, typename R>
+__device__ __forceinline__ void add_scaled(C<R> v[12], R a, const C<R> p[12])
 {
-  const int x = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (x >= V) return;
 #pragma unroll
-  for (int j = 0; j < 6; j++) {
-    float4 &v = xs[j * stride + x];
-    double2 &a = y[(2 * j) * ystride + x], &b = y[(2 * j + 1) * ystride + x];
-    const float4 w = v;
-    a = make_double2(a.x + (double)w.x, a.y + (double)w.y);
-    b = make_double2(b.x + (double)w.z, b.y + (double)w.w);
-    v = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int k = 0; k < 12; k++) {
+    v[k].re = qfma(a, p[k].re, v[k].re);
+    v[k].im = qfma(a, p[k].im, v[k].im);
   }
 }
 
-template <int P, typename R>
-__global__ void __launch_bounds__(128) k_cg_p(void *ps, float *psn, const void *rs, const float *rsn, int64_t stride,
-                                              int V, const double *s)
+// The directions alternate between two fields: pn (the one before last) <- rs
+// + beta po (the last). XUPD (odd iterations): also xs += alpha p for both, so
+// the increment is read and written every second iteration only, with the
+// directions the update reads anyway (it took two fifths of an iteration's
+// vector traffic: 24^3 x 48, FP16, 34 -> 28 us per iteration for the vector
+// kernels). The directions' alphas are S_A1 for pn, S_A0 for po; what is
+// pending at a reliable update is added by k_cg_flush.
+template <int P, typename R, bool XUPD>
+__global__ void __launch_bounds__(128) k_cg_p(void *pn, float *pnn, const void *po, const float *pon, const void *rs,
+                                              const float *rsn, void *xs, float *xsn, int64_t stride, int V,
+                                              const double *s)
 {
   int x = (int)(blockIdx.x * blockDim.x + threadIdx.x);
   if (x >= V) return;
   const R beta = (R)s[S_BETA];
-  C<R> vp[12], vr[12];
-  Spinor<P, R>::load(ps, psn, stride, x, vp);
-  Spinor<P, R>::load(rs, rsn, stride, x, vr);
-#pragma unroll
-  for (int k = 0; k < 12; k++) {
-    vp[k].re = qfma(beta, vp[k].re, vr[k].re);
-    vp[k].im = qfma(beta, vp[k].im, vr[k].im);
+  C<R> vp[12], v[12];
+  if (XUPD) {
+    Spinor<kIncPrec<P>, R>::load(xs, xsn, stride, x, v);
+    Spinor<P, R>::load(pn, pnn, stride, x, vp);
+    add_scaled<P, R>(v, (R)s[S_A1], vp);
   }
-  Spinor<P, R>::store(ps, psn, stride, x, vp);
+  Spinor<P, R>::load(po, pon, stride, x, vp);
+  if (XUPD) {
+    add_scaled<P, R>(v, (R)s[S_A0], vp);
+    Spinor<kIncPrec<P>, R>::store(xs, xsn, stride, x, v);
+  }
+  Spinor<P, R>::load(rs, rsn, stride, x, v);
+  add_scaled<P, R>(v, beta, vp);
+  Spinor<P, R>::store(pn, pnn, stride, x, v);
 }
 
-// per-block Re <a, b> (used for p^+ A p when the storage rounds D p: with
-// FP16 fields A p = D^+ round(D p), and |D p|^2 would not match it)
+// y += xs and the pending directions, xs = 0: the increment into the FP64
+// solution. After an even number of iterations the odd one's direction p1 is
+// pending, after an odd number (two) p1 and then p0.
+template <int P, typename R>
+__global__ void __launch_bounds__(128) k_cg_flush(double2 *y, int64_t ystride, void *xs, float *xsn, const void *p0,
+                                                  const float *p0n, const void *p1, const float *p1n, int64_t stride,
+                                                  int V, const double *s, int two)
+{
+  const int x = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  if (x >= V) return;
+  C<R> v[12], vp[12];
+  Spinor<kIncPrec<P>, R>::load(xs, xsn, stride, x, v);
+  Spinor<P, R>::load(p1, p1n, stride, x, vp);
+  add_scaled<P, R>(v, (R)s[S_A1], vp);
+  if (two) {
+    Spinor<P, R>::load(p0, p0n, stride, x, vp);
+    add_scaled<P, R>(v, (R)s[S_A0], vp);
+  }
+#pragma unroll
+  for (int k = 0; k < 12; k++) {
+    double2 &a = y[k * ystride + x];
+    a = make_double2(a.x + (double)v[k].re, a.y + (double)v[k].im);
+    v[k] = C<R>{(R)0, (R)0};
+  }
+  Spinor<kIncPrec<P>, R>::store(xs, xsn, stride, x, v);
+}
 
-#define QG_PREC_DISPATCH(prec, KERNEL, ...)                                          \
-  do {                                                                               \
-    if ((prec) == QCDGPU_F64) KERNEL<QCDGPU_F64, double><<<nb, 128, 0, st>>>(__VA_ARGS__); \
-    else if ((prec) == QCDGPU_F32) KERNEL<QCDGPU_F32, float><<<nb, 128, 0, st>>>(__VA_ARGS__); \
-    else KERNEL<QCDGPU_F16, float><<<nb, 128, 0, st>>>(__VA_ARGS__);                 \
+// KERNEL<precision, arithmetic, ...> by storage precision
+#define QG_PREC_DISPATCH(prec, LAUNCH)                       \
+  do {                                                       \
+    if ((prec) == QCDGPU_F64) { LAUNCH(QCDGPU_F64, double) } \
+    else if ((prec) == QCDGPU_F32) { LAUNCH(QCDGPU_F32, float) } \
+    else { LAUNCH(QCDGPU_F16, float) }                       \
   } while (0)
-
 
 __global__ void __launch_bounds__(512) k_cg_total(CgReduce r) { cg_sum(r); }
 
@@ -235,11 +261,11 @@ static int cgnr_core(qcdgpu_field y, qcdgpu_field c, double cn, const CgOps &ops
 {
   Held w;
   const int prec = p->inner_prec;
-  qcdgpu_field rt = w.get(ops.L, QCDGPU_F64), r = w.get(ops.L, QCDGPU_F64), up = w.get(ops.L, QCDGPU_F64);
-  qcdgpu_field rs = w.get(ops.L, prec), ps = w.get(ops.L, prec);
+  qcdgpu_field rt = w.get(ops.L, QCDGPU_F64), r = w.get(ops.L, QCDGPU_F64);
+  qcdgpu_field rs = w.get(ops.L, prec), ps[2] = {w.get(ops.L, prec), w.get(ops.L, prec)};
   qcdgpu_field xs = w.get(ops.L, prec == QCDGPU_F16 ? QCDGPU_F32 : prec);
   qcdgpu_field t = w.get(ops.L, prec), aps = w.get(ops.L, prec);
-  if (!rt || !r || !up || !rs || !xs || !ps || !t || !aps) return 3;
+  if (!rt || !r || !rs || !xs || !ps[0] || !ps[1] || !t || !aps) return 3;
   const int V = (int)rt->V;
   const unsigned nb = (unsigned)((V + 127) / 128);            // operator launches: 128 sites per block
   const unsigned nbr = (unsigned)((V + kCgSites - 1) / kCgSites);  // the fused reductions
@@ -285,7 +311,7 @@ static int cgnr_core(qcdgpu_field y, qcdgpu_field c, double cn, const CgOps &ops
   if (!blas_copy(rt, c)) return 3;
   double rr;
   if (!restart_residual(&rr)) return 3;
-  if (!blas_copy(ps, rs) || !blas_zero(xs)) return 3;
+  if (!blas_copy(ps[0], rs) || !blas_zero(ps[1]) || !blas_zero(xs)) return 3;
   double maxr = sqrt(rr), hint = p->tol * maxr;
   bool first = true;
   const double delta = p->delta > 0 ? p->delta : 0.1;
@@ -299,21 +325,28 @@ static int cgnr_core(qcdgpu_field y, qcdgpu_field c, double cn, const CgOps &ops
       // p = r + beta p opens each iteration (not the first), so a reliable
       // update between chunks enters the next direction through beta
       if (!first) {
-        QG_PREC_DISPATCH(prec, k_cg_p, ps->data, ps->norm, rs->data, rs->norm, ps->stride, V, s);
+        const qcdgpu_field pn = ps[j & 1], po = ps[(j & 1) ^ 1];
+#define QG_CG_P(P, R)                                                                                             \
+  if (j & 1)                                                                                                      \
+    k_cg_p<P, R, true><<<nb, 128, 0, st>>>(pn->data, pn->norm, po->data, po->norm, rs->data, rs->norm, xs->data,  \
+                                           xs->norm, pn->stride, V, s);                                           \
+  else                                                                                                            \
+    k_cg_p<P, R, false><<<nb, 128, 0, st>>>(pn->data, pn->norm, po->data, po->norm, rs->data, rs->norm, xs->data, \
+                                            xs->norm, pn->stride, V, s);
+        QG_PREC_DISPATCH(prec, QG_CG_P);
+#undef QG_CG_P
         if (!QG_LAUNCHED("cg_p")) return false;
       }
       first = false;
       // p^+ A^+ A p = |A p|^2, summed in the epilogue of the first operator and
       // added up beside the second
       const CgReduce pap{part, (int)ops.parts, s, 0, j};
-      if (!ops.op(t, ps, part) || !ops.opdag(aps, t, &pap)) return false;
-#define QG_CG_UPD(P, R)                                                                                           \
-  k_cg_update<P, R><<<nbr, kCgThreads, 0, st>>>(xs->data, xs->norm, ps->data, ps->norm, rs->data, rs->norm, aps->data, \
-                                                aps->norm, xs->stride, V, s, part, done, j)
-      // x += alpha p, r -= alpha A p, with |r|^2 and beta
-      if (prec == QCDGPU_F64) QG_CG_UPD(QCDGPU_F64, double);
-      else if (prec == QCDGPU_F32) QG_CG_UPD(QCDGPU_F32, float);
-      else QG_CG_UPD(QCDGPU_F16, float);
+      if (!ops.op(t, ps[j & 1], part) || !ops.opdag(aps, t, &pap)) return false;
+#define QG_CG_UPD(P, R)                                                                                          \
+  k_cg_update<P, R><<<nbr, kCgThreads, 0, st>>>(rs->data, rs->norm, aps->data, aps->norm, rs->stride, V, s, part, \
+                                                done, j);
+      // r -= alpha A p, with |r|^2 and beta
+      QG_PREC_DISPATCH(prec, QG_CG_UPD);
 #undef QG_CG_UPD
       if (!QG_LAUNCHED("cg_update")) return false;
     }
@@ -347,12 +380,12 @@ static int cgnr_core(qcdgpu_field y, qcdgpu_field c, double cn, const CgOps &ops
     }
     bool last = p->iters >= p->maxiter;
     if (update || hinted || last) {
-      if (prec == QCDGPU_F64) {
-        if (!blas_axpby(y, 1.0, 0.0, xs, 1.0, 0.0, y) || !blas_zero(xs)) return 3;
-      } else {
-        k_cg_flush<<<nb, 128, 0, st>>>((double2 *)y->data, y->stride, (float4 *)xs->data, xs->stride, V);
-        if (!QG_LAUNCHED("cg_flush")) return 3;
-      }
+#define QG_CG_FLUSH(P, R)                                                                                         \
+  k_cg_flush<P, R><<<nb, 128, 0, st>>>((double2 *)y->data, y->stride, xs->data, xs->norm, ps[0]->data, ps[0]->norm, \
+                                       ps[1]->data, ps[1]->norm, xs->stride, V, s, chunk & 1);
+      QG_PREC_DISPATCH(prec, QG_CG_FLUSH);
+#undef QG_CG_FLUSH
+      if (!QG_LAUNCHED("cg_flush") || !QG_CUDA(cudaMemsetAsync(s + S_A0, 0, 2 * sizeof(double), st))) return 3;
       p->reliable_updates++;
       since_update = 0;
       if (hinted) hint = rn * 0.3;

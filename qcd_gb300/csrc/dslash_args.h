@@ -69,8 +69,8 @@ __device__ __forceinline__ void block_partial(double v, double *partials)
   }
 }
 
-// scalar slots
-enum { S_RR = 0, S_PAP = 1, S_RRNEW = 2, S_ALPHA = 3, S_BETA = 4, S_RES = 5, S_HIST = 8 };
+// scalar slots (S_A0, S_A1: alpha of the last even and odd iteration of a chunk)
+enum { S_RR = 0, S_PAP = 1, S_RRNEW = 2, S_ALPHA = 3, S_BETA = 4, S_RES = 5, S_A0 = 6, S_A1 = 7, S_HIST = 8 };
 
 // the CG scalars from a reduced total: mode 0 t = p^+ A p -> alpha;
 // mode 1 t = |r|^2 -> beta and the residual history; mode 2 the total itself;
@@ -80,7 +80,7 @@ __device__ __forceinline__ void cg_scalars_from(double t, double *s, int mode, i
 {
   if (mode == 0) {
     s[S_PAP] = t;
-    s[S_ALPHA] = t > 0.0 ? s[S_RR] / t : nan("");  // p^+ A p <= 0: breakdown
+    s[S_ALPHA] = s[S_A0 + (hist & 1)] = t > 0.0 ? s[S_RR] / t : nan("");  // p^+ A p <= 0: breakdown
   } else if (mode == 1) {
     s[S_RRNEW] = t;
     s[S_BETA] = t / s[S_RR];

@@ -1244,6 +1244,7 @@ static MrhsTune mrhs_tune(const MArgs &a, bool dag)
   auto it = g_mrhs_tuned.find(key);
   if (it != g_mrhs_tuned.end()) return it->second;
   const MrhsTune fallback{MRHS_SIMT, 64};
+  if (a.z == a.out) return fallback;  // a repeated launch would read its own result
   cudaStream_t s = stream();
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return fallback;
@@ -1343,7 +1344,7 @@ bool dslash_mrhs_eo(qcdgpu_mfield out, qcdgpu_mfield in, qcdgpu_mfield z, qcdgpu
                     const float *mp4s, const float *tms, int par, double ch, bool ainv, int zmode, double *partials,
                     unsigned *nblocks)
 {
-  if (!out || !in || !g || out == in || out->N != in->N || out->V != in->V || (zmode && (!z || z == out)) ||
+  if (!out || !in || !g || out == in || out->N != in->N || out->V != in->V || (zmode && !z) ||
       (z && (z->N != in->N || z->V != in->V)) || g->prec != QCDGPU_F64 || !eo_lattice(g->L) ||
       in->L[0] * 2 != g->L[0] || in->L[1] != g->L[1] || in->L[2] != g->L[2] || in->L[3] != g->L[3] ||
       memcmp(out->L, in->L, sizeof(in->L)) != 0 || nact < 0 || nact > in->N || !mp4s || !tms) {

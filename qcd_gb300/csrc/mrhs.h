@@ -82,7 +82,8 @@ bool dslash_mrhs(qcdgpu_mfield out, qcdgpu_mfield in, qcdgpu_gauge g, double mp4
                  const float *mp4s, const float *tms, double *partials = nullptr, unsigned *nblocks = nullptr);
 unsigned mrhs_max_blocks(int64_t V, int N);
 // even/odd kernel on half-lattice fields (SIMT): out (parity par) =
-// ch * [A^{-1}] H in + {0 | z | A z} with the slots' diagonals A
+// ch * [A^{-1}] H in + {0 | A z} with the slots' diagonals A. z may be out: each
+// thread reads z at the site and slot that it stores
 bool dslash_mrhs_eo(qcdgpu_mfield out, qcdgpu_mfield in, qcdgpu_mfield z, qcdgpu_gauge g, bool dag, int nact,
                     const float *mp4s, const float *tms, int par, double ch, bool ainv, int zmode, double *partials,
                     unsigned *nblocks);

@@ -74,22 +74,36 @@ struct MX {
   __device__ __forceinline__ float4 &at(int j, int x, int r) const { return d[(r * 6 + j) * S + x]; }
 };
 
-// xs += alpha p ; rs -= alpha Ap ; partials <- |rs|^2 per slot
+// slot r of xs += a p at site x
+__device__ __forceinline__ void mx_add(MX xs, int x, int r, float a, const float2 p[12])
+{
+#pragma unroll
+  for (int j = 0; j < 6; j++) {
+    float4 &v = xs.at(j, x, r);
+    const float4 w = v;
+    v = make_float4(__fmaf_rn(a, p[2 * j].x, w.x), __fmaf_rn(a, p[2 * j].y, w.y), __fmaf_rn(a, p[2 * j + 1].x, w.z),
+                    __fmaf_rn(a, p[2 * j + 1].y, w.w));
+  }
+}
+
+// scalar layout, per slot r of N: rr, pAp, alpha, beta, alpha of the chunk's
+// last even and odd iteration, then history[j]
+enum { M_RR = 0, M_PAP = 1, M_ALPHA = 2, M_BETA = 3, M_A0 = 4, M_A1 = 5, M_HIST = 6 };
+constexpr int kMChunk = 16;
+
+// rs -= alpha Ap (XUPD: and xs += alpha p) ; partials <- |rs|^2 per slot
+template <bool XUPD>
 __global__ void __launch_bounds__(kMSites) k_mupdate(MX xs, MV ps, MV rs, MV aps, const double *alpha,
                                                      double *partials, int N)
 {
   const int r = blockIdx.y, x = blockIdx.x * kMSites + threadIdx.x;
   double n2 = 0.0;
-  if (x < xs.V) {
+  if (x < rs.V) {
     const float al = (float)alpha[r];
     float2 a[12], b[12];
-    mv_load(ps, x, r, b);
-#pragma unroll
-    for (int j = 0; j < 6; j++) {
-      float4 &v = xs.at(j, x, r);
-      const float4 w = v;
-      v = make_float4(__fmaf_rn(al, b[2 * j].x, w.x), __fmaf_rn(al, b[2 * j].y, w.y),
-                      __fmaf_rn(al, b[2 * j + 1].x, w.z), __fmaf_rn(al, b[2 * j + 1].y, w.w));
+    if (XUPD) {
+      mv_load(ps, x, r, b);
+      mx_add(xs, x, r, al, b);
     }
     mv_load(rs, x, r, a);
     mv_load(aps, x, r, b);
@@ -113,11 +127,53 @@ __global__ void __launch_bounds__(kMSites) k_mupdate(MX xs, MV ps, MV rs, MV aps
   }
 }
 
-// f (FP64 field) += slot r of xs, then slot r of xs <- 0
-__global__ void k_mx_flush(double2 *f, int64_t fstride, MX xs, int r)
+// pn <- rs + beta po. Even/odd batches alternate the directions between two
+// fields (pn holds the one before last, po the last one), so that odd
+// iterations (XUPD) add both of them to xs, as cg.cu's k_cg_p does. They hold
+// the second direction in place of A p, which their operator leaves where D p
+// was. The full operator needs both, and no batch takes more memory for its
+// update: pn and po are the same field there, and k_mupdate adds to xs. The two
+// kernels take 50 us an iteration for 8 slots of 16^3 x 32 (64 before), at the
+// memory's rate.
+template <bool XUPD>
+__global__ void __launch_bounds__(kMSites) k_mp(MV pn, MV po, MV rs, MX xs, const double *s, int N)
+{
+  const int r = blockIdx.y, x = blockIdx.x * kMSites + threadIdx.x;
+  if (x >= rs.V) return;
+  const float be = (float)s[M_BETA * N + r];
+  float2 p[12], q[12];
+  mv_load(po, x, r, p);
+  if (XUPD) {
+    const float a1 = (float)s[M_A1 * N + r], a0 = (float)s[M_A0 * N + r];
+    mv_load(pn, x, r, q);
+#pragma unroll
+    for (int j = 0; j < 6; j++) {
+      float4 &v = xs.at(j, x, r);
+      float4 w = v;
+      w = make_float4(__fmaf_rn(a1, q[2 * j].x, w.x), __fmaf_rn(a1, q[2 * j].y, w.y),
+                      __fmaf_rn(a1, q[2 * j + 1].x, w.z), __fmaf_rn(a1, q[2 * j + 1].y, w.w));
+      v = make_float4(__fmaf_rn(a0, p[2 * j].x, w.x), __fmaf_rn(a0, p[2 * j].y, w.y),
+                      __fmaf_rn(a0, p[2 * j + 1].x, w.z), __fmaf_rn(a0, p[2 * j + 1].y, w.w));
+    }
+  }
+  mv_load(rs, x, r, q);
+#pragma unroll
+  for (int k = 0; k < 12; k++) p[k] = make_float2(__fmaf_rn(be, p[k].x, q[k].x), __fmaf_rn(be, p[k].y, q[k].y));
+  mv_store(pn, x, r, p);
+}
+
+// f (FP64 field) += slot r of xs and, PEND, its pending direction p1 (a chunk
+// ends with an odd iteration), then slot r of xs <- 0
+template <bool PEND>
+__global__ void k_mx_flush(double2 *f, int64_t fstride, MX xs, MV p1, const double *s, int N, int r)
 {
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= xs.V) return;
+  if (PEND) {
+    float2 p[12];
+    mv_load(p1, x, r, p);
+    mx_add(xs, x, r, (float)s[M_A1 * N + r], p);
+  }
 #pragma unroll
   for (int j = 0; j < 6; j++) {
     float4 &v = xs.at(j, x, r);
@@ -143,20 +199,6 @@ __global__ void k_mx_copy(MX xs, int from, int to, int zero)
         zero ? make_float4(0.f, 0.f, 0.f, 0.f) : xs.at(j, x, from);
 }
 
-// ps = rs + beta ps
-__global__ void __launch_bounds__(kMSites) k_mp(MV ps, MV rs, const double *beta)
-{
-  const int r = blockIdx.y, x = blockIdx.x * kMSites + threadIdx.x;
-  if (x >= ps.V) return;
-  const float be = (float)beta[r];
-  float2 p[12], q[12];
-  mv_load(ps, x, r, p);
-  mv_load(rs, x, r, q);
-#pragma unroll
-  for (int k = 0; k < 12; k++) p[k] = make_float2(__fmaf_rn(be, p[k].x, q[k].x), __fmaf_rn(be, p[k].y, q[k].y));
-  mv_store(ps, x, r, p);
-}
-
 // slot `to` <- slot `from` (zero == 1: slot `to` <- 0)
 __global__ void k_mcopy(MV m, int from, int to, int zero)
 {
@@ -168,10 +210,6 @@ __global__ void k_mcopy(MV m, int from, int to, int zero)
     p[mword(m.S, j, x, to)] = zero ? make_uint4(0u, 0u, 0u, 0u) : p[mword(m.S, j, x, from)];
   m.n[mnorm_at(m.S, x, to)] = zero ? 0.f : m.n[mnorm_at(m.S, x, from)];
 }
-
-// scalar layout, per slot r of N: rr, pAp, alpha, beta, then history[j]
-enum { M_RR = 0, M_PAP = 1, M_ALPHA = 2, M_BETA = 3, M_HIST = 4 };
-constexpr int kMChunk = 16;
 
 // Per-slot sums of the nb block partials, in two levels: block g of kMSGroups sums a contiguous
 // range of the nb block partials for every slot (consecutive threads read
@@ -224,7 +262,7 @@ __global__ void __launch_bounds__(256) k_mscalars2(const double *partials, int n
     for (int kk = 0; kk < K; kk++) t += sh[kk * N + rr];
     if (mode == 0) {
       s[M_PAP * N + rr] = t;
-      s[M_ALPHA * N + rr] = t > 0.0 ? s[M_RR * N + rr] / t : nan("");
+      s[M_ALPHA * N + rr] = s[(M_A0 + (hist & 1)) * N + rr] = t > 0.0 ? s[M_RR * N + rr] / t : nan("");
     } else {
       s[M_BETA * N + rr] = t / s[M_RR * N + rr];
       s[M_RR * N + rr] = t;
@@ -268,7 +306,9 @@ struct qcdgpu_batch_s {
   bool eo;
   int Ls[4];
   int64_t Vs;
-  qcdgpu_mfield rs, ps, t, aps, u;  // u: odd intermediate (even/odd only)
+  // the directions of even and odd iterations (full operator: one field);
+  // even/odd: A p is left in t (aps == t), u is the odd intermediate
+  qcdgpu_mfield rs, ps[2], t, aps, u;
   float4 *xs;                  // FP32 solution increments (layout of MX)
   qcdgpu_field rt, r, up, bd;  // FP64 work shared by the slots' reliable updates
   qcdgpu_field u64, r32, u32, s32;  // even/odd: FP64 odd temp; FP32 restart fields
@@ -300,7 +340,9 @@ static void batch_free(qcdgpu_batch b)
 {
   if (!b) return;
   if (b->st) cudaStreamSynchronize(b->st);  // a chunk may still be running
-  for (auto m : {b->rs, b->ps, b->t, b->aps, b->u}) mfield_free(m);
+  if (b->ps[1] != b->ps[0]) mfield_free(b->ps[1]);
+  if (b->aps != b->t) mfield_free(b->aps);
+  for (auto m : {b->rs, b->ps[0], b->t, b->u}) mfield_free(m);
   cudaFree(b->xs);
   for (auto f : {b->rt, b->r, b->up, b->bd, b->u64, b->r32, b->u32, b->s32}) field_free(f);
   for (auto &sl : b->slots)
@@ -342,14 +384,15 @@ static qcdgpu_batch batch_new(qcdgpu_gauge g, int cap, bool eo)
   b->graphs.assign((size_t)cap + 1, nullptr);
   b->graph_launches.assign((size_t)cap + 1, 0);
   b->rs = mfield_new(b->Ls, cap);
-  b->ps = mfield_new(b->Ls, cap);
+  b->ps[0] = mfield_new(b->Ls, cap);
+  b->ps[1] = eo ? mfield_new(b->Ls, cap) : b->ps[0];
   b->t = mfield_new(b->Ls, cap);
-  b->aps = mfield_new(b->Ls, cap);
+  b->aps = eo ? b->t : mfield_new(b->Ls, cap);
   b->rt = field_new(b->Ls, QCDGPU_F64);
   b->r = field_new(b->Ls, QCDGPU_F64);
   b->up = field_new(b->Ls, QCDGPU_F64);
   b->bd = field_new(g->L, QCDGPU_F64);
-  bool ok = b->rs && b->ps && b->t && b->aps && b->rt && b->r && b->up && b->bd;
+  bool ok = b->rs && b->ps[0] && b->ps[1] && b->t && b->aps && b->rt && b->r && b->up && b->bd;
   if (eo) {
     b->u = mfield_new(b->Ls, cap);
     b->u64 = field_new(b->Ls, QCDGPU_F64);
@@ -420,7 +463,7 @@ static bool slot_residual(qcdgpu_batch B, int k, const BSlot &sl, double *res)
          blas_norm2_dev(B->r, res + 2) && mfield_set(B->rs, k, B->r);
 }
 
-// rr and beta of up to 64 slots after their reliable updates, in one launch
+// the scalars of up to 64 slots after their reliable updates, in one launch
 struct SlotRestart {
   int n;
   int slot[64];
@@ -432,6 +475,7 @@ __global__ void k_set_restart(double *s, int cap, SlotRestart r)
   if (i >= r.n) return;
   s[M_RR * cap + r.slot[i]] = r.rr[i];
   s[M_BETA * cap + r.slot[i]] = r.beta[i];
+  s[M_A1 * cap + r.slot[i]] = 0.0;  // the pending direction is in the solution
 }
 
 static bool set_scalar(qcdgpu_batch B, int slot_kind, int k, double v)
@@ -445,7 +489,7 @@ static bool set_scalar(qcdgpu_batch B, int slot_kind, int k, double v)
 static bool copy_slot(qcdgpu_batch B, int from, int to)
 {
   unsigned g = (unsigned)((B->Vs + 127) / 128);
-  for (auto m : {B->rs, B->ps}) {
+  for (auto m : {B->rs, B->ps[1]}) {  // between chunks the direction of odd iterations is the last one
     k_mcopy<<<g, 128, 0, stream()>>>(mv(m), from, to, 0);
     if (!QG_LAUNCHED("mrhs_copy_slot")) return false;
   }
@@ -553,11 +597,12 @@ int batch_add(qcdgpu_batch B, qcdgpu_field x, qcdgpu_field b, double kappa, doub
   k_mx_copy<<<g, 128, 0, stream()>>>(mx(B), 0, k, 1);
   float mp = (float)sl.mp4, tmf = (float)mu;
   // p = r (slot_residual left r in B->s32 for even/odd batches, else in B->r);
-  // a fresh slot starts with beta = 0, so the shared p update leaves p = r
-  if (!QG_LAUNCHED("mrhs_zero_slot") || !mfield_set(B->ps, k, B->eo ? B->s32 : B->r) ||
+  // a fresh slot starts with beta = 0, so the shared p update leaves p = r, and
+  // with no pending direction
+  if (!QG_LAUNCHED("mrhs_zero_slot") || !mfield_set(B->ps[1], k, B->eo ? B->s32 : B->r) ||
       !QG_CUDA(cudaMemcpyAsync(B->mp4s + k, &mp, sizeof(float), cudaMemcpyHostToDevice, stream())) ||
       !QG_CUDA(cudaMemcpyAsync(B->tms + k, &tmf, sizeof(float), cudaMemcpyHostToDevice, stream())) ||
-      !set_scalar(B, M_RR, k, rr) || !set_scalar(B, M_BETA, k, 0.0)) {
+      !set_scalar(B, M_RR, k, rr) || !set_scalar(B, M_BETA, k, 0.0) || !set_scalar(B, M_A1, k, 0.0)) {
     give_back();
     return -2;
   }
@@ -608,17 +653,19 @@ static bool chunk_enqueue(qcdgpu_batch B, int n)
   cudaStream_t st = stream();
   for (int j = 0; j < kMChunk; j++) {
     // p = r + beta p (beta = 0 keeps a fresh slot's p = r)
-    k_mp<<<grid, kMSites, 0, st>>>(mv(B->ps), mv(B->rs), B->s + M_BETA * cap);
+    const qcdgpu_mfield ps = B->ps[j & 1], po = B->ps[(j & 1) ^ 1];
+    if (B->eo && (j & 1)) k_mp<true><<<grid, kMSites, 0, st>>>(mv(ps), mv(po), mv(B->rs), mx(B), B->s, cap);
+    else k_mp<false><<<grid, kMSites, 0, st>>>(mv(ps), mv(po), mv(B->rs), mx(B), B->s, cap);
     if (!QG_LAUNCHED("mrhs_p")) return false;
     // p^+ A^+ A p = |A p|^2, summed per slot in the epilogue of t = A p
     // (A = D, or the Schur complement M = A_ee - H_eo A_oo^{-1} H_oe / 4 as
     // u = A^{-1} H_oe p, t = A p - H_eo u / 4)
     unsigned nbo = 0;
     if (B->eo) {
-      if (!dslash_mrhs_eo(B->u, B->ps, nullptr, B->g, false, n, B->mp4s, B->tms, 1, 1.0, true, 0, nullptr, nullptr) ||
-          !dslash_mrhs_eo(B->t, B->u, B->ps, B->g, false, n, B->mp4s, B->tms, 0, -0.25, false, 2, B->part, &nbo))
+      if (!dslash_mrhs_eo(B->u, ps, nullptr, B->g, false, n, B->mp4s, B->tms, 1, 1.0, true, 0, nullptr, nullptr) ||
+          !dslash_mrhs_eo(B->t, B->u, ps, B->g, false, n, B->mp4s, B->tms, 0, -0.25, false, 2, B->part, &nbo))
         return false;
-    } else if (!dslash_mrhs(B->t, B->ps, B->g, 4.0, 0.0, false, n, B->mp4s, B->tms, B->part, &nbo)) {
+    } else if (!dslash_mrhs(B->t, ps, B->g, 4.0, 0.0, false, n, B->mp4s, B->tms, B->part, &nbo)) {
       return false;
     }
     k_mscalars2<<<kMSGroups, 256, 0, st>>>(B->part, (int)nbo, cap, n, B->s, 0, j, B->l1, B->msdone);
@@ -630,7 +677,9 @@ static bool chunk_enqueue(qcdgpu_batch B, int n)
     } else if (!dslash_mrhs(B->aps, B->t, B->g, 4.0, 0.0, true, n, B->mp4s, B->tms)) {
       return false;
     }
-    k_mupdate<<<grid, kMSites, 0, st>>>(mx(B), mv(B->ps), mv(B->rs), mv(B->aps), B->s + M_ALPHA * cap, B->part, cap);
+    const double *alpha = B->s + M_ALPHA * cap;
+    if (B->eo) k_mupdate<false><<<grid, kMSites, 0, st>>>(mx(B), mv(ps), mv(B->rs), mv(B->aps), alpha, B->part, cap);
+    else k_mupdate<true><<<grid, kMSites, 0, st>>>(mx(B), mv(ps), mv(B->rs), mv(B->aps), alpha, B->part, cap);
     if (!QG_LAUNCHED("mrhs_update")) return false;
     k_mscalars2<<<kMSGroups, 256, 0, st>>>(B->part, (int)grid.x, cap, n, B->s, 1, j, B->l1, B->msdone);
     if (!QG_LAUNCHED("mrhs_scalars")) return false;
@@ -648,11 +697,11 @@ bool batch_launch(qcdgpu_batch B)
   if (!B->tuned) {
     // the operator's tuner times its variants outside stream capture; t and
     // u are scratch (recomputed by every iteration)
-    const bool ok = B->eo ? dslash_mrhs_eo(B->u, B->ps, nullptr, B->g, false, n, B->mp4s, B->tms, 1, 1.0, true, 0,
+    const bool ok = B->eo ? dslash_mrhs_eo(B->u, B->ps[1], nullptr, B->g, false, n, B->mp4s, B->tms, 1, 1.0, true, 0,
                                            nullptr, nullptr) &&
-                                dslash_mrhs_eo(B->t, B->u, B->ps, B->g, false, n, B->mp4s, B->tms, 0, -0.25, false, 2,
+                                dslash_mrhs_eo(B->t, B->u, B->ps[1], B->g, false, n, B->mp4s, B->tms, 0, -0.25, false, 2,
                                                nullptr, nullptr)
-                          : dslash_mrhs(B->t, B->ps, B->g, 4.0, 0.0, false, n, B->mp4s, B->tms);
+                          : dslash_mrhs(B->t, B->ps[1], B->g, 4.0, 0.0, false, n, B->mp4s, B->tms);
     if (!ok) return false;
     B->tuned = true;
   }
@@ -744,7 +793,10 @@ bool batch_finish(qcdgpu_batch B)
     if (!need[k]) continue;
     BSlot &sl = B->slots[(size_t)k];
     qcdgpu_field acc = B->eo ? sl.xe : sl.x;  // the slot's FP64 solution
-    k_mx_flush<<<(unsigned)((V + 127) / 128), 128, 0, st>>>((double2 *)acc->data, acc->stride, mx(B), k);
+    const unsigned g = (unsigned)((V + 127) / 128);
+    double2 *y = (double2 *)acc->data;
+    if (B->eo) k_mx_flush<true><<<g, 128, 0, st>>>(y, acc->stride, mx(B), mv(B->ps[1]), B->s, cap, k);
+    else k_mx_flush<false><<<g, 128, 0, st>>>(y, acc->stride, mx(B), mv(B->ps[1]), B->s, cap, k);
     if (!QG_LAUNCHED("mrhs_flush_slot")) return false;
     if (!slot_residual(B, k, sl, B->rudev + 4 * k)) return false;
     upd.push_back(k);
