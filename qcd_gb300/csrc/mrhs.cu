@@ -236,10 +236,13 @@ __global__ void __launch_bounds__(128) k_wilson_mrhs(const MArgs a)
 // run as FP32 FMAs. With `partials` the epilogue also writes, per 32 sites
 // (blockIdx.x) and slot, the sum of |out|^2 (partials[block * N + slot]) in a
 // fixed order that does not depend on the occupied slots.
-// Bound by instruction issue and FP32 arithmetic like the single-RHS FP16
-// kernel: 24^3 x 48, 16 slots, 0.637 ms (39.8 us a slot against 47.1). Packed
-// FP32 operations over the two slots (links stored twice, since a broadcast
-// costs two moves) needed more registers than they freed and took 0.74 ms.
+// Bound by latency at 16 warps per SM and by instruction issue (64 % of the
+// cycles), not by memory (39 % of the DRAM's rate): 24^3 x 48, 16 slots,
+// 0.612 ms (38.3 us a slot; one slot of the single-RHS FP16 kernel takes 47.1).
+// Packed FP32 operations over the two slots took longer: 0.74 ms with the links
+// stored twice in memory (more registers than they freed), 0.87 ms with them
+// staged twice in shared memory (7 % fewer instructions, since pairing values
+// costs moves, and less of the L1 left for neighbours).
 
 // spinor and norm of slot r at y
 __device__ __forceinline__ void mload_slot(const MArgs &a, const __half2 *d, const float *dn, int y, int r,
@@ -279,34 +282,58 @@ struct SlotPair {
   int64_t next;
 };
 
-template <int MU, bool BACK, bool DAG, bool EO>
+// the stored words and norm of one slot's spinor
+struct SlotWords {
+  uint4 w[3];
+  float n;
+};
+
+// slot q of the pair at the neighbour in direction D = 2 mu + (backward)
+template <int D, bool EO>
+__device__ __forceinline__ SlotWords load_words(const MArgs &a, const SlotPair &in, int q, int x, const int c[4])
+{
+  const int y = D & 1 ? bwd(a.geo, x, c, D >> 1) : fwd(a.geo, x, c, D >> 1);
+  const int ys = EO ? (y >> 1) : y;
+  const uint4 *p = in.w + q * in.next + ys;
+  SlotWords v;
+#pragma unroll
+  for (int j = 0; j < 3; j++) v.w[j] = __ldg(p + j * a.stride);
+  v.n = __ldg(in.n + q * 4 * in.next + ys);
+  return v;
+}
+
+template <int D, bool DAG>
+__device__ __forceinline__ void mhop_slot(const C<float> U[9], const SlotWords &v, C<float> acc[12])
+{
+  constexpr int MU = D >> 1;
+  constexpr bool BACK = D & 1;
+  constexpr int S = (DAG ? 1 : -1) * (BACK ? -1 : 1);  // projector sign
+  // the projection adds the stored half pairs, then the six projected
+  // components are converted; the slot's site norm scales the accumulation
+  C<float> h[6], uh[6];
+  project_words<MU, S>(v.w, h);
+#pragma unroll
+  for (int j = 0; j < 2; j++)
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+      uh[3 * j + i] =
+          BACK ? cmadd_conj(U[6 + i], h[3 * j + 2], cmadd_conj(U[3 + i], h[3 * j + 1], cdot(U[i], h[3 * j])))
+               : cmadd(U[3 * i + 2], h[3 * j + 2], cmadd(U[3 * i + 1], h[3 * j + 1], U[3 * i] * h[3 * j]));
+  accumulate_scaled<MU, S>(acc, uh, v.n);
+}
+
+// the hop of direction D. Both slots' words are asked for before the first
+// slot's arithmetic: one wait for memory per direction instead of two (16 slots
+// of 24^3 x 48, 637 -> 612 us; fetching the next direction's words as well
+// takes registers that the accumulators need, 640 us).
+template <int D, bool DAG, bool EO>
 __device__ __forceinline__ void mhop(const MArgs &a, const SlotPair &in, int x, const int c[4], C<float> acc[2][12])
 {
-  constexpr int S = (DAG ? 1 : -1) * (BACK ? -1 : 1);  // projector sign
-  const int y = BACK ? bwd(a.geo, x, c, MU) : fwd(a.geo, x, c, MU);
-  const int ys = EO ? (y >> 1) : y;
   C<float> U[9];
-  Link<QCDGPU_F32, 18, float>::load(a.gauge, a.gstride, BACK ? y : x, MU, U);
-#pragma unroll
-  for (int q = 0; q < 2; q++) {
-    // the projection adds the stored half pairs, then the six projected
-    // components are converted; the slot's site norm scales the accumulation
-    const uint4 *p = in.w + q * in.next + ys;
-    const float nrm = __ldg(in.n + q * 4 * in.next + ys);
-    uint4 w[3];
-#pragma unroll
-    for (int j = 0; j < 3; j++) w[j] = __ldg(p + j * a.stride);
-    C<float> h[6], uh[6];
-    project_words<MU, S>(w, h);
-#pragma unroll
-    for (int j = 0; j < 2; j++)
-#pragma unroll
-      for (int i = 0; i < 3; i++)
-        uh[3 * j + i] =
-            BACK ? cmadd_conj(U[6 + i], h[3 * j + 2], cmadd_conj(U[3 + i], h[3 * j + 1], cdot(U[i], h[3 * j])))
-                 : cmadd(U[3 * i + 2], h[3 * j + 2], cmadd(U[3 * i + 1], h[3 * j + 1], U[3 * i] * h[3 * j]));
-    accumulate_scaled<MU, S>(acc[q], uh, nrm);
-  }
+  Link<QCDGPU_F32, 18, float>::load(a.gauge, a.gstride, D & 1 ? bwd(a.geo, x, c, D >> 1) : x, D >> 1, U);
+  const SlotWords v0 = load_words<D, EO>(a, in, 0, x, c), v1 = load_words<D, EO>(a, in, 1, x, c);
+  mhop_slot<D, DAG>(U, v0, acc[0]);
+  mhop_slot<D, DAG>(U, v1, acc[1]);
 }
 
 // MODE 0: full lattice, out = A in - H in / 2. Even/odd (half fields): MODE 1
@@ -336,14 +363,14 @@ __global__ void __launch_bounds__(256, 2) k_wilson_mrhs_simt(const MArgs a, doub
     for (int q = 0; q < 2; q++)
 #pragma unroll
       for (int k = 0; k < 12; k++) acc[q][k] = C<float>{0.f, 0.f};
-    mhop<0, false, DAG, EO>(a, in, x, c, acc);
-    mhop<0, true, DAG, EO>(a, in, x, c, acc);
-    mhop<1, false, DAG, EO>(a, in, x, c, acc);
-    mhop<1, true, DAG, EO>(a, in, x, c, acc);
-    mhop<2, false, DAG, EO>(a, in, x, c, acc);
-    mhop<2, true, DAG, EO>(a, in, x, c, acc);
-    mhop<3, false, DAG, EO>(a, in, x, c, acc);
-    mhop<3, true, DAG, EO>(a, in, x, c, acc);
+    mhop<0, DAG, EO>(a, in, x, c, acc);
+    mhop<1, DAG, EO>(a, in, x, c, acc);
+    mhop<2, DAG, EO>(a, in, x, c, acc);
+    mhop<3, DAG, EO>(a, in, x, c, acc);
+    mhop<4, DAG, EO>(a, in, x, c, acc);
+    mhop<5, DAG, EO>(a, in, x, c, acc);
+    mhop<6, DAG, EO>(a, in, x, c, acc);
+    mhop<7, DAG, EO>(a, in, x, c, acc);
     constexpr bool ainv = MODE == 1;
     constexpr float ch = MODE == 0 ? -0.5f : MODE == 1 ? 1.0f : -0.25f;
 #pragma unroll

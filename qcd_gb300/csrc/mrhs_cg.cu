@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(kMSites) k_mupdate(MX xs, MV ps, MV rs, MV aps
 // the second direction in place of A p, which their operator leaves where D p
 // was. The full operator needs both, and no batch takes more memory for its
 // update: pn and po are the same field there, and k_mupdate adds to xs. The two
-// kernels take 50 us an iteration for 8 slots of 16^3 x 32 (64 before), at the
+// kernels take 50 us an iteration for 12 slots of 16^3 x 32 (64 before), at the
 // memory's rate.
 template <bool XUPD>
 __global__ void __launch_bounds__(kMSites) k_mp(MV pn, MV po, MV rs, MX xs, const double *s, int N)
