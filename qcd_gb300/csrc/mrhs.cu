@@ -1170,11 +1170,21 @@ static std::map<std::pair<int64_t, int>, MrhsTune> g_mrhs_tuned;
 // (slot, site) block of the mma.sync variant's norm kernel
 static dim3 mnorm_block(int N) { return dim3((unsigned)N, (unsigned)(256 / N)); }
 
-// the largest block count of any launch that writes per-slot partial sums
+// the largest block count of any launch that writes per-slot partial sums: SIMT,
+// mma.sync (its norm kernel), tcgen05 (on small lattices the largest)
 unsigned mrhs_max_blocks(int64_t V, int N)
 {
   const unsigned simt = (unsigned)((V + 31) / 32), y = mnorm_block(N).y, mma = (unsigned)((V + y - 1) / y);
-  return simt > mma ? simt : mma;
+  const unsigned tc = mrhs_tc_grid(V), m = simt > mma ? simt : mma;
+  return m > tc ? m : tc;
+}
+
+// the caller's buffer holds mrhs_max_blocks sums per slot
+static bool partials_fit(const MArgs &a, const double *partials, unsigned blocks)
+{
+  if (!partials || blocks <= mrhs_max_blocks(a.V, a.N)) return true;
+  set_error("multi-RHS operator: %u blocks of partial sums, room for %u", blocks, mrhs_max_blocks(a.V, a.N));
+  return false;
 }
 
 static bool launch_mrhs(const MArgs &a, bool dag, MrhsTune t, double *partials, unsigned *nblocks)
@@ -1193,6 +1203,7 @@ static bool launch_mrhs(const MArgs &a, bool dag, MrhsTune t, double *partials, 
     }
     const TcCtl ctl{g_tc_polls, g_tc_skip_mma, g_tc_fail_dev};
     const unsigned grid = mrhs_tc_grid(a.V);
+    if (!partials_fit(a, partials, grid)) return false;
     const int mode = a.eo_par < 0 ? 0 : a.ainv ? 1 : 2;
     if (dag) {
       if (mode == 0) launch_tc<true, 0>(a, partials, grid, s, ctl);
@@ -1214,6 +1225,7 @@ static bool launch_mrhs(const MArgs &a, bool dag, MrhsTune t, double *partials, 
     // sums does not depend on the occupied slots.
     const int pairs = (a.nact + 1) / 2, pb = pairs < t.threads / 32 ? pairs : t.threads / 32;
     const dim3 grid((unsigned)((a.V + 31) / 32), (unsigned)((pairs + pb - 1) / pb)), blk(32, (unsigned)pb);
+    if (!partials_fit(a, partials, grid.x)) return false;
     // kernel mode from the epilogue (see k_wilson_mrhs_simt)
     const int mode = a.eo_par < 0 ? 0 : a.ainv ? 1 : 2;
 #define QG_SIMT(MODE)                                                            \
@@ -1247,6 +1259,7 @@ static bool launch_mrhs(const MArgs &a, bool dag, MrhsTune t, double *partials, 
       const dim3 blk = mnorm_block(a.N);
       const unsigned nb = (unsigned)((a.V + blk.y - 1) / blk.y);
       const size_t shm = sizeof(double) * a.N * blk.y;
+      if (!partials_fit(a, partials, nb)) return false;
       if (nblocks) *nblocks = nb;
       k_mnorm<<<nb, blk, shm, s>>>(a.out, a.out_norm, a.stride, a.V, a.N, a.nact, partials);
       if (!QG_LAUNCHED("mrhs_norm")) return false;
