@@ -186,22 +186,22 @@ __device__ __forceinline__ void put_link(void *dst, int64_t stride, int64_t x, i
     for (int k = 0; k < 9; k++) d[k * stride] = make_double2(U[k].re, U[k].im);
   } else if (P == QCDGPU_F32) {
     if (recon == 12) {
-      float4 *d = (float4 *)dst + (int64_t)mu * 3 * stride + x;
+      float4 *d = (float4 *)dst + gword<3>(x, mu, 0);
       for (int j = 0; j < 3; j++)
-        d[j * stride] = make_float4((float)U[2 * j].re, (float)U[2 * j].im, (float)U[2 * j + 1].re,
+        d[32 * j] = make_float4((float)U[2 * j].re, (float)U[2 * j].im, (float)U[2 * j + 1].re,
                                     (float)U[2 * j + 1].im);
     } else {
-      float2 *d = (float2 *)dst + (int64_t)mu * 9 * stride + x;
-      for (int k = 0; k < 9; k++) d[k * stride] = make_float2((float)U[k].re, (float)U[k].im);
+      float2 *d = (float2 *)dst + gword<9>(x, mu, 0);
+      for (int k = 0; k < 9; k++) d[32 * k] = make_float2((float)U[k].re, (float)U[k].im);
     }
   } else {
-    uint2 *d = (uint2 *)dst + (int64_t)mu * 3 * stride + x;
+    uint2 *d = (uint2 *)dst + gword<3>(x, mu, 0);
     for (int j = 0; j < 3; j++) {
       uint2 v;
       __half2 *h = reinterpret_cast<__half2 *>(&v);
       h[0] = __floats2half2_rn((float)U[2 * j].re, (float)U[2 * j].im);
       h[1] = __floats2half2_rn((float)U[2 * j + 1].re, (float)U[2 * j + 1].im);
-      d[j * stride] = v;
+      d[32 * j] = v;
     }
   }
 }
@@ -369,7 +369,7 @@ bool gauge_to_ff(qcdgpu_gauge d, qcdgpu_gauge s);  // dslash_df64.cu
 // links of direction mu times e^{i theta_mu / L_mu} (FP32, all 18 reals):
 // the multi-RHS kernels' copy carries the boundary phases, so its forward
 // hops need no phase multiply and its backward hops get the conjugate from U^+
-__global__ void k_fold_phases(float2 *d, int64_t stride, int64_t V, float4 phr, float4 phi)
+__global__ void k_fold_phases(float2 *d, int64_t V, float4 phr, float4 phi)
 {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= V * 4) return;
@@ -377,11 +377,11 @@ __global__ void k_fold_phases(float2 *d, int64_t stride, int64_t V, float4 phr, 
   const int64_t x = i % V;
   const float pr = mu == 0 ? phr.x : mu == 1 ? phr.y : mu == 2 ? phr.z : phr.w;
   const float pi = mu == 0 ? phi.x : mu == 1 ? phi.y : mu == 2 ? phi.z : phi.w;
-  float2 *p = d + (int64_t)mu * 9 * stride + x;
+  float2 *p = d + gword<9>(x, mu, 0);
 #pragma unroll
   for (int k = 0; k < 9; k++) {
-    const float2 u = p[k * stride];
-    p[k * stride] = make_float2(pr * u.x - pi * u.y, pr * u.y + pi * u.x);
+    const float2 u = p[32 * k];
+    p[32 * k] = make_float2(pr * u.x - pi * u.y, pr * u.y + pi * u.x);
   }
 }
 
@@ -401,7 +401,7 @@ bool gauge_fold_phases(qcdgpu_gauge g)
   if (!any) return true;
   const float4 fr = make_float4((float)pr[0], (float)pr[1], (float)pr[2], (float)pr[3]);
   const float4 fi = make_float4((float)pi[0], (float)pi[1], (float)pi[2], (float)pi[3]);
-  k_fold_phases<<<grid_for(g->V * 4, 128), 128, 0, stream()>>>((float2 *)g->data, g->stride, g->V, fr, fi);
+  k_fold_phases<<<grid_for(g->V * 4, 128), 128, 0, stream()>>>((float2 *)g->data, g->V, fr, fi);
   return QG_LAUNCHED("fold_phases");
 }
 

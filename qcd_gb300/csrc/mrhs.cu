@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(128) k_wilson_mrhs(const MArgs a)
               rneg = negB;
             }
             if (nz) {
-              float2 u = __ldg(a.gauge + ((int64_t)mu * 9 + (back ? 3 * cp + cc : 3 * cc + cp)) * a.gstride + ly);
+              float2 u = __ldg(a.gauge + gword<9>(ly, mu, back ? 3 * cp + cc : 3 * cc + cp));
               float wr = u.x, wi = back ? -u.y : u.y;
               if (tw) {
                 float tr = wr * pr - wi * pi;
@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(128) k_wilson_mrhs(const MArgs a)
 // fixed order that does not depend on the occupied slots.
 // Bound by latency at 16 warps per SM and by instruction issue (64 % of the
 // cycles), not by memory (39 % of the DRAM's rate): 24^3 x 48, 16 slots,
-// 0.612 ms (38.3 us a slot; one slot of the single-RHS FP16 kernel takes 47.1).
+// 0.593 ms (37.1 us a slot; one slot of the single-RHS FP16 kernel takes 47).
 // Packed FP32 operations over the two slots took longer: 0.74 ms with the links
 // stored twice in memory (more registers than they freed), 0.87 ms with them
 // staged twice in shared memory (7 % fewer instructions, since pairing values
@@ -850,10 +850,10 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_wilson_mrhs_tc(const MArgs a,
           const int mu = lh >> 1;
           const bool back = lh & 1;
           const int y = nb[ls * 9 + lh];
-          const float2 *gp = a.gauge + (int64_t)mu * 9 * a.gstride + (back ? y : lx);
+          const float2 *gp = a.gauge + gword<9>(back ? y : lx, mu, 0);
 #pragma unroll
           for (int j = 0; j < 3; j++) {
-            const float2 v = __ldg(gp + (int64_t)(back ? 3 * j + li : 3 * li + j) * a.gstride);
+            const float2 v = __ldg(gp + 32 * (back ? 3 * j + li : 3 * li + j));
             m[j] = C<float>{v.x, back ? -v.y : v.y};
           }
         }
