@@ -493,19 +493,19 @@ int qcdgpu_mfield_get(qcdgpu_field f, qcdgpu_mfield m, int r);
  * the FP64 gauge field */
 int qcdgpu_dslash_mrhs(qcdgpu_mfield out, qcdgpu_mfield in, qcdgpu_gauge g, double kappa, double mu, int op,
                        int nact);
-/* The operator has three kernels: SIMT (one thread per site and RHS, links
- * shared through L1), tcgen05 tensor cores (one FP16 GEMM per site and
+/* The operator has three kernels: SIMT (one thread per site and one or two RHS,
+ * links shared through L1), tcgen05 tensor cores (one FP16 GEMM per site and
  * 16-slot group, the eight hops concatenated along K, FP32 accumulators in
  * tensor memory; slot counts that are multiples of 16) and mma.sync tensor
- * cores (one warp per site, TF32; full lattice only). By default (-1) the
- * first call for a lattice volume and slot count times the SIMT kernel with
- * 64-, 128- and 256-thread blocks and one or two slots per thread and the
- * tensor-core kernels, and keeps the fastest; 1 forces the mma.sync kernel,
- * 2 the tcgen05 kernel, 64 / 128 / 256 (+1: two slots per thread) the SIMT
- * kernel with that block size. */
+ * cores (one warp per site, TF32; full lattice only). By default (-1) the SIMT
+ * kernel runs, with slots per thread and a block size chosen by the volume and
+ * the occupied slots (the tensor-core kernels are slower at every size
+ * measured); 1 forces the mma.sync kernel, 2 the tcgen05 kernel, 64 / 128 / 256
+ * (+1: two slots per thread) the SIMT kernel with that block size. */
 int qcdgpu_set_mrhs_variant(int variant);
-/* the tuned choice for (L, nrhs): variant 0 SIMT / 1 mma.sync / 2 tcgen05
- * and the SIMT block size; returns 1 when nothing has been tuned for it yet */
+/* the choice for (L, nrhs) with all slots occupied: variant 0 SIMT / 1 mma.sync /
+ * 2 tcgen05 and the SIMT block size (+1: two slots per thread); returns 1 before
+ * the first apply of that shape */
 int qcdgpu_mrhs_tuned(const int L[4], int nrhs, int *variant, int *threads);
 /* Every wait of the tcgen05 kernel for its MMAs is bounded. A wait that runs
  * out makes the launch abandon its work (its output is invalid) and sets a

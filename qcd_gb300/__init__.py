@@ -503,12 +503,12 @@ def twop_proton(up, dn, xsrc, t0: int, t1: int, moms) -> np.ndarray:
 
 
 def set_mrhs_variant(v: int) -> None:
-    """-1: tuned; 1: tensor-core kernel; 64 / 128 / 256: SIMT kernel with that block size."""
+    """-1: chosen by size; 1, 2: tensor-core kernels; 64 / 128 / 256 (+1: two slots per thread): SIMT of that block size."""
     _check(lib().qcdgpu_set_mrhs_variant(v), "qcdgpu_set_mrhs_variant")
 
 
 def mrhs_tuned(L, nrhs):
-    """(variant, threads) the tuner chose for this volume and slot count, or None."""
+    """(variant, threads) that calls of this volume and slot count run, or None before the first."""
     v, t = C.c_int(), C.c_int()
     if lib().qcdgpu_mrhs_tuned(np.asarray(L, np.int32), nrhs, C.byref(v), C.byref(t)) != 0:
         return None

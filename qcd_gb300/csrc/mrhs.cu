@@ -21,6 +21,7 @@
 #include <string.h>
 
 #include <map>
+#include <mutex>
 #include <utility>
 
 #include "mrhs.h"
@@ -229,10 +230,10 @@ __global__ void __launch_bounds__(128) k_wilson_mrhs(const MArgs a)
 }
 
 // ------------------------------------------------ SIMT variant (FP32 cores)
-// One thread per site and two adjacent RHS slots; a warp takes 32 consecutive
-// sites of a slot pair, the warps of a block the same sites of several pairs:
-// each link a thread loads serves two slots, and the block's pairs meet in L1
-// for it, while the per-RHS spin projection, link products and reconstruction
+// One thread per site and two adjacent RHS slots (or one: simt_shape); a warp
+// takes 32 consecutive sites of a slot pair, the warps of a block the same sites
+// of several pairs: each link a thread loads serves two slots, and the block's
+// pairs meet in L1 for it, while the per-RHS spin projection, link products and reconstruction
 // run as FP32 FMAs. With `partials` the epilogue also writes, per 32 sites
 // (blockIdx.x) and slot, the sum of |out|^2 (partials[block * N + slot]) in a
 // fixed order that does not depend on the occupied slots.
@@ -275,7 +276,8 @@ __device__ __forceinline__ void project_words(const uint4 w[3], C<float> h[6])
 }
 
 // two adjacent slots of a field: the first one's words and norms, and how far
-// the second one's lie (in words; four floats each)
+// the second one's lie (in words; four floats each). Behind the last occupied
+// slot there is none: the thread reads the first one's twice (distance 0)
 struct SlotPair {
   const uint4 *w;
   const float *n;
@@ -326,26 +328,31 @@ __device__ __forceinline__ void mhop_slot(const C<float> U[9], const SlotWords &
 // slot's arithmetic: one wait for memory per direction instead of two (16 slots
 // of 24^3 x 48, 637 -> 612 us; fetching the next direction's words as well
 // takes registers that the accumulators need, 640 us).
-template <int D, bool DAG, bool EO>
-__device__ __forceinline__ void mhop(const MArgs &a, const SlotPair &in, int x, const int c[4], C<float> acc[2][12])
+template <int D, bool DAG, bool EO, int NS>
+__device__ __forceinline__ void mhop(const MArgs &a, const SlotPair &in, int x, const int c[4], C<float> acc[NS][12])
 {
   C<float> U[9];
   Link<QCDGPU_F32, 18, float>::load(a.gauge, a.gstride, D & 1 ? bwd(a.geo, x, c, D >> 1) : x, D >> 1, U);
-  const SlotWords v0 = load_words<D, EO>(a, in, 0, x, c), v1 = load_words<D, EO>(a, in, 1, x, c);
-  mhop_slot<D, DAG>(U, v0, acc[0]);
-  mhop_slot<D, DAG>(U, v1, acc[1]);
+  const SlotWords v0 = load_words<D, EO>(a, in, 0, x, c);
+  if constexpr (NS == 2) {
+    const SlotWords v1 = load_words<D, EO>(a, in, 1, x, c);
+    mhop_slot<D, DAG>(U, v0, acc[0]);
+    mhop_slot<D, DAG>(U, v1, acc[1]);
+  } else {
+    mhop_slot<D, DAG>(U, v0, acc[0]);
+  }
 }
 
 // MODE 0: full lattice, out = A in - H in / 2. Even/odd (half fields): MODE 1
 // out = A^{-1} H in; MODE 2 out = A z - H in / 4 (the two halves of the Schur
 // complement). The epilogue is fixed at compile time for each mode.
-template <bool DAG, int MODE>
-__global__ void __launch_bounds__(256, 2) k_wilson_mrhs_simt(const MArgs a, double *partials)
+template <bool DAG, int MODE, int NS>
+__global__ void __launch_bounds__(256, NS == 2 ? 2 : 3) k_wilson_mrhs_simt(const MArgs a, double *partials)
 {
   constexpr bool EO = MODE != 0;
-  const int r0 = 2 * (blockIdx.y * blockDim.y + threadIdx.y);
+  const int r0 = NS * (blockIdx.y * blockDim.y + threadIdx.y);
   const int e = blockIdx.x * 32 + threadIdx.x;  // output index
-  double n2[2] = {0.0, 0.0};
+  double n2[NS] = {};
   if (r0 < a.nact && e < a.V) {
     int c[4], x = e;
     if (EO) {  // the site of parity eo_par among full indices 2e, 2e + 1 (even t extent)
@@ -357,28 +364,28 @@ __global__ void __launch_bounds__(256, 2) k_wilson_mrhs_simt(const MArgs a, doub
       coords(a.geo, x, c);
     }
     const SlotPair in{(const uint4 *)a.in + mword(a.stride, 0, 0, r0), a.in_norm + mnorm_at(a.stride, 0, r0),
-                      mword(a.stride, 0, 0, 1)};
-    C<float> acc[2][12];
+                      r0 + 1 < a.nact ? mword(a.stride, 0, 0, 1) : 0};
+    C<float> acc[NS][12];
 #pragma unroll
-    for (int q = 0; q < 2; q++)
+    for (int q = 0; q < NS; q++)
 #pragma unroll
       for (int k = 0; k < 12; k++) acc[q][k] = C<float>{0.f, 0.f};
-    mhop<0, DAG, EO>(a, in, x, c, acc);
-    mhop<1, DAG, EO>(a, in, x, c, acc);
-    mhop<2, DAG, EO>(a, in, x, c, acc);
-    mhop<3, DAG, EO>(a, in, x, c, acc);
-    mhop<4, DAG, EO>(a, in, x, c, acc);
-    mhop<5, DAG, EO>(a, in, x, c, acc);
-    mhop<6, DAG, EO>(a, in, x, c, acc);
-    mhop<7, DAG, EO>(a, in, x, c, acc);
+    mhop<0, DAG, EO, NS>(a, in, x, c, acc);
+    mhop<1, DAG, EO, NS>(a, in, x, c, acc);
+    mhop<2, DAG, EO, NS>(a, in, x, c, acc);
+    mhop<3, DAG, EO, NS>(a, in, x, c, acc);
+    mhop<4, DAG, EO, NS>(a, in, x, c, acc);
+    mhop<5, DAG, EO, NS>(a, in, x, c, acc);
+    mhop<6, DAG, EO, NS>(a, in, x, c, acc);
+    mhop<7, DAG, EO, NS>(a, in, x, c, acc);
     constexpr bool ainv = MODE == 1;
     constexpr float ch = MODE == 0 ? -0.5f : MODE == 1 ? 1.0f : -0.25f;
 #pragma unroll
-    for (int q = 0; q < 2; q++) {
+    for (int q = 0; q < NS; q++) {
       const int r = r0 + q;
-      // slots past nact hold zeros; their results are not stored
-      const float mp4r = a.mp4s ? a.mp4s[r] : a.mp4;
-      const float tmr = a.tms ? (DAG ? -a.tms[r] : a.tms[r]) : a.tm;
+      const int rz = NS == 1 || r < a.nact ? r : r0;  // results of slots past nact are not stored
+      const float mp4r = a.mp4s ? a.mp4s[rz] : a.mp4;
+      const float tmr = a.tms ? (DAG ? -a.tms[rz] : a.tms[rz]) : a.tm;
       float mx = 0.f;
       if constexpr (ainv) {  // ch A^{-1} = ch (mp4 - i tm g5) / (mp4^2 + tm^2), no addend
         const float den = ch / (mp4r * mp4r + tmr * tmr), ar = mp4r * den, ai = -tmr * den;
@@ -391,7 +398,7 @@ __global__ void __launch_bounds__(256, 2) k_wilson_mrhs_simt(const MArgs a, doub
       } else {  // ch H in + A z
         C<float> s[12];
         float zs;
-        mload_slot(a, EO ? a.z : a.in, EO ? a.z_norm : a.in_norm, e, r, s, zs);
+        mload_slot(a, EO ? a.z : a.in, EO ? a.z_norm : a.in_norm, e, rz, s, zs);
         const float zm = mp4r * zs, zt = tmr * zs;
 #pragma unroll
         for (int k = 0; k < 12; k++) {
@@ -424,7 +431,7 @@ __global__ void __launch_bounds__(256, 2) k_wilson_mrhs_simt(const MArgs a, doub
   }
   if (partials) {
 #pragma unroll
-    for (int q = 0; q < 2; q++) {
+    for (int q = 0; q < NS; q++) {
       double t = n2[q];
       for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
       if (threadIdx.x == 0 && r0 + q < a.N) partials[(int64_t)blockIdx.x * a.N + r0 + q] = t;
@@ -448,9 +455,7 @@ qcdgpu_mfield mfield_new(const int L[4], int N)
   m->V = (int64_t)L[0] * L[1] * L[2] * L[3];
   m->stride = pad_stride(m->V);
   m->N = N;
-  // the operator's threads hold two slots: an odd count has a spare one, which
-  // is read (as zeros) and never written
-  m->bytes = slot * (size_t)(N + N % 2);
+  m->bytes = slot * (size_t)N;
   if (!QG_CUDA(cudaMalloc(&m->data, m->bytes))) {
     delete m;
     return nullptr;
@@ -506,6 +511,27 @@ __global__ void k_unpack(void *f, float *fn, int64_t stride, const __half2 *d, c
   Spinor<P, float>::store(f, fn, stride, x, s);
 }
 
+// An FP16 field in or out of its slot: the same image (a copy kernel, four words
+// of 16 bytes in flight per thread; the runtime's device copy takes 8 us from a
+// few MB on)
+__global__ void __launch_bounds__(256) k_slot_copy(uint4 *d, const uint4 *s, int64_t n)
+{
+  const int64_t i0 = (int64_t)blockIdx.x * 1024 + threadIdx.x;
+  uint4 w[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++)
+    if (i0 + 256 * k < n) w[k] = s[i0 + 256 * k];
+#pragma unroll
+  for (int k = 0; k < 4; k++)
+    if (i0 + 256 * k < n) d[i0 + 256 * k] = w[k];
+}
+static bool slot_copy(void *d, const void *s, size_t bytes)
+{
+  const int64_t n = (int64_t)(bytes / sizeof(uint4));  // whole words: 52 bytes times a multiple of 128 sites
+  k_slot_copy<<<(unsigned)((n + 1023) / 1024), 256, 0, stream()>>>((uint4 *)d, (const uint4 *)s, n);
+  return QG_LAUNCHED("mrhs_slot_copy");
+}
+
 bool mfield_set(qcdgpu_mfield m, int r, qcdgpu_field f)
 {
   if (!m || !f || r < 0 || r >= m->N || f->V != m->V) {
@@ -515,8 +541,7 @@ bool mfield_set(qcdgpu_mfield m, int r, qcdgpu_field f)
   const unsigned g = (unsigned)((m->V + 127) / 128);
   __half2 *d = (__half2 *)m->data;
   if (f->prec == QCDGPU_F16)
-    return QG_CUDA(cudaMemcpyAsync((char *)m->data + (size_t)r * f->bytes, f->data, f->bytes, cudaMemcpyDeviceToDevice,
-                                   stream()));
+    return slot_copy((char *)m->data + (size_t)r * f->bytes, f->data, f->bytes);
   if (f->prec == QCDGPU_F64) k_pack<QCDGPU_F64><<<g, 128, 0, stream()>>>(d, m->norm, m->stride, (int)m->V, r, f->data, f->norm, f->stride);
   else k_pack<QCDGPU_F32><<<g, 128, 0, stream()>>>(d, m->norm, m->stride, (int)m->V, r, f->data, f->norm, f->stride);
   return QG_LAUNCHED("mrhs_pack");
@@ -531,8 +556,7 @@ bool mfield_get(qcdgpu_field f, qcdgpu_mfield m, int r)
   const unsigned g = (unsigned)((m->V + 127) / 128);
   const __half2 *d = (const __half2 *)m->data;
   if (f->prec == QCDGPU_F16)
-    return QG_CUDA(cudaMemcpyAsync(f->data, (const char *)m->data + (size_t)r * f->bytes, f->bytes,
-                                   cudaMemcpyDeviceToDevice, stream()));
+    return slot_copy(f->data, (const char *)m->data + (size_t)r * f->bytes, f->bytes);
   if (f->prec == QCDGPU_F64) k_unpack<QCDGPU_F64><<<g, 128, 0, stream()>>>(f->data, f->norm, f->stride, d, m->norm, m->stride, (int)m->V, r);
   else k_unpack<QCDGPU_F32><<<g, 128, 0, stream()>>>(f->data, f->norm, f->stride, d, m->norm, m->stride, (int)m->V, r);
   return QG_LAUNCHED("mrhs_unpack");
@@ -540,7 +564,7 @@ bool mfield_get(qcdgpu_field f, qcdgpu_mfield m, int r)
 
 // out = D in (dag: D^+ in) for the first nact RHS of the two fields; with
 // mp4s / tms (device float arrays) each slot r uses its own diagonal
-// ------------------------------------------------------------ launch + tuner
+// ------------------------------------------------------------ launch
 // per-slot sum of |v|^2 over the block's sites (for the tensor-core variant,
 // whose epilogue has no reduction); block (N, SB) like the SIMT variant
 __global__ void k_mnorm(const __half2 *d, const float *dn, int64_t S, int V, int N, int nact, double *partials)
@@ -1161,10 +1185,12 @@ bool mrhs_tc_failed() { return g_tc_fail_host && *g_tc_fail_host; }
 
 struct MrhsTune {
   int variant;  // MRHS_SIMT, MRHS_MMA or MRHS_TC
-  int threads;  // SIMT: threads per block, 64, 128 or 256
+  int threads;  // SIMT: threads per block (0: by simt_shape)
+  int slots;    // SIMT: slots per thread, 1 or 2 (0: by simt_shape)
 };
 
 static int g_mrhs_variant = MRHS_AUTO;
+static std::mutex g_mrhs_mu;  // of the map
 static std::map<std::pair<int64_t, int>, MrhsTune> g_mrhs_tuned;
 
 // (slot, site) block of the mma.sync variant's norm kernel
@@ -1177,6 +1203,36 @@ unsigned mrhs_max_blocks(int64_t V, int N)
   const unsigned simt = (unsigned)((V + 31) / 32), y = mnorm_block(N).y, mma = (unsigned)((V + y - 1) / y);
   const unsigned tc = mrhs_tc_grid(V), m = simt > mma ? simt : mma;
   return m > tc ? m : tc;
+}
+
+// A SIMT launch: slots per thread, warps (of 32 sites and one slot or slot pair)
+// per block, and blocks over the slots. A slot's result does not depend on it.
+struct SimtShape {
+  int slots, warps, groups;
+};
+
+// Two slots per thread share a link's registers; one slot per thread has the
+// most warps and leaves no half of the last pair idle. So one slot for odd
+// counts below 16 (24^3 x 48, one and two per thread: 1 slot 54 and 78 us, 3
+// slots 120 and 149, 9 slots 363 and 400, 15 slots 584 and 588; the links' share
+// is 38.3 us a slot against 37.1), and where the pairs' warps are fewer than
+// eight per SM (8^3 x 16: 2 slots 6.4 and 8.4 us, 8 slots the same).
+// Warps per block, whose slots' links meet in the L1: all of up to four; of more
+// pairs two (16 slots of 32^3 x 64: two 1.926 ms, four 1.970, eight 2.026; 12
+// slots of 24^3 x 48: 445, three 460 us), or four where the lattice is small and
+// four divide them (32 slots of 16^3 x 32: 235 and 230 us); an odd number of them
+// in even shares of up to four (10 slots of 24^3 x 48: two 438, three 405 us).
+static SimtShape simt_shape(int V, int nact, const MrhsTune &t)
+{
+  if (t.slots) {  // asked for
+    const int n = (nact + t.slots - 1) / t.slots, w = n < t.threads / 32 ? n : t.threads / 32;
+    return {t.slots, w, (n + w - 1) / w};
+  }
+  const bool one = (nact % 2 && nact < 16) || (int64_t)((V + 31) / 32) * ((nact + 1) / 2) < 8 * 152;
+  const int n = one ? nact : (nact + 1) / 2;
+  if (!one && n > 4 && n % 2 == 0 && !(n % 4 == 0 && V <= (1 << 18))) return {2, 2, n / 2};
+  const int groups = (n + 3) / 4, w = (n + groups - 1) / groups;
+  return {one ? 1 : 2, w, (n + w - 1) / w};
 }
 
 // the caller's buffer holds mrhs_max_blocks sums per slot
@@ -1223,14 +1279,20 @@ static bool launch_mrhs(const MArgs &a, bool dag, MrhsTune t, double *partials, 
     // warps: 32 sites of one slot pair; a block holds several pairs of the
     // same sites (their links meet in L1). The grouping of a slot's partial
     // sums does not depend on the occupied slots.
-    const int pairs = (a.nact + 1) / 2, pb = pairs < t.threads / 32 ? pairs : t.threads / 32;
-    const dim3 grid((unsigned)((a.V + 31) / 32), (unsigned)((pairs + pb - 1) / pb)), blk(32, (unsigned)pb);
+    const SimtShape sh = simt_shape(a.V, a.nact, t);
+    const dim3 grid((unsigned)((a.V + 31) / 32), (unsigned)sh.groups), blk(32, (unsigned)sh.warps);
     if (!partials_fit(a, partials, grid.x)) return false;
     // kernel mode from the epilogue (see k_wilson_mrhs_simt)
     const int mode = a.eo_par < 0 ? 0 : a.ainv ? 1 : 2;
 #define QG_SIMT(MODE)                                                            \
-  if (dag) k_wilson_mrhs_simt<true, MODE><<<grid, blk, 0, s>>>(a, partials);     \
-  else k_wilson_mrhs_simt<false, MODE><<<grid, blk, 0, s>>>(a, partials);
+  if (sh.slots == 2) {                                                           \
+    if (dag) k_wilson_mrhs_simt<true, MODE, 2><<<grid, blk, 0, s>>>(a, partials); \
+    else k_wilson_mrhs_simt<false, MODE, 2><<<grid, blk, 0, s>>>(a, partials);   \
+  } else if (dag) {                                                              \
+    k_wilson_mrhs_simt<true, MODE, 1><<<grid, blk, 0, s>>>(a, partials);         \
+  } else {                                                                       \
+    k_wilson_mrhs_simt<false, MODE, 1><<<grid, blk, 0, s>>>(a, partials);        \
+  }
     if (mode == 0) {
       QG_SIMT(0)
     } else if (mode == 1) {
@@ -1268,53 +1330,24 @@ static bool launch_mrhs(const MArgs &a, bool dag, MrhsTune t, double *partials, 
   return true;
 }
 
-// Pick the SIMT kernel's block size for (V, N) by timing each candidate three
-// times on the caller's fields (the output is overwritten with the same
-// result). Not while the stream is being captured: then 64-thread blocks run
-// until a tuned choice exists. The tensor-core kernels have lost to SIMT at
-// every volume and slot count measured (by factors of 2 and 9): they run when
-// asked for, and a first apply does not spend its time on them.
-static MrhsTune mrhs_tune(const MArgs &a, bool dag)
+// the variant of a call: the one asked for, or SIMT with the shape of
+// simt_shape. The tensor-core kernels have lost to SIMT at every volume and slot
+// count measured (by factors of 2 and 9) and run when asked for.
+static MrhsTune mrhs_choice(const MArgs &a)
 {
-  if (g_mrhs_variant == MRHS_MMA) return MrhsTune{MRHS_MMA, 256};
-  if (g_mrhs_variant == MRHS_TC) return MrhsTune{MRHS_TC, kTcThreads};
-  if (g_mrhs_variant >= 64) return MrhsTune{MRHS_SIMT, g_mrhs_variant & ~1};  // forced block size
-  // even/odd kernels are tuned separately (key: minus the half volume)
+  if (g_mrhs_variant == MRHS_MMA) return MrhsTune{MRHS_MMA, 256, 0};
+  if (g_mrhs_variant == MRHS_TC) return MrhsTune{MRHS_TC, kTcThreads, 0};
+  if (g_mrhs_variant >= 64) return MrhsTune{MRHS_SIMT, g_mrhs_variant & ~1, 1 + (g_mrhs_variant & 1)};
+  const MrhsTune t{MRHS_SIMT, 0, 0};
+  // what a call of this volume and slot count runs, for qcdgpu_mrhs_tuned
+  // (even/odd kernels apart: minus the half volume)
   const auto key = std::make_pair(a.eo_par < 0 ? (int64_t)a.V : -(int64_t)a.V, a.N);
-  auto it = g_mrhs_tuned.find(key);
-  if (it != g_mrhs_tuned.end()) return it->second;
-  const MrhsTune fallback{MRHS_SIMT, 64};
-  if (a.z == a.out) return fallback;  // a repeated launch would read its own result
-  cudaStream_t s = stream();
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return fallback;
-  const MrhsTune cands[] = {{MRHS_SIMT, 64}, {MRHS_SIMT, 128}, {MRHS_SIMT, 256}};
-  cudaEvent_t e0, e1;
-  if (cudaEventCreate(&e0) != cudaSuccess) return fallback;
-  if (cudaEventCreate(&e1) != cudaSuccess) {
-    cudaEventDestroy(e0);
-    return fallback;
+  std::lock_guard<std::mutex> lk(g_mrhs_mu);
+  if (g_mrhs_tuned.find(key) == g_mrhs_tuned.end()) {
+    const SimtShape sh = simt_shape(a.V, a.N, t);
+    g_mrhs_tuned[key] = MrhsTune{MRHS_SIMT, 32 * sh.warps, sh.slots};
   }
-  MrhsTune best = fallback;
-  float best_ms = 1e30f;
-  for (const MrhsTune &c : cands) {
-    if (!launch_mrhs(a, dag, c, nullptr, nullptr)) break;  // warm-up
-    cudaEventRecord(e0, s);
-    bool ok = true;
-    for (int i = 0; i < 3 && ok; i++) ok = launch_mrhs(a, dag, c, nullptr, nullptr);
-    cudaEventRecord(e1, s);
-    if (!ok || cudaEventSynchronize(e1) != cudaSuccess) break;
-    float ms = 0.f;
-    cudaEventElapsedTime(&ms, e0, e1);
-    if (ms < best_ms) {
-      best_ms = ms;
-      best = c;
-    }
-  }
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
-  g_mrhs_tuned[key] = best;
-  return best;
+  return t;
 }
 
 bool dslash_mrhs(qcdgpu_mfield out, qcdgpu_mfield in, qcdgpu_gauge g, double mp4, double tm, bool dag, int nact,
@@ -1371,7 +1404,7 @@ bool dslash_mrhs(qcdgpu_mfield out, qcdgpu_mfield in, qcdgpu_gauge g, double mp4
     if (nblocks) *nblocks = 0;
     return true;
   }
-  const MrhsTune tune = mrhs_tune(a, dag);
+  const MrhsTune tune = mrhs_choice(a);
   if (!launch_mrhs(a, dag, tune, partials, nblocks)) return false;
   return true;
 }
@@ -1435,7 +1468,7 @@ bool dslash_mrhs_eo(qcdgpu_mfield out, qcdgpu_mfield in, qcdgpu_mfield z, qcdgpu
     if (nblocks) *nblocks = 0;
     return true;
   }
-  return launch_mrhs(a, dag, mrhs_tune(a, dag), partials, nblocks);
+  return launch_mrhs(a, dag, mrhs_choice(a), partials, nblocks);
 }
 
 }  // namespace qg
@@ -1458,7 +1491,7 @@ int qcdgpu_set_mrhs_variant(int v)
 {
   if (v != qg::MRHS_AUTO && v != qg::MRHS_MMA && v != qg::MRHS_TC && v != 64 && v != 128 && v != 256 && v != 65 &&
       v != 129 && v != 257) {
-    qg::set_error("multi-RHS variant: -1 (tuned), 1 (tensor cores, mma.sync), 2 (tensor cores, tcgen05; slot "
+    qg::set_error("multi-RHS variant: -1 (chosen by size), 1 (tensor cores, mma.sync), 2 (tensor cores, tcgen05; slot "
                   "counts that are multiples of 16), 64 / 128 / 256 (SIMT, slots x sites per block), +1 for two "
                   "slots per thread");
     return 1;
@@ -1492,10 +1525,11 @@ int qcdgpu_mrhs_tc_test_hook(int skip_mma, int polls)
 int qcdgpu_mrhs_tuned(const int L[4], int nrhs, int *variant, int *threads)
 {
   const int64_t V = (int64_t)L[0] * L[1] * L[2] * L[3];
+  std::lock_guard<std::mutex> lk(qg::g_mrhs_mu);
   auto it = qg::g_mrhs_tuned.find(std::make_pair(V, nrhs));
   if (it == qg::g_mrhs_tuned.end()) return 1;
   *variant = it->second.variant;
-  *threads = it->second.threads + 1;  // two slots per thread
+  *threads = it->second.threads + (it->second.slots == 2 ? 1 : 0);
   return 0;
 }
 

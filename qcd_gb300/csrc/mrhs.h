@@ -92,7 +92,7 @@ bool dslash_mrhs_eo(qcdgpu_mfield out, qcdgpu_mfield in, qcdgpu_mfield z, qcdgpu
 // host-mapped flag the kernel sets: reading it needs no synchronisation)
 bool mrhs_tc_failed();
 
-// operator variants picked by the tuner
+// operator variants
 enum { MRHS_AUTO = -1, MRHS_SIMT = 0, MRHS_MMA = 1, MRHS_TC = 2 };
 
 }  // namespace qg

@@ -310,7 +310,7 @@ struct qcdgpu_batch_s {
   // even/odd: A p is left in t (aps == t), u is the odd intermediate
   qcdgpu_mfield rs, ps[2], t, aps, u;
   float4 *xs;                  // FP32 solution increments (layout of MX)
-  qcdgpu_field rt, r, up, bd;  // FP64 work shared by the slots' reliable updates
+  qcdgpu_field rt, r, bd;      // FP64 work shared by the slots' reliable updates
   qcdgpu_field u64, r32, u32, s32;  // even/odd: FP64 odd temp; FP32 restart fields
   std::vector<qcdgpu_field> spare;  // even/odd: free per-slot x_e fields
   double *s;                   // device scalars, (M_HIST + kMChunk) * cap
@@ -327,7 +327,7 @@ struct qcdgpu_batch_s {
   cudaEvent_t ev_in;           // caller's stream at admission
   int nchunk;                  // occupied slots of the launched chunk
   bool use_graphs;
-  bool tuned;                  // the operator variant has been chosen
+  bool tried;                  // the operator has run once outside stream capture
   std::vector<cudaGraphExec_t> graphs;  // chunk graph per occupied-slot count
   std::vector<uint64_t> graph_launches;  // kernels in each graph
 };
@@ -344,7 +344,7 @@ static void batch_free(qcdgpu_batch b)
   if (b->aps != b->t) mfield_free(b->aps);
   for (auto m : {b->rs, b->ps[0], b->t, b->u}) mfield_free(m);
   cudaFree(b->xs);
-  for (auto f : {b->rt, b->r, b->up, b->bd, b->u64, b->r32, b->u32, b->s32}) field_free(f);
+  for (auto f : {b->rt, b->r, b->bd, b->u64, b->r32, b->u32, b->s32}) field_free(f);
   for (auto &sl : b->slots)
     for (auto f : {sl.ce, sl.to, sl.xe}) field_free(f);
   for (auto f : b->spare) field_free(f);
@@ -381,6 +381,7 @@ static qcdgpu_batch batch_new(qcdgpu_gauge g, int cap, bool eo)
   b->st = nullptr;
   b->nchunk = 0;
   b->use_graphs = true;
+  b->tried = false;
   b->graphs.assign((size_t)cap + 1, nullptr);
   b->graph_launches.assign((size_t)cap + 1, 0);
   b->rs = mfield_new(b->Ls, cap);
@@ -390,9 +391,8 @@ static qcdgpu_batch batch_new(qcdgpu_gauge g, int cap, bool eo)
   b->aps = eo ? b->t : mfield_new(b->Ls, cap);
   b->rt = field_new(b->Ls, QCDGPU_F64);
   b->r = field_new(b->Ls, QCDGPU_F64);
-  b->up = field_new(b->Ls, QCDGPU_F64);
   b->bd = field_new(g->L, QCDGPU_F64);
-  bool ok = b->rs && b->ps[0] && b->ps[1] && b->t && b->aps && b->rt && b->r && b->up && b->bd;
+  bool ok = b->rs && b->ps[0] && b->ps[1] && b->t && b->aps && b->rt && b->r && b->bd;
   if (eo) {
     b->u = mfield_new(b->Ls, cap);
     b->u64 = field_new(b->Ls, QCDGPU_F64);
@@ -694,16 +694,16 @@ bool batch_launch(qcdgpu_batch B)
   StreamScope scope(B->st);
   const int n = B->nchunk;
   if (!gauge_at(B->g, kGaugeF32Full)) return false;  // resident before any capture
-  if (!B->tuned) {
-    // the operator's tuner times its variants outside stream capture; t and
-    // u are scratch (recomputed by every iteration)
+  if (!B->tried) {
+    // what a variant sets up on its first launch cannot be set up under stream
+    // capture; t and u are scratch (recomputed by every iteration)
     const bool ok = B->eo ? dslash_mrhs_eo(B->u, B->ps[1], nullptr, B->g, false, n, B->mp4s, B->tms, 1, 1.0, true, 0,
                                            nullptr, nullptr) &&
                                 dslash_mrhs_eo(B->t, B->u, B->ps[1], B->g, false, n, B->mp4s, B->tms, 0, -0.25, false, 2,
                                                nullptr, nullptr)
                           : dslash_mrhs(B->t, B->ps[1], B->g, 4.0, 0.0, false, n, B->mp4s, B->tms);
     if (!ok) return false;
-    B->tuned = true;
+    B->tried = true;
   }
   if (B->use_graphs) {
     cudaGraphExec_t &ex = B->graphs[(size_t)n];
@@ -890,7 +890,7 @@ int qcdgpu_batch_poll(qcdgpu_batch b, int *tags, int *status, int *iters, double
 size_t qcdgpu_batch_bytes(qcdgpu_batch b)
 {
   if (!b) return 0;
-  size_t n = 4 * b->rs->bytes + (size_t)12 * qg::pad_stride(b->Vs) * b->cap * sizeof(float2) + 3 * b->rt->bytes + b->bd->bytes;
+  size_t n = 4 * b->rs->bytes + (size_t)12 * qg::pad_stride(b->Vs) * b->cap * sizeof(float2) + 2 * b->rt->bytes + b->bd->bytes;
   if (b->eo) n += b->u->bytes + b->u64->bytes + 3 * b->r32->bytes + (size_t)b->cap * b->rt->bytes;
   for (const auto &sl : b->slots)  // c_e, A^{-1} b_o outside x (x too small for both)
     for (auto f : {sl.ce, sl.to})

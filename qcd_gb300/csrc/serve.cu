@@ -79,9 +79,9 @@ static size_t batch_bytes_est(const int L[4], int slots)
   const bool eo = use_eo(L);
   const int Ls[4] = {eo ? L[0] / 2 : L[0], L[1], L[2], L[3]};
   const int64_t Vs = (int64_t)Ls[0] * Ls[1] * Ls[2] * Ls[3];
-  const size_t S = (size_t)pad_stride(Vs), mf = S * 52 * (size_t)(slots + slots % 2);
+  const size_t S = (size_t)pad_stride(Vs), mf = S * 52 * (size_t)slots;
   const size_t f64 = field_bytes_f64(Ls), f32 = f64 / 2;
-  size_t n = 4 * mf + 12 * S * slots * sizeof(float2) + 3 * f64 + field_bytes_f64(L);
+  size_t n = 4 * mf + 12 * S * slots * sizeof(float2) + 2 * f64 + field_bytes_f64(L);
   if (eo) {
     n += mf + f64 + 3 * f32 + (size_t)slots * f64;
     // c_e and A^{-1} b_o get their own memory when x cannot hold both

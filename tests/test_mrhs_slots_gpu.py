@@ -1,5 +1,5 @@
 """Multi-RHS fields and batches where slots and sites do not fill the kernels'
-pairs and warps: odd slot counts (a spare slot pads the last pair), odd
+pairs and warps: odd slot counts (the last pair is one slot), odd
 occupied counts, site counts off 32. The operator against the oracle (4e-3 per
 RHS, the FP16 bar of test_mrhs_gpu.py); FP16 fields go in and come out
 unchanged; odd-capacity batches reach their tolerance."""
@@ -61,4 +61,30 @@ def test_odd_capacity_batches(gpu, orc, cap, n, eo):
         assert orc.true_residual(x.store(), v, u, L, TH, 0.14, 0.01) <= 1e-10
     batch.close()
     for o in fb + fx + [g]:
+        o.close()
+
+
+@pytest.mark.parametrize("L", [(8, 8, 8, 8), (16, 16, 16, 16)])
+@pytest.mark.parametrize("N", [1, 7, 10, 16, 18])
+def test_launch_shapes_agree(gpu, orc, L, N):
+    """Slots per thread, warps per block and blocks over the slots follow the
+    lattice and the occupied slots; a slot's result is the same bits in all."""
+    u = orc.gauge_synthetic(L, 91, EPS_PLAQ_060)
+    g = q.Gauge(L, TH).load(u)
+    inp, out = q.MField(L, N), q.MField(L, N)
+    f = q.Field(L)
+    for r in range(N):
+        inp.set(r, f.load(orc.gaussian_spinor(L, 910 + r)))
+    want = {}
+    try:
+        for v in (64, 65, 128, 129, 256, 257, -1):
+            q.set_mrhs_variant(v)
+            for n in {1, 2, 3, N}:
+                if n <= N:
+                    q.dslash_mrhs(out, inp, g, 0.15, 0.02, nact=n)
+                    x = out.get(n - 1, f).store()
+                    assert np.array_equal(want.setdefault(n, x), x), (v, n)
+    finally:
+        q.set_mrhs_variant(-1)
+    for o in (g, inp, out, f):
         o.close()
