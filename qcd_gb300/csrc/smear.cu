@@ -296,9 +296,12 @@ __device__ __forceinline__ bool nonzero(const double2 v[3])
 // all 32 sites adds nothing, so its product is skipped. A point source fills
 // one spin of four, and the sites within k of it after k steps; dense spinors
 // take the same path and skip nothing. A 32^3 slice, 50 steps of a point
-// source: 115 us a step with one thread per site, in place; 19.6 us now (12 us
-// are the FP64 operations of one full spin, 228 a site; the rest is the launch
-// and one latency chain a step). One-warp blocks spread their work over the
+// source, twelve times: 72.9 ms with one thread per site, in place; 15.1 now (a
+// step is 25 us, 12 of them the FP64 operations of one full spin, 234 a site;
+// the rest is the launch and one latency chain). The six products of a site are
+// summed by direction, in chains of 12 multiply-adds: one chain of 36 takes 14.1
+// ms, but rounds more (3.8e-16 off the 64-bit result after 50 steps instead of
+// 2.1e-16; 2.5e-16 for separately summed products). One-warp blocks spread their work over the
 // SMs most evenly (128 threads, a warp per spin: 5 % slower); loading a hop's
 // link while the one before it is computed takes 168 registers and 8 % longer.
 constexpr int kGaussSites = 32;
@@ -324,17 +327,25 @@ __global__ void __launch_bounds__(kGaussSites) k_gauss3d(double2 *out, const dou
 #pragma unroll
   for (int k = 0; k < 3; k++) h[k] = C<double>{0.0, 0.0};
 #pragma unroll
-  for (int d = 0; d < 6; d++) {
-    if (!__any_sync(0xffffffffu, all || nonzero(p[d]))) continue;
-    const int mu = d >> 1, z = d & 1 ? bwd(geo, x, c, 1 + mu) : x;
+  for (int mu = 0; mu < 3; mu++) {
+    C<double> t[3];
 #pragma unroll
-    for (int b = 0; b < 3; b++) {
-      const C<double> w{p[d][b].x, p[d][b].y};
+    for (int k = 0; k < 3; k++) t[k] = C<double>{0.0, 0.0};
 #pragma unroll
-      for (int a = 0; a < 3; a++)
-        h[a] = d & 1 ? cmadd_conj(load_entry(u, stride, z, mu, 3 * b + a), w, h[a])
-                     : cmadd(load_entry(u, stride, x, mu, 3 * a + b), w, h[a]);
+    for (int d = 2 * mu; d < 2 * mu + 2; d++) {
+      if (!__any_sync(0xffffffffu, all || nonzero(p[d]))) continue;
+      const int z = d & 1 ? bwd(geo, x, c, 1 + mu) : x;
+#pragma unroll
+      for (int b = 0; b < 3; b++) {
+        const C<double> w{p[d][b].x, p[d][b].y};
+#pragma unroll
+        for (int a = 0; a < 3; a++)
+          t[a] = d & 1 ? cmadd_conj(load_entry(u, stride, z, mu, 3 * b + a), w, t[a])
+                       : cmadd(load_entry(u, stride, x, mu, 3 * a + b), w, t[a]);
+      }
     }
+#pragma unroll
+    for (int k = 0; k < 3; k++) h[k] = h[k] + t[k];
   }
   if (id >= V3) return;
 #pragma unroll
