@@ -859,7 +859,7 @@ def main():
     ap.add_argument("--mrhs-n", type=int, default=16, help="--only mrhs / batch: RHS per block / batch slots")
     ap.add_argument("--eo", action="store_true", help="--only batch: even/odd preconditioned batch")
     ap.add_argument("--mrhs-variant", type=int, default=-1,
-                    help="--only mrhs: -1 tuned, 1 tensor cores, 64/128/256 SIMT block size")
+                    help="--only mrhs: -1 by size, 1 tensor cores, 64/128/256 SIMT block size")
     ap.add_argument("--serve-sweep", default="0.5,1,2,4", help="--only serve: arrival rates (requests/s)")
     ap.add_argument("--only", choices=["f64", "df64", "f32", "f16", "mrhs", "batch", "solve", "serve"],
                     help="profiling target: time only this operator variant (a few launches under ncu)")

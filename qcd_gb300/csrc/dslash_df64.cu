@@ -15,8 +15,9 @@
 // neither contract nor reorder them. The double -> float-pair splits of the
 // spinors (four per hop and thread) and the widenings of the results use
 // integer bit operations, because the hardware conversions run on the FP64
-// pipe. The links come from a copy of the gauge field stored as float pairs, made once per field, with the boundary phase e^{i th/L}
-// multiplied into the links of twisted directions (U' h for the forward hop,
+// pipe. The links come from a copy of the gauge field stored as float pairs,
+// made once per field, with the boundary phase e^{i th/L} multiplied into the
+// links of twisted directions (U' h for the forward hop,
 // U'^+ h = e^{-i th/L} U^+ h for the backward one, as qcd_wilson.c applies it).
 // The result differs from FP64 by a few 2^-46 relative, within the 1e-13
 // per-site parity bar. Spinor values must lie in [2^-74, 2^127) in magnitude

@@ -4,11 +4,12 @@
 // (site, RHS), slot after slot in the layout of an FP16 field (mrhs.h).
 //
 // Operator: three kernels. SIMT, the one that runs unless another is asked
-// for: one thread per site and two slots, links shared through L1, its block
-// size picked per (volume, slot count) by timing. tcgen05: one FP16 GEMM per site with the eight hops concatenated along K
-// (see k_wilson_mrhs_tc). mma.sync (below): one warp per site. For each of
-// the eight hops the warp builds, for 16 RHS at a time, the matrix A (16 RHS x 12 reals of the
-// projected half spinor, padded to 16) and multiplies it with
+// for: one thread per site and one or two slots, links shared through L1, its
+// shape by a rule on the volume and the occupied slots (simt_shape). tcgen05:
+// one FP16 GEMM per site with the eight hops concatenated along K (see
+// k_wilson_mrhs_tc). mma.sync (below): one warp per site. For each of the eight
+// hops the warp builds, for 16 RHS at a time, the matrix A (16 RHS x 12 reals
+// of the projected half spinor, padded to 16) and multiplies it with
 //   B = realified ( R_mu (x) U_mu )   (12 x 24, padded to 16 x 24)
 // where U_mu is the link (or U^+ for backward hops, phase e^{+-i th/L}
 // folded in) and R_mu the 4 x 2 spin matrix that rebuilds the lower spinor
