@@ -289,70 +289,63 @@ __device__ __forceinline__ bool nonzero(const double2 v[3])
   return m != 0;
 }
 
-// out = (in + alpha H in) / (1 + 6 alpha) on a dense time-slice: a warp takes
-// one spin (blockIdx.y) of 32 sites; the step does not mix spins. Zeros are
-// left out while the links are finite: an empty spin stays empty (the host
-// clears it in both arrays), and a neighbour whose three colours are zero at
-// all 32 sites adds nothing, so its product is skipped. A point source fills
-// one spin of four, and the sites within k of it after k steps; dense spinors
-// take the same path and skip nothing. A 32^3 slice, 50 steps of a point
-// source, twelve times: 72.9 ms with one thread per site, in place; 15.1 now (a
-// step is 25 us, 12 of them the FP64 operations of one full spin, 234 a site;
-// the rest is the launch and one latency chain). The six products of a site are
-// summed by direction, in chains of 12 multiply-adds: one chain of 36 takes 14.1
-// ms, but rounds more (3.8e-16 off the 64-bit result after 50 steps instead of
-// 2.1e-16; 2.5e-16 for separately summed products). One-warp blocks spread their work over the
-// SMs most evenly (128 threads, a warp per spin: 5 % slower); loading a hop's
-// link while the one before it is computed takes 168 registers and 8 % longer.
+// out = (in + alpha H in) / (1 + 6 alpha) on a dense time-slice: a block takes
+// one spin (blockIdx.y) of 32 sites, one warp per direction, whose sums meet in
+// shared memory; the step does not mix spins. Zeros are left out while the
+// links are finite: an empty spin stays empty (the host clears it in both
+// arrays), and a neighbour whose three colours are zero at all 32 sites adds
+// nothing, so its product is skipped. A point source fills one spin of four,
+// and the sites within k of it after k steps; dense spinors take the same path
+// and skip nothing. Twelve point sources on a 32^3 slice, 50 steps: 72.9 ms with
+// one thread per site, in place; 15.0 with one warp per spin and 32 sites (its
+// six neighbours one latency chain after the other); 13.7 now (a step is 23 us,
+// 12 of them the FP64 operations of one full spin, 234 a site). The sum by
+// direction, chains of 12 multiply-adds, also rounds less than one chain of 36:
+// 2.1e-16 off the 64-bit result after 50 steps, 3.8e-16, and 2.5e-16 for
+// separately summed products.
 constexpr int kGaussSites = 32;
-__global__ void __launch_bounds__(kGaussSites) k_gauss3d(double2 *out, const double2 *in, const double2 *u,
-                                                         int64_t stride, Geom geo, int V3, double alpha, double nrm,
-                                                         const int *flag)
+__global__ void __launch_bounds__(3 * kGaussSites) k_gauss3d(double2 *out, const double2 *in, const double2 *u,
+                                                             int64_t stride, Geom geo, int V3, double alpha,
+                                                             double nrm, const int *flag)
 {
-  const int id = (int)(blockIdx.x * kGaussSites + threadIdx.x), sp = (int)blockIdx.y;
+  __shared__ double2 part[3][3][kGaussSites];  // [direction][colour][site]
+  const int lane = threadIdx.x, mu = threadIdx.y, id = (int)blockIdx.x * kGaussSites + lane, sp = (int)blockIdx.y;
   const bool all = flag[0] != 0 || !isfinite(alpha) || !isfinite(nrm);
-  if (!all && flag[1 + sp] == 0) return;
-  const int x = id < V3 ? id : V3 - 1;  // idle lanes repeat the last site
+  if (!all && flag[1 + sp] == 0) return;  // the whole block
+  const int x = id < V3 ? id : V3 - 1;    // idle lanes repeat the last site
   int c[4];
   coords(geo, x, c);
   const double2 *v = in + (int64_t)(3 * sp) * stride;
-  double2 p[6][3];
+  const int xf = fwd(geo, x, c, 1 + mu), xb = bwd(geo, x, c, 1 + mu);
+  double2 p[2][3];
 #pragma unroll
-  for (int d = 0; d < 6; d++) {
-    const int y = d & 1 ? bwd(geo, x, c, 1 + (d >> 1)) : fwd(geo, x, c, 1 + (d >> 1));
-#pragma unroll
-    for (int b = 0; b < 3; b++) p[d][b] = v[b * stride + y];
+  for (int b = 0; b < 3; b++) {
+    p[0][b] = v[b * stride + xf];
+    p[1][b] = v[b * stride + xb];
   }
-  C<double> h[3];
+  const double2 w0 = v[mu * stride + x];
+  C<double> t[3];
 #pragma unroll
-  for (int k = 0; k < 3; k++) h[k] = C<double>{0.0, 0.0};
+  for (int k = 0; k < 3; k++) t[k] = C<double>{0.0, 0.0};
 #pragma unroll
-  for (int mu = 0; mu < 3; mu++) {
-    C<double> t[3];
+  for (int d = 0; d < 2; d++) {
+    if (!__any_sync(0xffffffffu, all || nonzero(p[d]))) continue;
 #pragma unroll
-    for (int k = 0; k < 3; k++) t[k] = C<double>{0.0, 0.0};
+    for (int b = 0; b < 3; b++) {
+      const C<double> w{p[d][b].x, p[d][b].y};
 #pragma unroll
-    for (int d = 2 * mu; d < 2 * mu + 2; d++) {
-      if (!__any_sync(0xffffffffu, all || nonzero(p[d]))) continue;
-      const int z = d & 1 ? bwd(geo, x, c, 1 + mu) : x;
-#pragma unroll
-      for (int b = 0; b < 3; b++) {
-        const C<double> w{p[d][b].x, p[d][b].y};
-#pragma unroll
-        for (int a = 0; a < 3; a++)
-          t[a] = d & 1 ? cmadd_conj(load_entry(u, stride, z, mu, 3 * b + a), w, t[a])
-                       : cmadd(load_entry(u, stride, x, mu, 3 * a + b), w, t[a]);
-      }
+      for (int a = 0; a < 3; a++)
+        t[a] = d ? cmadd_conj(load_entry(u, stride, xb, mu, 3 * b + a), w, t[a])
+                 : cmadd(load_entry(u, stride, x, mu, 3 * a + b), w, t[a]);
     }
-#pragma unroll
-    for (int k = 0; k < 3; k++) h[k] = h[k] + t[k];
   }
+#pragma unroll
+  for (int k = 0; k < 3; k++) part[mu][k][lane] = make_double2(t[k].re, t[k].im);
+  __syncthreads();
   if (id >= V3) return;
-#pragma unroll
-  for (int k = 0; k < 3; k++) {
-    const double2 w = v[k * stride + x];
-    out[(int64_t)(3 * sp + k) * stride + x] = make_double2((w.x + alpha * h[k].re) * nrm, (w.y + alpha * h[k].im) * nrm);
-  }
+  const double2 a = part[0][mu][lane], b = part[1][mu][lane], d = part[2][mu][lane];
+  out[(int64_t)(3 * sp + mu) * stride + x] =
+      make_double2((w0.x + alpha * (a.x + b.x + d.x)) * nrm, (w0.y + alpha * (a.y + b.y + d.y)) * nrm);
 }
 
 static Geom make_geom(const int L[4])
@@ -436,7 +429,7 @@ static bool smear_slice(qcdgpu_field v, qcdgpu_gauge g, double ape_alpha, int ap
   const double nrm = 1.0 / (1.0 + 6.0 * alpha);
   const dim3 ng((unsigned)((V3 + kGaussSites - 1) / kGaussSites), 4);
   for (int i = 0; ok && i < n; i++) {
-    k_gauss3d<<<ng, kGaussSites, 0, st>>>(b, a, u, S, geo, V3, alpha, nrm, flag);
+    k_gauss3d<<<ng, dim3(kGaussSites, 3), 0, st>>>(b, a, u, S, geo, V3, alpha, nrm, flag);
     ok = QG_LAUNCHED("gauss3d");
     double2 *tmp = a;
     a = b;
