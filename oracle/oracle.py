@@ -40,11 +40,11 @@ _ip = np.ctypeslib.ndpointer(dtype=np.int32, flags="C_CONTIGUOUS")
 
 def build(with_ref: bool | None = None, ref_tree: str | None = None) -> None:
     """Compile the restatement and, when a reference source tree is given
-    (``ref_tree`` or $QCD_REFERENCE_TREE) and exists, the reference."""
+    (``ref_tree`` or $QCD_REFERENCE_TREE) and holds the sources, the reference."""
     subprocess.run(["make", "-s", "-C", HERE, "all"], check=True)
     ref_tree = ref_tree or os.environ.get(REF_TREE_ENV)
     if with_ref is None:
-        with_ref = bool(ref_tree) and os.path.isdir(ref_tree)
+        with_ref = bool(ref_tree) and os.path.isdir(os.path.join(ref_tree, "lib", "src"))
     if with_ref:
         if not ref_tree:
             raise RuntimeError(f"building the reference needs its source tree (${REF_TREE_ENV})")
