@@ -255,21 +255,14 @@ bool twop_proton(const qcdgpu_field *up, const qcdgpu_field *dn, const int xsrc[
   geo.st[2] = f0->L[0] * f0->L[1];
   geo.st[3] = f0->L[0] * f0->L[1] * f0->L[2];
   const int nt = t1 - t0 + 1, V3 = f0->L[1] * f0->L[2] * f0->L[3];
-  // block, corr, the phase tables and the momenta in one work field of the
-  // propagators' lattice, or (more momenta than it holds) in memory of their own
+  // block, corr, the phase tables and the momenta
   const size_t nb = (size_t)nt * V3, nc = (size_t)nt * nmom;
   const size_t np = (size_t)nmom * (f0->L[1] + (size_t)f0->L[2] * f0->L[3]);
   const size_t need = sizeof(double2) * (nb + nc + np) + sizeof(int) * 3 * (size_t)nmom;
   cudaStream_t st = stream();
-  qcdgpu_field w = nullptr;
-  void *own = nullptr;
-  if (need <= f0->bytes) {
-    w = work_get(f0->L, QCDGPU_F64);
-    if (!w) return false;
-  } else if (!QG_CUDA(cudaMalloc(&own, need))) {
-    return false;
-  }
-  double2 *block = (double2 *)(w ? w->data : own), *dcorr = block + nb, *ph = dcorr + nc;
+  Scratch w(need);
+  if (!w.data) return false;
+  double2 *block = (double2 *)w.data, *dcorr = block + nb, *ph = dcorr + nc;
   int *dmom = (int *)(ph + np);
   bool ok = QG_CUDA(cudaMemcpyAsync(dmom, mom, sizeof(int) * 3 * (size_t)nmom, cudaMemcpyHostToDevice, st)) &&
             QG_CUDA(cudaFuncSetAttribute(k_twop_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTwShared));
@@ -287,10 +280,7 @@ bool twop_proton(const qcdgpu_field *up, const qcdgpu_field *dn, const int xsrc[
     ok = QG_LAUNCHED("twop_ft") &&
          QG_CUDA(cudaMemcpyAsync(corr, dcorr, sizeof(double2) * nc, cudaMemcpyDeviceToHost, st));
   }
-  ok = QG_CUDA(cudaStreamSynchronize(st)) && ok;
-  work_put(w);
-  cudaFree(own);
-  return ok;
+  return QG_CUDA(cudaStreamSynchronize(st)) && ok;
 }
 
 }  // namespace qg

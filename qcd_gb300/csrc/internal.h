@@ -113,10 +113,26 @@ qcdgpu_gauge gauge_new(const int L[4], const double theta[4], int prec, int reco
 void gauge_free(qcdgpu_gauge g);
 bool same_shape(qcdgpu_field a, qcdgpu_field b);
 
-// pooled work fields (runtime.cu): returned fields are zero-free garbage
+// pooled work fields (runtime.cu): their sites hold anything, their padding
+// zeros, as any field's: a call that wants raw memory takes a Scratch
 qcdgpu_field work_get(const int L[4], int prec);
 void work_put(qcdgpu_field f);
-void work_trim();  // frees the pooled fields
+void work_trim();  // frees the pooled fields and the scratch memory
+
+// Raw device memory for the duration of a call (runtime.cu; data null: none to
+// be had). Taken and given back in the order of the current stream, so that
+// work still queued on it when the call returns keeps its memory, whatever
+// stream the next call runs on.
+struct Scratch {
+  void *data = nullptr;
+  explicit Scratch(size_t bytes);
+  ~Scratch();
+  Scratch(const Scratch &) = delete;
+  Scratch &operator=(const Scratch &) = delete;
+
+ private:
+  cudaStream_t st;
+};
 
 // scratch for reductions: 2 * kMaxPartials doubles + result slots
 constexpr int kMaxPartials = 2048;

@@ -217,12 +217,74 @@ void work_put(qcdgpu_field f)
   g_pool.push_back(f);
 }
 
+// -------------------------------------------------------- call scratch
+// One stream-ordered memory pool per device. It keeps up to kScratchKeep bytes
+// between calls, so that a repeated call maps no memory anew; what a call takes
+// beyond that goes back at the stream's next synchronisation.
+constexpr uint64_t kScratchKeep = 256ull << 20;
+constexpr int kMaxDevices = 64;
+static std::mutex g_mempool_mu;
+static cudaMemPool_t g_mempool[kMaxDevices];
+
+static cudaMemPool_t scratch_pool()
+{
+  int dev = -1;
+  if (!QG_CUDA(cudaGetDevice(&dev))) return nullptr;
+  if (dev < 0 || dev >= kMaxDevices) {
+    set_error("device ordinal %d out of range", dev);
+    return nullptr;
+  }
+  std::lock_guard<std::mutex> lk(g_mempool_mu);
+  if (!g_mempool[dev]) {
+    cudaMemPoolProps p = {};
+    p.allocType = cudaMemAllocationTypePinned;
+    p.location.type = cudaMemLocationTypeDevice;
+    p.location.id = dev;
+    cudaMemPool_t m = nullptr;
+    uint64_t keep = kScratchKeep;
+    if (!QG_CUDA(cudaMemPoolCreate(&m, &p))) return nullptr;
+    if (!QG_CUDA(cudaMemPoolSetAttribute(m, cudaMemPoolAttrReleaseThreshold, &keep))) {
+      cudaMemPoolDestroy(m);
+      return nullptr;
+    }
+    g_mempool[dev] = m;
+  }
+  return g_mempool[dev];
+}
+
+Scratch::Scratch(size_t bytes) : st(g_stream)
+{
+  if (alloc_fault()) {
+    set_error("out of device memory (injected) for %zu bytes of scratch", bytes);
+    return;
+  }
+  cudaMemPool_t m = scratch_pool();
+  if (!m) return;
+  cudaError_t e = cudaMallocFromPoolAsync(&data, bytes, m, st);
+  if (e == cudaErrorMemoryAllocation) {  // give back what the pools hold and retry once
+    cudaGetLastError();
+    work_trim();
+    e = cudaMallocFromPoolAsync(&data, bytes, m, st);
+  }
+  if (!QG_CUDA(e)) data = nullptr;
+}
+
+Scratch::~Scratch()
+{
+  if (data) QG_CUDA(cudaFreeAsync(data, st));
+}
+
 void work_trim()
 {
-  std::lock_guard<std::mutex> lk(g_pool_mu);
-  if (!g_pool.empty()) cudaStreamSynchronize(g_stream);
-  for (qcdgpu_field f : g_pool) field_free(f);
-  g_pool.clear();
+  {
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    if (!g_pool.empty()) cudaStreamSynchronize(g_stream);
+    for (qcdgpu_field f : g_pool) field_free(f);
+    g_pool.clear();
+  }
+  std::lock_guard<std::mutex> lk(g_mempool_mu);
+  for (cudaMemPool_t m : g_mempool)
+    if (m) cudaMemPoolTrimTo(m, 0);  // what queued work still holds stays
 }
 
 // ------------------------------------------------------- reduction scratch

@@ -1,0 +1,51 @@
+"""GCR's passes over whole fields, after calls that used the library's memory
+before it, on lattices whose component blocks are padded (a volume that is no
+multiple of 128). Against the oracle, 1e-11 as in test_solvers_gpu.py."""
+import numpy as np
+import pytest
+
+import qcd_gb300 as q
+from tests.conftest import EPS_PLAQ_060
+from tests.golden.make_golden import twop_inputs
+
+pytestmark = pytest.mark.gpu
+TH = (np.pi, 0.0, 0.0, 0.0)
+
+
+class Gcr:
+    """gcr() and the oracle's on one lattice"""
+
+    def __init__(self, orc, L, seed=71):
+        self.orc, self.L = orc, L
+        self.u, self.b = orc.gauge_synthetic(L, seed, EPS_PLAQ_060), orc.gaussian_spinor(L, seed + 1)
+        self.geo = q.Geometry(L, TH)
+        self.g, self.src, self.sol = q.GaugeField(self.geo), q.Vector(self.geo), q.Vector(self.geo)
+        self.g.a[:] = self.u
+
+    def run(self, src, sol, n):
+        return q.lib().gcr(sol.ref, src.ref, self.g.ref, 0.15, 0.02, n, self.geo.s)
+
+    def check(self, n, src=None, sol=None):
+        src, sol = src or self.src, sol or self.sol
+        src.a[:] = self.b
+        assert self.run(src, sol, n) == 0
+        ref, rc = self.orc.gcr(self.b, self.u, self.L, TH, 0.15, 0.02, n, fixed=True)
+        assert rc == 0
+        assert np.max(np.abs(sol.a - ref)) <= 1e-11 * np.max(np.abs(ref))
+
+    def close(self):
+        for o in (self.src, self.sol, self.g, self.geo):
+            o.close()
+
+
+def test_gcr_after_a_contraction(gpu, orc):
+    L = (3, 5, 4, 7)
+    _, cu, cd, _ = twop_inputs(orc, L, 51)
+    fu, fd = [q.Field(L).load(c) for c in cu], [q.Field(L).load(c) for c in cd]
+    s = Gcr(orc, L)
+    q.release_work()
+    q.twop_proton(fu, fd, (1, 2, 0, 4), 0, L[0] - 1, [(-1, -1, k - 3) for k in range(7)])
+    s.check(9)
+    s.close()
+    for f in fu + fd:
+        f.close()
