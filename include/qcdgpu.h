@@ -417,9 +417,9 @@ enum {
 int qcdgpu_solve(qcdgpu_field x, qcdgpu_field b, qcdgpu_gauge g, double kappa, double mu,
                  qcdgpu_solve_params *p);
 
-/* Solvers keep their work fields in a pool between calls, contractions up to
- * 256 MB of scratch memory; this frees both (the next call allocates again).
- * Returns 0. */
+/* Solvers keep their work fields in a pool between calls, contractions and
+ * smearings up to 256 MB of scratch memory; this frees both (the next call
+ * allocates again). Returns 0. */
 int qcdgpu_release_work(void);
 /* Fault injection for tests (no reference counterpart): the next n
  * allocations of host vectors and gauge fields (qcd_initVector,

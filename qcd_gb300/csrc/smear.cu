@@ -393,14 +393,11 @@ static bool smear_slice(qcdgpu_field v, qcdgpu_gauge g, double ape_alpha, int ap
   const int V3 = (int)(v->V / v->L[0]);
   const int64_t S = pad_stride(V3);
   // dense copies: two of the spinor's 12 blocks, one or two of the 27 link
-  // blocks, and the flags, in a work field with as many time-slices as that takes
+  // blocks, and the flags
   const int64_t blocks = 24 + (ape_n > 0 ? 54 : 27);
-  int Lw[4] = {2, v->L[1], v->L[2], v->L[3]};
-  const int64_t lt = (blocks * S + 2 + 12ll * V3 - 1) / (12ll * V3);
-  if (lt > Lw[0]) Lw[0] = (int)lt;
-  qcdgpu_field w = work_get(Lw, QCDGPU_F64);
-  if (!w) return false;
-  double2 *a = (double2 *)w->data, *b = a + 12 * S, *u = b + 12 * S, *u2 = u + 27 * S;
+  Scratch w(sizeof(double2) * (size_t)(blocks * S) + 5 * sizeof(int));
+  if (!w.data) return false;
+  double2 *a = (double2 *)w.data, *b = a + 12 * S, *u = b + 12 * S, *u2 = u + 27 * S;
   int *flag = (int *)(a + blocks * S);
   cudaStream_t st = stream();
   Geom geo = make_geom(v->L);
@@ -439,7 +436,6 @@ static bool smear_slice(qcdgpu_field v, qcdgpu_gauge g, double ape_alpha, int ap
     k_slice_put<<<dim3(nb, 12), 128, 0, st>>>((double2 *)v->data, v->stride, a, S, V3, t, v->L[0]);
     ok = QG_LAUNCHED("slice_put");
   }
-  work_put(w);
   return ok;
 }
 
