@@ -51,7 +51,7 @@ def test_gcr_after_a_contraction(gpu, orc):
         f.close()
 
 
-@pytest.mark.parametrize("ape_n,Ls,L", [(2, (5, 6, 6, 6), (8, 6, 6, 6)), (0, (4, 3, 5, 3), (13, 3, 5, 3))])
+@pytest.mark.parametrize("ape_n,Ls,L", [(2, (5, 6, 6, 6), (8, 6, 6, 6)), (0, (4, 3, 4, 3), (16, 3, 4, 3))])
 def test_gcr_after_a_smeared_source(gpu, orc, ape_n, Ls, L):
     """L: the lattice of as many time-slices as the smearing's copies of a slice of Ls take"""
     g, f = q.Gauge(Ls, TH).load(orc.gauge_synthetic(Ls, 73, EPS_PLAQ_060)), q.Field(Ls)
