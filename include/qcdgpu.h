@@ -457,7 +457,9 @@ int qcdgpu_dot_noalloc(const double *a, const double *b, int64_t n, double *resu
  * != in); n Gaussian steps of v on time-slice t; and the smeared point source
  * of the 24^3 x 48 workload: a unit point at x (t, x, y, z), spin, colour,
  * Gaussian-smeared gauss_n times with gauss_alpha on links APE-smeared ape_n
- * times with ape_alpha (on time-slice x[0]). Return 0, or 1 on error. */
+ * times with ape_alpha (on time-slice x[0]). Links of two or more APE steps and
+ * sources with ape_n > 0 are there when the call returns; otherwise the work is
+ * queued on the current stream. Return 0, or 1 on error. */
 /* LIME files straight into / out of device fields (byte order and site
  * order converted on the GPU); source != 0 writes an ETMC source file */
 int qcdgpu_gauge_load_lime(qcdgpu_gauge g, const char *fname);

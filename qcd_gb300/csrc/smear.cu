@@ -493,7 +493,10 @@ int qcdgpu_smeared_source(qcdgpu_field f, qcdgpu_gauge g, const int x[4], int sp
   if (gauss_n == 0) return 0;
   // the Gaussian steps read the links of the source's time-slice only, and
   // the APE steps do not couple time-slices: only that slice is smeared
-  return qg::smear_slice(f, g, ape_alpha, ape_n, gauss_alpha, x[0], gauss_n) ? 0 : 1;
+  const bool ok = qg::smear_slice(f, g, ape_alpha, ape_n, gauss_alpha, x[0], gauss_n);
+  // with APE steps the call ends when the source is there, for callers that
+  // go on on another stream
+  return (ape_n <= 0 || QG_CUDA(cudaStreamSynchronize(qg::stream()))) && ok ? 0 : 1;
 }
 
 }  // extern "C"

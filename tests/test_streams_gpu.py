@@ -1,0 +1,63 @@
+"""Calls on one stream after the other: each result is the one of the calls
+apart, bit for bit (the kernels sum in a fixed order)."""
+import contextlib
+
+import numpy as np
+import pytest
+
+import qcd_gb300 as q
+from tests.conftest import EPS_PLAQ_060
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+TH = (np.pi, 0.0, 0.0, 0.0)
+
+
+@contextlib.contextmanager
+def on_stream(s):
+    q.set_stream(s.cuda_stream)
+    try:
+        yield
+    finally:
+        q.set_stream(None)
+
+
+def two_streams():
+    torch.cuda.synchronize()
+    return torch.cuda.Stream(), torch.cuda.Stream()
+
+
+def test_smeared_source_is_there_when_the_call_returns(gpu):
+    L = (2, 24, 24, 24)
+    g, f = q.Gauge(L, TH).synthetic(81, EPS_PLAQ_060), q.Field(L)
+    args = ((1, 3, 4, 5), 2, 1, 0.5, 4, 4.0, 100)
+    q.smeared_source(f, g, *args)
+    ref = f.store()
+    f.load(np.zeros_like(ref))
+    a, b = two_streams()
+    with on_stream(a):
+        q.smeared_source(f, g, *args)
+    with on_stream(b):
+        out = f.store()
+    assert np.array_equal(out, ref)
+    f.close()
+    g.close()
+
+
+def test_gauss3d_on_two_streams(gpu):
+    L = (2, 24, 24, 24)
+    g = q.Gauge(L, TH).synthetic(82, EPS_PLAQ_060)
+    fs, ref = [q.Field(L) for _ in range(2)], []
+    for k, f in enumerate(fs):
+        q.gauss3d(f.gaussian(83 + k), g, 4.0, k, 100)
+        ref.append(f.store())
+        f.gaussian(83 + k)
+    streams = two_streams()
+    for k, s in enumerate(streams):
+        with on_stream(s):
+            q.gauss3d(fs[k], g, 4.0, k, 100)
+    torch.cuda.synchronize()
+    for f, r in zip(fs, ref):
+        assert np.array_equal(f.store(), r)
+        f.close()
+    g.close()
