@@ -174,6 +174,8 @@ int gcr_dropin(qcdgpu_field sol, qcdgpu_field src, qcdgpu_gauge g, double mp4, d
   if (!blas_zero(sol) || !QG_CUDA(cudaMemcpyAsync(coef, sol_coef.data(), sizeof(cplx) * n, cudaMemcpyHostToDevice, st)) ||
       !gs_update(sol, res.data(), coef, n, nullptr, scratch, nullptr, nullptr))
     return 1;
+  // the scalars' buffer and the pooled fields are the next call's, whatever its stream
+  if (!QG_CUDA(cudaStreamSynchronize(st))) return 1;
   if (sick) {
     set_error("gcr: Krylov space is sick (NaN norm)");
     return 1;

@@ -61,3 +61,39 @@ def test_gauss3d_on_two_streams(gpu):
         assert np.array_equal(f.store(), r)
         f.close()
     g.close()
+
+
+def test_gcr_on_two_streams(gpu, orc):
+    """on resident vectors no copy to the host makes the caller wait"""
+    L = (16, 12, 12, 12)
+    geo = q.Geometry(L, TH)
+    g = q.GaugeField(geo)
+    g.a[:] = orc.gauge_synthetic(L, 85, EPS_PLAQ_060)
+    lib = q.lib()
+    assert lib.qcdgpu_gauge_upload(g.ref) == 0
+    src, sol = [q.Vector(geo) for _ in range(2)], [q.Vector(geo) for _ in range(2)]
+    for k in range(2):
+        src[k].a[:] = orc.gaussian_spinor(L, 86 + k)
+        for v in (src[k], sol[k]):
+            assert lib.qcdgpu_vector_make_resident(v.ref) == 0
+
+    def gcr(k):
+        assert lib.gcr(sol[k].ref, src[k].ref, g.ref, 0.15, 0.02, 17, geo.s) == 0
+
+    def result(k):
+        assert lib.qcdgpu_vector_to_host(sol[k].ref) == 0
+        return sol[k].a.copy()
+
+    ref = []
+    for k in range(2):
+        gcr(k)
+        ref.append(result(k))
+    streams = two_streams()
+    for k, s in enumerate(streams):
+        with on_stream(s):
+            gcr(k)
+    torch.cuda.synchronize()
+    for k in range(2):
+        assert np.array_equal(result(k), ref[k])
+    for o in (*src, *sol, g, geo):
+        o.close()
