@@ -138,12 +138,17 @@ __global__ void __launch_bounds__(4 * kTwSites, 3) k_twop_block(Props p, Geom ge
     // C g5 and bar C g5: entry (mu, mu ^ 1) = +1 for even mu, -1 for odd; the
     // other sign for ku
     const bool neg = ((mu ^ ku) & 1) == 0;
+    // a sum for each ku, then their sum: one chain of all four rounds more
+    // (3.4e-16 off 113 bits in the root mean square, against 2.6e-16 and 2.9e-16
+    // for the written-out sum)
+    C<double> sum{0.0, 0.0};
 #pragma unroll
     for (int k = 0; k < 9; k++) {
       C<double> d = pr(p.d, p.stride, v, mu ^ 1, ku ^ 1, k / 3, k % 3);
       if (neg) d = -d;
-      acc = cmadd(E[k], d, acc);
+      sum = cmadd(E[k], d, sum);
     }
+    acc = acc + sum;
   }
   __syncthreads();  // X is read no more
   X[mu * kTwSites + lane] = make_double2(acc.re, acc.im);
@@ -196,13 +201,21 @@ __global__ void __launch_bounds__(kFtThreads) k_twop_ft(const double2 *block, Ge
   C<double> sum{0.0, 0.0};
   if (ty < ny)
     for (int x = tx; x < Lx; x += nx) {
-      C<double> a{0.0, 0.0};
-#pragma unroll 4
-      for (int r = ty; r < rows; r += ny) {
-        const double2 b = b0[(int64_t)r * Lx + x], e = eyz[r];
-        a = cmadd(C<double>{b.x, b.y}, C<double>{e.x, e.y}, a);
+      // four partial sums: 58 rows in one chain round to 5.4e-16 at 24^3 sites
+      // (root mean square against 113 bits), so split to 4.3e-16
+      C<double> a[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) a[k] = C<double>{0.0, 0.0};
+      for (int r0 = ty; r0 < rows; r0 += 4 * ny) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          const int r = r0 + k * ny;
+          if (r >= rows) continue;
+          const double2 b = b0[(int64_t)r * Lx + x], e = eyz[r];
+          a[k] = cmadd(C<double>{b.x, b.y}, C<double>{e.x, e.y}, a[k]);
+        }
       }
-      sum = cmadd(a, C<double>{ex[x].x, ex[x].y}, sum);
+      sum = cmadd((a[0] + a[1]) + (a[2] + a[3]), C<double>{ex[x].x, ex[x].y}, sum);
     }
   __shared__ double sr[kFtThreads], si[kFtThreads];
   sr[threadIdx.x] = sum.re;
