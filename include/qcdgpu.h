@@ -507,8 +507,9 @@ int qcdgpu_dslash_mrhs(qcdgpu_mfield out, qcdgpu_mfield in, qcdgpu_gauge g, doub
  * (+1: two slots per thread) the SIMT kernel with that block size. */
 int qcdgpu_set_mrhs_variant(int variant);
 /* the choice for (L, nrhs) with all slots occupied: variant 0 SIMT / 1 mma.sync /
- * 2 tcgen05 and the SIMT block size (+1: two slots per thread); returns 1 before
- * the first apply of that shape */
+ * 2 tcgen05 and the SIMT block size, rounded up to a value that
+ * qcdgpu_set_mrhs_variant takes (+1: two slots per thread); returns 1 before the
+ * first apply of that shape */
 int qcdgpu_mrhs_tuned(const int L[4], int nrhs, int *variant, int *threads);
 /* Every wait of the tcgen05 kernel for its MMAs is bounded. A wait that runs
  * out makes the launch abandon its work (its output is invalid) and sets a

@@ -1346,7 +1346,8 @@ static MrhsTune mrhs_choice(const MArgs &a)
   std::lock_guard<std::mutex> lk(g_mrhs_mu);
   if (g_mrhs_tuned.find(key) == g_mrhs_tuned.end()) {
     const SimtShape sh = simt_shape(a.V, a.N, t);
-    g_mrhs_tuned[key] = MrhsTune{MRHS_SIMT, 32 * sh.warps, sh.slots};
+    // the block size as qcdgpu_set_mrhs_variant takes it
+    g_mrhs_tuned[key] = MrhsTune{MRHS_SIMT, sh.warps <= 2 ? 64 : sh.warps <= 4 ? 128 : 256, sh.slots};
   }
   return t;
 }
