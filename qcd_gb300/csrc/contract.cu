@@ -27,9 +27,6 @@
 // multiply-adds, against 18,432 products of three factors in the written-out
 // sum (115 ms at 24^3 x 48 in that form; the FP64 floor of this one is 8 ms).
 #include <math.h>
-#include <string.h>
-
-#include <vector>
 
 #include "dslash_args.h"
 

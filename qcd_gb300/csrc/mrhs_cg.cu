@@ -409,8 +409,8 @@ static qcdgpu_batch batch_new(qcdgpu_gauge g, int cap, bool eo)
   unsigned nb = mgrid(b->Vs, 1).x;
   if (mrhs_max_blocks(b->Vs, cap) > nb) nb = mrhs_max_blocks(b->Vs, cap);
   ok = ok && QG_CUDA(cudaMalloc(&b->xs, (size_t)12 * pad_stride(b->Vs) * cap * sizeof(float2))) &&
-            QG_CUDA(cudaMalloc(&b->s, ns * sizeof(double))) && QG_CUDA(cudaMalloc(&b->mp4s, (cap + 1) * sizeof(float))) &&
-            QG_CUDA(cudaMalloc(&b->tms, (cap + 1) * sizeof(float))) &&
+            QG_CUDA(cudaMalloc(&b->s, ns * sizeof(double))) && QG_CUDA(cudaMalloc(&b->mp4s, cap * sizeof(float))) &&
+            QG_CUDA(cudaMalloc(&b->tms, cap * sizeof(float))) &&
             QG_CUDA(cudaMalloc(&b->part, (size_t)nb * cap * sizeof(double))) &&
             QG_CUDA(cudaMalloc(&b->l1, (size_t)kMSGroups * cap * sizeof(double) + 256)) &&
             QG_CUDA(cudaMalloc(&b->rudev, (size_t)4 * cap * sizeof(double))) &&

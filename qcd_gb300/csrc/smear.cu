@@ -26,14 +26,6 @@
 
 namespace qg {
 
-__device__ __forceinline__ void m3dag(const C<double> a[9], C<double> r[9])
-{
-#pragma unroll
-  for (int i = 0; i < 3; i++)
-#pragma unroll
-    for (int j = 0; j < 3; j++) r[3 * i + j] = conj(a[3 * j + i]);
-}
-
 __device__ __forceinline__ C<double> m3det(const C<double> m[9])
 {
   C<double> d = m[0] * (m[4] * m[8] - m[5] * m[7]);
