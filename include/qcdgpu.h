@@ -313,7 +313,7 @@ int qcdgpu_sync(void);
 void qcdgpu_set_gcr_compat(int shipped);
 /* arithmetic of the FP64 operator used by the qcd.h entry points, the FP64
  * solvers and qcdgpu_dslash with arith < 0. Default QCDGPU_ARITH_DF64:
- * float-float on the FP32 pipes, 3.6x the native rate on GB300 at the same
+ * float-float on the FP32 pipes, 4.3x the native rate on GB300 at the same
  * per-site parity (<= 1e-13); |x| below 2^-1022 counts as zero there.
  * QCDGPU_ARITH_F64 selects native IEEE double. */
 int qcdgpu_set_f64_arith(int arith);

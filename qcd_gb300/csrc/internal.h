@@ -17,7 +17,8 @@
 //                in blocks of 32 sites (gword below)
 //
 // A block has `stride` elements, stride = V rounded up to a multiple of 128;
-// the padding sites hold zeros so whole-buffer reductions are exact.
+// the padding sites hold zeros, so that a caller's reductions over the whole
+// storage are exact; no sum of the library's reads them.
 #pragma once
 
 #include <cuda_runtime.h>

@@ -119,8 +119,10 @@ __device__ __forceinline__ void polar_step(C<double> M[9], C<double> d, double i
 // each, against 113 bits). i1^3 / (27 i3) is 1 for equal singular values and
 // 1.02 at kappa = 1.3; links beyond that take one or two steps of polar_step
 // first (kappa 3 -> 1.2, 10 -> at most 1.9), about 350 operations each where any
-// of a warp's 32 links needs it. Then the error is 0.90 to 1.02 times the
-// iteration's for smooth, rough and random links and for kappa = 1.2 to 20.
+// of a warp's 32 links needs it (a smeared source at 24^3 x 48, whose links are
+// beyond in the first APE steps only: 2.98 -> 3.05 ms). Then the error is 0.90 to
+// 1.02 times the iteration's for smooth, rough and random links and for kappa =
+// 1.2 to 20.
 // Links with i1^3 > 135 i3 (from kappa = 8.4 to 15.6 on, by the middle singular
 // value), those still beyond after two steps and those whose root has not
 // settled (out of FP32's range, singular, not finite) take the iteration.

@@ -202,9 +202,12 @@ __device__ __forceinline__ void hop_pair(const DArgs &a, int x, const int c[4], 
 //
 // FP32 / FP16 storage: registers capped for seven blocks per SM (72; 80
 // uncapped; FP16 alone eight, 64). Measured at 24^3 x 48, uncapped against seven
-// blocks: FP16 48.9 -> 47.1 us, FP32 57.3 -> 55.3 us per apply; at 32^3 x 64,
-// seven against eight: FP16 133.3 -> 131.9 us, FP32 loses. The even/odd kernel
-// below keeps the uncapped form, which solves 0.7 % faster.
+// blocks, before the modes were compiled apart: FP16 48.9 -> 47.1 us, FP32 57.3
+// -> 55.3 us per apply. Seven against eight, FP16 alone: 8^3 x 16 and 16^3 x 32
+// the same (6.15 and 12.3 us), 24^3 x 48 46.6 -> 45.9, 45 x 31 x 29 x 33 86.0 ->
+// 85.2, 32^3 x 64 130.2 -> 129.0, 48^3 x 96 644.1 -> 632.5 us; FP32 loses at
+// 32^3 x 64. The even/odd kernel below keeps the uncapped form, which solves
+// 0.7 % faster.
 template <bool DAG, int SP, int RECON, typename R, int MODE>
 __global__ void __launch_bounds__(128, SP == QCDGPU_F64 ? 1 : SP == QCDGPU_F16 && MODE == 0 ? 8 : 7) k_wilson(const DArgs a)
 {
