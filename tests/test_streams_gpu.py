@@ -97,3 +97,29 @@ def test_gcr_on_two_streams(gpu, orc):
         assert np.array_equal(result(k), ref[k])
     for o in (*src, *sol, g, geo):
         o.close()
+
+
+def test_gauss3d_under_capture(gpu):
+    """a recorded smearing, replayed beside a smearing on another stream"""
+    L = (2, 12, 12, 12)
+    g = q.Gauge(L, TH).synthetic(89, EPS_PLAQ_060)
+    f, other = q.Field(L).gaussian(90), q.Field(L).gaussian(91)
+    q.gauss3d(f, g, 4.0, 1, 6)
+    ref = f.store()
+    f.gaussian(90)
+    a, b = two_streams()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=a), on_stream(a):
+        q.gauss3d(f, g, 4.0, 1, 6)
+    for _ in range(2):
+        f.gaussian(90)
+        torch.cuda.synchronize()
+        with torch.cuda.stream(a):
+            graph.replay()
+        with on_stream(b):
+            q.gauss3d(other, g, 4.0, 1, 20)
+        torch.cuda.synchronize()
+        assert np.array_equal(f.store(), ref)
+    del graph
+    for o in (f, other, g):
+        o.close()
