@@ -423,8 +423,8 @@ int qcdgpu_solve(qcdgpu_field x, qcdgpu_field b, qcdgpu_gauge g, double kappa, d
 int qcdgpu_release_work(void);
 /* Fault injection for tests (no reference counterpart): the next n
  * allocations of host vectors and gauge fields (qcd_initVector,
- * qcd_initGaugeField) and of device fields and gauge fields fail as if memory
- * were exhausted, so that callers' out-of-memory paths run without
+ * qcd_initGaugeField), of device fields and gauge fields and of a call's scratch
+ * memory fail as if memory were exhausted, so that callers' out-of-memory paths run without
  * exhausting memory; n = 0 switches it off. */
 int qcdgpu_inject_alloc_failures(int n);
 /* Device bytes held by the lazily allocated partial-sum scratch of the

@@ -28,7 +28,7 @@ void set_error(const char *fmt, ...)
 }
 
 // fault injection (tests): the next g_alloc_faults allocations of fields,
-// gauge fields and host vectors fail as if memory were exhausted
+// gauge fields, host vectors and scratch fail as if memory were exhausted
 static std::atomic<int> g_alloc_faults{0};
 
 bool alloc_fault()
