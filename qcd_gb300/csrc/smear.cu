@@ -120,7 +120,7 @@ __device__ __forceinline__ void polar_step(C<double> M[9], C<double> d, double i
 // 1.02 at kappa = 1.3; links beyond that take one or two steps of polar_step
 // first (kappa 3 -> 1.2, 10 -> at most 1.9), about 350 operations each where any
 // of a warp's 32 links needs it (a smeared source at 24^3 x 48, whose links are
-// beyond in the first APE steps only: 2.98 -> 3.05 ms). Then the error is 0.90 to
+// beyond in the first APE steps only: 2.99 -> 3.04 ms). Then the error is 0.90 to
 // 1.02 times the iteration's for smooth, rough and random links and for kappa =
 // 1.2 to 20.
 // Links with i1^3 > 135 i3 (from kappa = 8.4 to 15.6 on, by the middle singular
@@ -531,7 +531,7 @@ int qcdgpu_smeared_source(qcdgpu_field f, qcdgpu_gauge g, const int x[4], int sp
   // the APE steps do not couple time-slices: only that slice is smeared
   const bool ok = qg::smear_slice(f, g, ape_alpha, ape_n, gauss_alpha, x[0], gauss_n);
   // with APE steps the call ends when the source is there, for callers that
-  // go on on another stream
+  // go on on another stream (15 to 22 us a call where calls follow each other)
   return (ape_n <= 0 || QG_CUDA(cudaStreamSynchronize(qg::stream()))) && ok ? 0 : 1;
 }
 
